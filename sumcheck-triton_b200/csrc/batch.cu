@@ -78,7 +78,7 @@ struct sc_batch {
   size_t state_words = 0;
   std::vector<BatchClass> classes;
   int total_heads = 0;
-  DevBuf fold_pool, state, partials, rounds, items, heads, exprs;
+  DevBuf fold_pool, state, rounds, items, heads, exprs;
   uint32_t* host_state = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ready = nullptr, done = nullptr, fork = nullptr;
@@ -217,7 +217,7 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
     const uint64_t N = uint64_t{1} << B->n[p];
     B->so.push_back(state_offsets(B->n[p], B->K[p], L));
     B->state_base.push_back(B->state_words);
-    B->state_words += (B->so[p].total_words + 3) & ~size_t{3};
+    B->state_words += state_words_aligned(B->so[p]);
     fold_a[p] = fold_words;
     fold_words += (B->n[p] >= 2 ? static_cast<size_t>(B->K[p]) * L * (N / 2) : 0) + 4;
     fold_b[p] = fold_words;
@@ -225,7 +225,8 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
     fold_words = (fold_words + 3) & ~size_t{3};
   }
   if ((rc = ensure(ctx, B->fold_pool, fold_words * 4))) return rc;
-  if ((rc = ensure(ctx, B->state, B->state_words * 4))) return rc;
+  // the proofs' states, then their rounds' sums (copied back: the states alone)
+  if ((rc = ensure(ctx, B->state, B->state_words * 4 + count * sums_bytes(L)))) return rc;
   SC_CUDA(cudaMallocHost(&B->host_state, B->state_words * 4));
   uint32_t* st = static_cast<uint32_t*>(B->state.p);
   uint32_t* pool = static_cast<uint32_t*>(B->fold_pool.p);
@@ -233,7 +234,6 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
   const ExprDev* exprs_dev = static_cast<const ExprDev*>(B->exprs.p);
   // every class's ticks: rounds and items, in one array each (class and tick offsets)
   std::vector<BatchRound> rounds;
-  std::vector<size_t> partial_item;  // per round: index of its first partial slot
   std::vector<BatchItem> items;
   for (BatchClass& C : B->classes) {
     C.head0 = B->total_heads;
@@ -278,6 +278,7 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
         A.st.finals = s + o.finals;
         A.st.claim0 = s + o.claim0;
         A.st.claim = s + o.claim;
+        A.sums = reinterpret_cast<uint64_t*>(st + B->state_words) + static_cast<size_t>(p) * kSumCopies * kMaxPoints * L;
         R.expr = exprs_dev + p;
         if (t == ticks - 1 && ticks < n) {
           R.tail_rounds = n - ticks;
@@ -290,7 +291,6 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
         R.num_items = static_cast<int>(nitems);
         R.item_base = 0;
         R.round_items = static_cast<int>(nitems);
-        partial_item.push_back(items.size());
         const int ridx = static_cast<int>(rounds.size()) - C.tick_round0[t];
         for (uint64_t i = 0; i < nitems; ++i) {
           BatchItem I;
@@ -306,12 +306,9 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
       C.tick_items.push_back(tick_items);
     }
   }
-  if ((rc = ensure(ctx, B->partials, items.size() * kMaxPoints * L * 4))) return rc;
   if ((rc = ensure(ctx, B->rounds, rounds.size() * sizeof(BatchRound)))) return rc;
   if ((rc = ensure(ctx, B->items, items.size() * sizeof(BatchItem)))) return rc;
   if ((rc = ensure(ctx, B->heads, static_cast<size_t>(std::max(1, B->total_heads)) * 4))) return rc;
-  for (size_t r = 0; r < rounds.size(); ++r)
-    rounds[r].partials = static_cast<uint32_t*>(B->partials.p) + partial_item[r] * kMaxPoints * L;
   SC_CUDA(cudaMemcpy(B->rounds.p, rounds.data(), rounds.size() * sizeof(BatchRound), cudaMemcpyHostToDevice));
   SC_CUDA(cudaMemcpy(B->items.p, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice));
   SC_CUDA(cudaMemcpy(B->exprs.p, ed.data(), ed.size() * sizeof(ExprDev), cudaMemcpyHostToDevice));
@@ -320,7 +317,7 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
 
 // The launch sequence of one run (captured once into the graph).
 int batch_issue(sc_batch* B) {
-  SC_CUDA(cudaMemsetAsync(B->state.p, 0, B->state_words * 4, B->stream));
+  SC_CUDA(cudaMemsetAsync(B->state.p, 0, B->state_words * 4 + B->count * sums_bytes(B->L), B->stream));
   SC_CUDA(cudaMemsetAsync(B->heads.p, 0, static_cast<size_t>(std::max(1, B->total_heads)) * 4, B->stream));
   SC_CUDA(cudaEventRecordWithFlags(B->origin, B->stream, cudaEventRecordExternal));
   SC_CUDA(cudaEventRecord(B->fork, B->stream));
@@ -551,7 +548,7 @@ int sc_batch_destroy(sc_batch* B) {
   cudaSetDevice(B->ctx->device);
   if (B->stream) cudaStreamSynchronize(B->stream);
   if (B->exec) cudaGraphExecDestroy(B->exec);
-  for (DevBuf* b : {&B->fold_pool, &B->state, &B->partials, &B->rounds, &B->items, &B->heads, &B->exprs})
+  for (DevBuf* b : {&B->fold_pool, &B->state, &B->rounds, &B->items, &B->heads, &B->exprs})
     if (b->p) cudaFree(b->p);
   if (B->host_state) cudaFreeHost(B->host_state);
   for (BatchClass& C : B->classes) {

@@ -86,7 +86,7 @@ struct ProveRun {
     if ((rc = ensure(ctx, ctx->fold_a, fold_a_words * 4))) return rc;
     if ((rc = ensure(ctx, ctx->fold_b, fold_b_words * 4))) return rc;
     const StateOffsets so = state_offsets(n, K_, L);
-    if ((rc = ensure(ctx, ctx->state, so.total_words * 4))) return rc;
+    if ((rc = ensure(ctx, ctx->state, state_and_sums_bytes(so, L)))) return rc;
 
     ExprDev E;
     build_expr_dev<L>(*ex, *f, E);
@@ -111,23 +111,21 @@ struct ProveRun {
       while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
       smem = static_cast<size_t>(threads) * per_thread;
     } else {
-      smem = shape_round_smem_bytes(L, K, shape, threads);  // block_reduce scratch (+ the pair stage)
+      smem = shape_round_smem_bytes(L, K, shape, threads);  // reduction scratch (+ the pair stage)
     }
     int blocks_per_sm = 0;
     SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, threads, smem));
     if (blocks_per_sm < 1) return fail(SC_ERR_UNSUPPORTED, "round kernel does not fit on an SM (K=%d, L=%d)", K_, L);
     const uint64_t grid_max = static_cast<uint64_t>(blocks_per_sm) * ctx->sm_count;
-    if ((rc = ensure(ctx, ctx->partials, grid_max * kMaxPoints * L * 4))) return rc;
 
     FieldParams<L, K> F;
     for (int l = 0; l < L; ++l) F.p[l] = f->hf.p[l];
     F.np = f->hf.np;
 
     uint32_t* st = static_cast<uint32_t*>(ctx->state.p);
+    SC_CUDA(cudaMemsetAsync(st, 0, state_and_sums_bytes(so, L), ctx->stream));
     if (state_io)
       SC_CUDA(cudaMemcpyAsync(st, state_io, so.total_words * 4, cudaMemcpyHostToDevice, ctx->stream));
-    else
-      SC_CUDA(cudaMemsetAsync(st, 0, so.total_words * 4, ctx->stream));
     if (mode == SC_CHALLENGE_EXPLICIT)
       SC_CUDA(cudaMemcpyAsync(st + so.chals, explicit_ch, static_cast<size_t>(n) * L * 4, cudaMemcpyHostToDevice,
                               ctx->stream));
@@ -136,7 +134,7 @@ struct ProveRun {
     std::memset(&A, 0, sizeof(A));
     A.num_rounds = n;
     A.mode = mode;
-    A.partials = static_cast<uint32_t*>(ctx->partials.p);
+    A.sums = state_sums(st, so);
     A.fc = f->dev;
     A.st.counter = st + so.counter;
     A.st.status = st + so.status;
@@ -191,7 +189,6 @@ struct ProveRun {
         TailDesc* dev = static_cast<TailDesc*>(ctx->tail.p);
         desc.r.args = A;
         desc.r.expr = &dev->e;
-        desc.r.partials = A.partials;
         desc.r.num_items = 1;
         desc.r.round_items = 1;
         desc.r.tail_rounds = n - 1 - j;
@@ -379,7 +376,7 @@ int sc_ctx_destroy(sc_ctx* ctx) {
   if (!ctx) return SC_OK;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  for (DevBuf* b : {&ctx->fold_a, &ctx->fold_b, &ctx->partials, &ctx->state, &ctx->tail})
+  for (DevBuf* b : {&ctx->fold_a, &ctx->fold_b, &ctx->state, &ctx->tail})
     if (b->p) cudaFree(b->p);
   for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
   if (ctx->host_state) cudaFreeHost(ctx->host_state);

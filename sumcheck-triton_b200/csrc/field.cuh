@@ -295,7 +295,8 @@ __device__ __forceinline__ Fe<L> fe_mul(const Fe<L>& a, const Fe<L>& b, const Fi
 }
 
 // Lazy Goldilocks arithmetic (field_gold.cuh): values are any representative in [0, 2^64)
-// between operations and are made canonical (gold_canon) only where they leave a thread.
+// between operations; point sums leave a thread as they are (the round's integer sums are
+// reduced mod p once, prover.cuh).
 // Which forms, measured on B200 (plain_goldilocks n = 24 p50 / the mixed stream's 64-bit
 // group alone, 240 proofs; canonical arithmetic 1.65 / 6.07 ms):
 //   point steps (value + canonical difference) on the ALU, SC_GOLD_LAZY_STEP_ALU = 1:
@@ -336,12 +337,6 @@ __device__ __forceinline__ Fe<2> gl_mul(const Fe<2>& a, const Fe<2>& b, const Go
 #endif
   return r;
 }
-__device__ __forceinline__ Fe<2> gl_canon(const Fe<2>& a, const GoldK k) {
-  Fe<2> r;
-  gold_canon(r.w, a.w, k);
-  return r;
-}
-
 template <int L>
 __device__ __forceinline__ bool fe_is_zero(const Fe<L>& a) {
   uint32_t o = 0;
@@ -374,6 +369,14 @@ __device__ __forceinline__ Fe<L> fe_shfl_down(const Fe<L>& a, int delta) {
   Fe<L> r;
 #pragma unroll
   for (int i = 0; i < L; ++i) r.w[i] = __shfl_down_sync(0xffffffffu, a.w[i], delta);
+  return r;
+}
+
+template <int L>
+__device__ __forceinline__ Fe<L> fe_shfl_xor(const Fe<L>& a, int mask) {
+  Fe<L> r;
+#pragma unroll
+  for (int i = 0; i < L; ++i) r.w[i] = __shfl_xor_sync(0xffffffffu, a.w[i], mask);
   return r;
 }
 

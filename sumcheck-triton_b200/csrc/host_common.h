@@ -71,7 +71,7 @@ struct sc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
-  DevBuf fold_a, fold_b, partials, state;
+  DevBuf fold_a, fold_b, state;       // state: the proof state's words, then the round's sums
   DevBuf tail;                        // the tail launch's BatchRound and ExprDev
   void* tail_host = nullptr;          // pinned staging of the same
   cudaEvent_t tail_copied = nullptr;  // the staging's last copy to the device
@@ -417,6 +417,14 @@ inline StateOffsets state_offsets(int n, int K, int L) {
   return o;
 }
 
+
+// A device buffer of the proof state and the round's integer sums behind it (RoundArgs::sums);
+// both are zero before a proof's first round, so one memset covers them.
+inline size_t state_words_aligned(const StateOffsets& so) { return (so.total_words + 3) & ~size_t{3}; }
+inline size_t state_and_sums_bytes(const StateOffsets& so, int L) { return state_words_aligned(so) * 4 + sums_bytes(L); }
+inline uint64_t* state_sums(uint32_t* state, const StateOffsets& so) {
+  return reinterpret_cast<uint64_t*>(state + state_words_aligned(so));
+}
 
 // ---- transcripts: a proof stopped at a round boundary, resumable from the same tables
 //

@@ -54,64 +54,71 @@ constexpr KeccakConsts make_keccak_consts() {
 
 static __constant__ KeccakConsts kKeccak = make_keccak_consts();
 
-__device__ __forceinline__ uint64_t rotl64(uint64_t v, uint32_t r) {
-  return (v << r) | (v >> ((64u - r) & 63u));
-}
-
-// Keccak-f[1600] on the warp-distributed state (all 32 lanes must call).
-__device__ __forceinline__ void keccak_f1600_warp(uint64_t& a, int lane) {
+// Keccak-f[1600] on the warp-distributed state: lane i < 25 holds word A[i % 5, i / 5] as
+// (lo, hi). All 32 lanes must call; lanes 25..31 carry values nothing reads.
+//
+// The permutation is one dependent chain, so its time is the latency of the exchanges between
+// lanes. A round has three: the column parities, the neighbour columns' parities (theta), and
+// one for pi and chi together -- chi's two neighbours are read straight from the rotated words
+// they come from, instead of a pi exchange followed by a chi exchange. Words are two 32-bit
+// registers: the per-lane rotation is a swap and two funnel shifts. Two rounds a loop pass
+// (24 unrolled rounds would be fetched anew at every round's end). Measured on B200, one warp:
+// 4530 clocks, against 5205 with four exchanges and 64-bit shifts. Exchanging through shared
+// memory (4970-5340), and theta in one exchange of ten words (5060), were slower.
+__device__ __forceinline__ void keccak_f1600_warp(uint32_t& lo, uint32_t& hi, int lane) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int x = lane % 5, y = (lane / 5) % 5;
   const int row = 5 * y;
   const uint32_t rot = lane < 25 ? kKeccak.rot[lane] : 0u;
+  const bool swap = rot >= 32;
+  const uint32_t s = rot & 31;
+  const int x1 = (x + 1) % 5, x2 = (x + 2) % 5, xm = (x + 4) % 5;
+  const int c1 = x + 5 * ((y + 1) % 5), c2 = x + 5 * ((y + 2) % 5), c3 = x + 5 * ((y + 3) % 5), c4 = x + 5 * ((y + 4) % 5);
   // pi (FIPS 202 3.2.3): A'[x, y] = A[(x + 3y) mod 5, x]
-  const int src_pi = (x + 3 * y) % 5 + 5 * x;
-#pragma unroll 1
+  const int p0 = (x + 3 * y) % 5 + 5 * x, p1 = (x1 + 3 * y) % 5 + 5 * x1, p2 = (x2 + 3 * y) % 5 + 5 * x2;
+  const uint32_t iota = lane == 0 ? ~0u : 0u;
+#pragma unroll 2
   for (int ir = 0; ir < 24; ++ir) {
+    const uint64_t rc = kKeccak.rc[ir];
+    const uint32_t rc_lo = static_cast<uint32_t>(rc) & iota, rc_hi = static_cast<uint32_t>(rc >> 32) & iota;
     // theta
-    uint64_t c = a;
-#pragma unroll
-    for (int k = 1; k < 5; ++k) c ^= __shfl_sync(0xffffffffu, a, x + 5 * ((y + k) % 5));
-    const uint64_t cm = __shfl_sync(0xffffffffu, c, (x + 4) % 5 + row);
-    const uint64_t cp = __shfl_sync(0xffffffffu, c, (x + 1) % 5 + row);
-    a ^= cm ^ rotl64(cp, 1);
-    // rho then pi
-    const uint64_t b = __shfl_sync(0xffffffffu, rotl64(a, rot), src_pi);
-    // chi
-    const uint64_t b1 = __shfl_sync(0xffffffffu, b, (x + 1) % 5 + row);
-    const uint64_t b2 = __shfl_sync(0xffffffffu, b, (x + 2) % 5 + row);
-    a = b ^ (~b1 & b2);
-    // iota
-    if (lane == 0) a ^= kKeccak.rc[ir];
+    uint32_t cl = lo ^ __shfl_sync(kAll, lo, c1) ^ __shfl_sync(kAll, lo, c2);
+    uint32_t ch = hi ^ __shfl_sync(kAll, hi, c1) ^ __shfl_sync(kAll, hi, c2);
+    cl = cl ^ __shfl_sync(kAll, lo, c3) ^ __shfl_sync(kAll, lo, c4);
+    ch = ch ^ __shfl_sync(kAll, hi, c3) ^ __shfl_sync(kAll, hi, c4);
+    const uint32_t ml = __shfl_sync(kAll, cl, xm + row), mh = __shfl_sync(kAll, ch, xm + row);
+    const uint32_t ul = __shfl_sync(kAll, cl, x1 + row), uh = __shfl_sync(kAll, ch, x1 + row);
+    lo ^= ml ^ __funnelshift_l(uh, ul, 1);
+    hi ^= mh ^ __funnelshift_l(ul, uh, 1);
+    // rho
+    const uint32_t s0 = swap ? hi : lo, s1 = swap ? lo : hi;
+    const uint32_t rl = __funnelshift_l(s1, s0, s), rh = __funnelshift_l(s0, s1, s);
+    // pi and chi, then iota
+    const uint32_t b0l = __shfl_sync(kAll, rl, p0), b0h = __shfl_sync(kAll, rh, p0);
+    const uint32_t b1l = __shfl_sync(kAll, rl, p1), b1h = __shfl_sync(kAll, rh, p1);
+    const uint32_t b2l = __shfl_sync(kAll, rl, p2), b2h = __shfl_sync(kAll, rh, p2);
+    lo = (b0l ^ (~b1l & b2l)) ^ rc_lo;
+    hi = (b0h ^ (~b1h & b2h)) ^ rc_hi;
   }
-  if (lane >= 25) a = 0;
 }
 
-// SHA3-256 of msg[0..len) held in shared memory. The buffer must have room for the padding
-// (len rounded up to a multiple of 136 bytes) and be 8-byte aligned; it is padded in place.
-// Every lane of the calling warp gets the 32-byte digest as 8 little-endian words.
-__device__ __forceinline__ void sha3_256_warp(uint8_t* msg, int len, uint32_t (&digest)[8]) {
+// SHA3-256 by one warp (every lane calls). word(q) is the message's 32-bit little-endian word
+// q, with the padding's 0x06 after the last byte and zeros beyond; len its length in bytes.
+// digest: lanes 0..3 get 64-bit word `lane` of the digest as (lo, hi); the others' are unused.
+template <typename Word>
+__device__ __forceinline__ void sha3_256_warp(Word word, int len, uint32_t& lo, uint32_t& hi) {
   const int lane = threadIdx.x & 31;
   constexpr int kRate = 136;
   const int nblocks = len / kRate + 1;
-  const int padded = nblocks * kRate;
-  for (int i = len + lane; i < padded; i += 32) msg[i] = 0;
-  __syncwarp();
-  if (lane == 0) {
-    msg[len] ^= 0x06;
-    msg[padded - 1] ^= 0x80;
-  }
-  __syncwarp();
-  uint64_t a = 0;
-  const uint64_t* m64 = reinterpret_cast<const uint64_t*>(msg);
+  lo = hi = 0;
   for (int b = 0; b < nblocks; ++b) {
-    if (lane < kRate / 8) a ^= m64[b * (kRate / 8) + lane];
-    keccak_f1600_warp(a, lane);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint64_t w = __shfl_sync(0xffffffffu, a, i);
-    digest[2 * i] = static_cast<uint32_t>(w);
-    digest[2 * i + 1] = static_cast<uint32_t>(w >> 32);
+    if (lane < kRate / 8) {
+      const int q = b * (kRate / 4) + 2 * lane;
+      lo ^= word(q);
+      hi ^= word(q + 1);
+      if (b == nblocks - 1 && lane == kRate / 8 - 1) hi ^= 0x80000000u;
+    }
+    keccak_f1600_warp(lo, hi, lane);
   }
 }
 

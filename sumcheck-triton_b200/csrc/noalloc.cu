@@ -6,7 +6,7 @@
 // the proving path. sc_prove grows its context's scratch with cudaMalloc and stages the
 // results in pinned host memory; this variant does neither.
 //
-// Its scratch -- the field constants, the proof state, the block partials and the two fold
+// Its scratch -- the field constants, the proof state, the round's sums and the two fold
 // buffers -- lives in one file-scope __device__ array of kNoAllocScratchBytes (32 MiB).
 // Every GPU that loads the library holds that array until the process exits. A proof fits
 // when K L 2^n (3/4) words of fold buffers plus the small rest fit; larger proofs are
@@ -20,7 +20,7 @@
 // first call on the device, or later calls would launch into an unmapped address.
 // The call is synchronous: it returns once the results are in the caller's arrays.
 // All calls share the one array and it keeps the last call's contents; what must start at
-// zero (the proof state's counter, status and checksum) is cleared by every call. Two
+// zero (the proof state, the round's sums) is cleared by every call. Two
 // calls whose work overlaps on the same GPU race on the array: issue them on one stream,
 // or wait for one before starting the next.
 #include <mutex>
@@ -84,12 +84,11 @@ static int run(sc_ctx* ctx, const sc_field* f, const sc_expr* ex, int n, const u
   if (bps < 1) return fail(SC_ERR_UNSUPPORTED, "round kernel does not fit on an SM (K=%d, L=%d)", K_, L);
   const uint64_t grid_max = std::min<uint64_t>(static_cast<uint64_t>(bps) * ctx->sm_count, kNoAllocMaxBlocks);
 
-  // carve the scratch array: field constants, proof state, partials, fold A, fold B
+  // carve the scratch array: field constants, proof state and sums, fold A, fold B
   const StateOffsets so = state_offsets(n, K_, L);
   const size_t w_fc = 0;
   const size_t w_state = w_fc + align64(sizeof(FieldConsts) / 4);
-  const size_t w_part = w_state + align64(so.total_words);
-  const size_t w_a = w_part + align64(grid_max * kMaxPoints * L);
+  const size_t w_a = w_state + align64(state_and_sums_bytes(so, L) / 4);
   const size_t w_b = w_a + align64(n >= 2 ? static_cast<size_t>(K_) * L * (N / 2) : 0);
   const size_t w_end = w_b + align64(n >= 3 ? static_cast<size_t>(K_) * L * (N / 4) : 0);
   if (w_end * 4 > kNoAllocScratchBytes)
@@ -105,7 +104,7 @@ static int run(sc_ctx* ctx, const sc_field* f, const sc_expr* ex, int n, const u
 
   uint32_t* st = base + w_state;
   SC_CUDA(cudaMemcpyAsync(base + w_fc, &f->consts, sizeof(FieldConsts), cudaMemcpyHostToDevice, ctx->stream));
-  SC_CUDA(cudaMemsetAsync(st, 0, so.total_words * 4, ctx->stream));
+  SC_CUDA(cudaMemsetAsync(st, 0, state_and_sums_bytes(so, L), ctx->stream));
   if (mode == SC_CHALLENGE_EXPLICIT)
     SC_CUDA(cudaMemcpyAsync(st + so.chals, explicit_ch, static_cast<size_t>(n) * L * 4, cudaMemcpyHostToDevice,
                             ctx->stream));
@@ -114,7 +113,7 @@ static int run(sc_ctx* ctx, const sc_field* f, const sc_expr* ex, int n, const u
   std::memset(&A, 0, sizeof(A));
   A.num_rounds = n;
   A.mode = mode;
-  A.partials = base + w_part;
+  A.sums = state_sums(st, so);
   A.fc = reinterpret_cast<const FieldConsts*>(base + w_fc);
   A.st.counter = st + so.counter;
   A.st.status = st + so.status;

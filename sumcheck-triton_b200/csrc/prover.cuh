@@ -10,9 +10,10 @@
 //      field_sumcheck.cu:326-348) and evaluates the constraint at each point
 //      (field_sumcheck.cu:389-590), accumulating d+1 sums per thread (see eval_pair for the
 //      exact-arithmetic shortcuts: extrapolated low-degree terms, g(1) from the claim);
-//   3. reduce: warp shuffles, then shared memory, then one partial per block in global
-//      memory; the last block to finish (atomic ticket) sums the partials -- a single-pass
-//      grid reduction in place of the reference's log-depth launch tree
+//   3. reduce: the point sums are summed word by word as integers -- over the warp, the block
+//      (shared memory) and the grid (64-bit atomic adds) -- with no modular arithmetic until
+//      the last block to finish (atomic ticket) reads (d + 1) L integers and reduces them
+//      mod p: a single-pass grid reduction in place of the reference's log-depth launch tree
 //      (field_sumcheck.cu:635-675, :996-1010);
 //   4. finalise (last block only): stores g_j(0..d), adds the round's checksum, derives r_j
 //      by SHA3 over the round polynomial on the device (field_sumcheck.cu:857-907), and when
@@ -36,6 +37,14 @@ constexpr int kMaxVars = 32;
 constexpr int kMaxTerms = 32;
 constexpr int kMaxFlat = 128;
 constexpr int kMaxRounds = 40;
+
+// Copies of a round's grid-wide integer sums: block (or item) i adds to copy i % kSumCopies, so
+// that a few hundred blocks finishing together do not queue on the same addresses; the last
+// block adds the copies up. One round at a time uses them.
+constexpr int kSumCopies = 16;
+__host__ __device__ constexpr size_t sums_bytes(int L) { return sizeof(uint64_t) * kSumCopies * kMaxPoints * L; }
+// Shared-memory words of the block reduction's scratch: a 64-bit sum per warp, point and limb.
+__host__ __device__ constexpr int reduce_scratch_words(int threads, int L) { return (threads / 32) * kMaxPoints * L * 2; }
 
 enum ChallengeMode : int32_t { kChallengeSha3 = 0, kChallengeFixed = 1, kChallengeExplicit = 2 };
 
@@ -118,7 +127,8 @@ struct RoundArgs {
   int32_t mode;          // ChallengeMode
   int32_t skip1;         // g(1) = claim - g(0) instead of evaluating point 1
   int32_t want_claim;    // store g_j(r_j) for the next round
-  uint32_t* partials;    // [gridDim.x][kMaxPoints][L]
+  uint64_t* sums;        // the grid's integer sums, [kSumCopies][kMaxPoints * L]: zero before
+                         // the round, zero again after it
   const FieldConsts* fc;
   ProofState st;
   uint32_t* ext_out;     // non-null: the round's sums g_j(0..d) go here and the round is not
@@ -376,7 +386,7 @@ __host__ __device__ constexpr bool shape_async_stage(int L, int K, int shape) {
 }
 // Dynamic shared memory (bytes) of a compile-time shape round kernel of `threads` threads.
 __host__ __device__ constexpr size_t shape_round_smem_bytes(int L, int K, int shape, int threads) {
-  return 4 * (static_cast<size_t>(threads / 32) * kMaxPoints * L +
+  return 4 * (static_cast<size_t>(reduce_scratch_words(threads, L)) +
               (shape_async_stage(L, K, shape) ? static_cast<size_t>(threads) * shape_tables(shape) * L * 4 : 0));
 }
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
@@ -415,7 +425,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
   constexpr bool kAsync = (kGoldLazy && SC_GOLD_ASYNC) || l8_async_stage(L, SHAPE);
   const int nv = SHAPE == kShapeGeneric ? E.num_vars : NR;
   // kAsync: this thread's stage, after the block reduction's scratch (16-byte aligned)
-  uint32_t* const stage = sv + (nthr / 32) * kMaxPoints * L;
+  uint32_t* const stage = sv + reduce_scratch_words(nthr, L);
   auto issue = [&](uint64_t qn) {  // copies of pair qn into the stage
 #pragma unroll
     for (int i = 0; i < NR; ++i)
@@ -595,61 +605,89 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       }
     }
   }
-  if constexpr (kGoldLazy || lazy_generic<L, K>()) {
-    const GoldK gk = gold_k(F);
-#pragma unroll
-    for (int t = 0; t <= DMAX; ++t) acc[t] = gl_canon(acc[t], gk);
-  }
 }
 
-// Reduce acc[0..d] over the block; the block sums land in red_out[t * L + l] (shared).
-template <int L, int K, int N>
-__device__ __forceinline__ void block_reduce(Fe<L> (&acc)[N], int d, uint32_t* scratch, uint32_t* red_out,
-                                             const FieldParams<L, K>& F) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+// ---- reduction
+//
+// Point sums are added word by word as integers: a 32-bit word splits into 16-bit halves whose
+// warp sums (redux) cannot overflow, and every wider sum is 64 bits. Nothing is reduced mod p
+// before the whole round's sum is known, so any representative of a residue may be summed and
+// no modular additions run in the tail of a round. Measured on B200 (clocks of one block): the
+// shuffle tree of modular additions it replaces took 3.3k at 2 limbs and degree 4, 6.7k at 8
+// limbs and degree 4, 17k at 8 limbs and degree 7, and ran twice a round with a loop over the
+// blocks' partials in between (6.3k / 10.9k).
+
+// This warp's integer sums of acc[0..d] into its row of scratch.
+template <int L, int N>
+__device__ __forceinline__ void warp_sums(const Fe<L> (&acc)[N], int d, uint32_t* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t* row = reinterpret_cast<uint64_t*>(scratch) + warp * kMaxPoints * L;
+  constexpr int NV = (N * L + 31) / 32;
+  uint64_t mine[NV];  // lane i keeps the sums of words i, i + 32, ...
+#pragma unroll
+  for (int v = 0; v < NV; ++v) mine[v] = 0;
 #pragma unroll
   for (int t = 0; t < N; ++t) {
     if (t > d) break;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[t] = fe_add(acc[t], fe_shfl_down(acc[t], off), F);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int t = 0; t < N; ++t) {
-      if (t > d) break;
-      st_fe<L>(scratch + (warp * kMaxPoints + t) * L, acc[t]);
+    for (int l = 0; l < L; ++l) {
+      const uint32_t lo = __reduce_add_sync(0xffffffffu, acc[t].w[l] & 0xffffu);
+      const uint32_t hi = __reduce_add_sync(0xffffffffu, acc[t].w[l] >> 16);
+      if (lane == (t * L + l) % 32) mine[(t * L + l) / 32] = lo + (static_cast<uint64_t>(hi) << 16);
     }
   }
-  __syncthreads();
-  if (warp == 0) {
 #pragma unroll
-    for (int t = 0; t < N; ++t) {
-      if (t > d) break;
-      Fe<L> v = lane < nwarps ? ld_fe<L>(scratch + (lane * kMaxPoints + t) * L) : fe_zero<L>();
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = fe_add(v, fe_shfl_down(v, off), F);
-      if (lane == 0) st_fe<L>(red_out + t * L, v);
-    }
-  }
-  __syncthreads();
+  for (int v = 0; v < NV; ++v)
+    if (v * 32 + lane < N * L) row[v * 32 + lane] = mine[v];
 }
 
-// Sums the partials of blocks/items [first, first + count) into g_sm[t * L + l] (block-wide).
-template <int L, int K, int N>
-__device__ __forceinline__ void reduce_partials(const uint32_t* partials, uint64_t first, uint64_t count, int d,
-                                                uint32_t* scratch, uint32_t* g_sm, const FieldParams<L, K>& F) {
-  Fe<L> acc[N];
-#pragma unroll
-  for (int t = 0; t < N; ++t) acc[t] = fe_zero<L>();
-  for (uint64_t b = threadIdx.x; b < count; b += blockDim.x) {
-    const uint32_t* pb = partials + (first + b) * kMaxPoints * L;
-#pragma unroll
-    for (int t = 0; t < N; ++t) {
-      if (t > d) break;
-      acc[t] = fe_add(acc[t], ld_fe_cg<L>(pb + t * L), F);
-    }
+// After warp_sums and a barrier: the block's sums, into s_sm (alone: the block is the whole
+// round) or added to copy `copy` of the round's sums.
+template <int L>
+__device__ __forceinline__ void block_sums(const uint32_t* scratch, int d, bool alone, uint64_t* s_sm, uint64_t* sums,
+                                           uint32_t copy) {
+  const int nwarps = blockDim.x >> 5;
+  const uint64_t* rows = reinterpret_cast<const uint64_t*>(scratch);
+  for (int i = threadIdx.x; i < (d + 1) * L; i += blockDim.x) {
+    uint64_t s = 0;
+    for (int w = 0; w < nwarps; ++w) s += rows[w * kMaxPoints * L + i];
+    if (alone)
+      s_sm[i] = s;
+    else
+      atomicAdd(reinterpret_cast<unsigned long long*>(sums + (copy % kSumCopies) * kMaxPoints * L + i),
+                static_cast<unsigned long long>(s));
   }
-  block_reduce<L, K, N>(acc, d, scratch, g_sm, F);
+}
+
+// Block-wide, after warp_sums: true in the block that completes the round (its `parts`-th block
+// or item), with the round's integer sums in s_sm; every thread calls. Ends with a barrier.
+template <int L>
+__device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32_t part, uint32_t parts, uint64_t* sums,
+                                          uint32_t* counter, uint64_t* s_sm, int* is_last) {
+  __syncthreads();
+  block_sums<L>(scratch, d, parts == 1, s_sm, sums, part);
+  if (parts > 1) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) *is_last = atomicAdd(counter, 1u) == parts - 1;
+    __syncthreads();
+    if (!*is_last) return false;
+    __threadfence();
+    for (int i = threadIdx.x; i < (d + 1) * L; i += blockDim.x) {
+      uint64_t v[kSumCopies], s = 0;
+#pragma unroll
+      for (int c = 0; c < kSumCopies; ++c) v[c] = c < static_cast<int>(parts) ? __ldcg(sums + c * kMaxPoints * L + i) : 0;
+#pragma unroll
+      for (int c = 0; c < kSumCopies; ++c) {
+        s += v[c];
+        if (c < static_cast<int>(parts)) sums[c * kMaxPoints * L + i] = 0;
+      }
+      s_sm[i] = s;
+    }
+    if (threadIdx.x == 0) *counter = 0;
+  }
+  __syncthreads();
+  return true;
 }
 
 template <int L>
@@ -657,114 +695,212 @@ __device__ __forceinline__ Fe<L> fc_get(const uint32_t* row) {
   return ld_fe<L>(row);
 }
 
-// g(r) for the polynomial with values g_sm[t] at t = 0..d (Lagrange form with the field's
-// precomputed weights); lane t < d + 1 forms one term, the warp sums them (all lanes call).
+// a b R^-1 mod p, fully reduced, for a < p and any b < 2^(32 L).
 template <int L, int K>
-__device__ __forceinline__ Fe<L> lagrange_at(const uint32_t* g_sm, int d, const Fe<L>& r, const FieldConsts& fc,
-                                             const FieldParams<L, K>& F) {
-  const int lane = threadIdx.x & 31;
-  Fe<L> term = fe_zero<L>();
-  if (lane <= d) {
-    term = fe_mul(ld_fe<L>(g_sm + lane * L), fc_get<L>(fc.lag[d][lane]), F);
-    for (int s = 0; s <= d; ++s)
-      if (s != lane) term = fe_mul(term, fe_sub(r, fc_get<L>(fc.pts[s]), F), F);
-  }
+__device__ __forceinline__ Fe<L> fe_mul_any(const Fe<L>& a, Fe<L> b, const FieldParams<L, K>& F) {
+  if constexpr (K == kFieldMersenne127 && L == 4) {
+    // the product wants operands <= p = 2^127 - 1: bit 127 is worth 1
+    const uint32_t top = b.w[3] >> 31;
+    b.w[3] &= 0x7fffffffu;
+    uint64_t c = top;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) term = fe_add(term, fe_shfl_down(term, off), F);
-  return fe_shfl(term, 0);
+    for (int l = 0; l < 4; ++l) {
+      c += b.w[l];
+      b.w[l] = static_cast<uint32_t>(c);
+      c >>= 32;
+    }
+    return fe_mul(a, b, F);
+  } else if constexpr (K == kFieldGoldilocks && L == 2) {
+    Fe<2> r;
+    gold_mul(r.w, a.w, b.w);  // h < p and b' < p below, whatever b is
+    return r;
+  } else {
+    return fe_mul(a, b, F);  // the rows scan b's words against a: t < a + p throughout
+  }
 }
 
-// Last block of a round: g_j is in g_sm[t * L + l] (point 1 still empty when skip1).
-// Warp 0 does all of this.
+// The round's integer sums to g_j: sum_l s[t L + l] 2^(32 l) mod p for t = 0..d, into
+// g_sm[t L + l]. The low L words times `one` and the word above them times R^2 are one product
+// each, in lanes t and 8 + t of the calling warp.
 template <int L, int K>
-__device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F, uint32_t* g_sm,
-                               uint8_t* msg) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void sums_to_points(const uint64_t* s_sm, int d, const FieldConsts& fc,
+                                               const FieldParams<L, K>& F, uint32_t* g_sm) {
+  const int lane = threadIdx.x & 31, t = lane & 7;
+  const Fe<L> con = fc_get<L>(lane < 8 ? fc.one : fc.r2);
+  Fe<L> v = fe_zero<L>();
+  if (t <= d && lane < 16) {
+    uint64_t c = 0;
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+      c += s_sm[t * L + l];
+      v.w[l] = static_cast<uint32_t>(c);
+      c >>= 32;
+    }
+    if (lane >= 8) {
+      v = fe_zero<L>();
+      v.w[0] = static_cast<uint32_t>(c);
+    }
+  }
+  const Fe<L> x = fe_mul_any(con, v, F);
+  const Fe<L> g = fe_add(x, fe_shfl_down(x, 8), F);
+  if (lane <= d) st_fe<L>(g_sm + lane * L, g);
+  __syncwarp();
+}
+
+// g(1) = claim - g(0), when the round did not evaluate point 1 (one warp).
+template <int L, int K>
+__device__ __forceinline__ void point1_from_claim(const uint32_t* claim, uint32_t* g_sm, const FieldParams<L, K>& F) {
+  if ((threadIdx.x & 31) == 0) st_fe<L>(g_sm + L, fe_sub(ld_fe_cg<L>(claim), ld_fe<L>(g_sm), F));
+  __syncwarp();
+}
+
+// The transcript's domain string as little-endian words; word 5 holds its last byte.
+struct TranscriptDomain {
+  uint32_t w[6];
+};
+constexpr TranscriptDomain make_transcript_domain() {
+  const char dom[] = "zkduel:field-sweep:v1";
+  TranscriptDomain t{};
+  for (int i = 0; i < 21; ++i) t.w[i / 4] |= static_cast<uint32_t>(static_cast<unsigned char>(dom[i])) << (8 * (i % 4));
+  return t;
+}
+static __constant__ TranscriptDomain kTranscriptDomain = make_transcript_domain();
+
+// The end of round j, with g_j complete in g_sm[t * L + l]; every thread of the block calls,
+// after a barrier. Warp 0 derives r_j (into r_sm[L] too, for a caller that goes on with the
+// next round in this block, after a barrier of its own); the next warp, if there is one,
+// stores the round polynomial, the checksum and the claim of round 0 meanwhile.
+template <int L, int K>
+__device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F, const uint32_t* g_sm,
+                               uint32_t* r_sm) {
+  __shared__ __align__(8) uint32_t dig_sm[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d = E.degree;
   const int j = A.round;
   const FieldConsts& fc = *A.fc;
-  // 0. g(1) from the claim this round must meet, or, when asked, that claim checked
-  if (A.skip1) {
-    if (lane == 0) st_fe<L>(g_sm + L, fe_sub(ld_fe_cg<L>(A.st.claim), ld_fe<L>(g_sm), F));
-    __syncwarp();
-  } else if (A.check_claim && lane == 0) {
-    const Fe<L> s = fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F);
-    const Fe<L> c = ld_fe_cg<L>(A.st.claim);
-    bool eq = true;
-#pragma unroll
-    for (int l = 0; l < L; ++l) eq = eq && s.w[l] == c.w[l];
-    if (!eq) atomicOr(A.st.status, kStatusClaim);
-  }
-  // 1. round polynomial and checksum
-  for (int i = lane; i < (d + 1) * L; i += 32) A.st.polys[(j * kMaxPoints + i / L) * L + i % L] = g_sm[i];
-  if (lane == 0) {
+  if (warp == (blockDim.x > 32 ? 1 : 0)) {
+    // round polynomial, checksum, claim checks
     uint64_t cs = 0;
-    for (int t = 0; t <= d; ++t)
-      for (int l = 0; l < L; ++l) cs += static_cast<uint64_t>(l + 1) * g_sm[t * L + l];
-    *A.st.checksum += cs;
-    if (j == 0) {
-      const Fe<L> c0 = fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F);
-      st_fe<L>(A.st.claim0, c0);
+    for (int i = lane; i < (d + 1) * L; i += 32) {
+      const uint32_t w = g_sm[i];
+      A.st.polys[(j * kMaxPoints + i / L) * L + i % L] = w;
+      cs += static_cast<uint64_t>(i % L + 1) * w;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) cs += __shfl_down_sync(0xffffffffu, cs, off);
+    if (lane == 0) {
+      *A.st.checksum += cs;
+      if (j == 0 || (A.check_claim && !A.skip1)) {
+        const Fe<L> s = fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F);
+        if (j == 0) st_fe<L>(A.st.claim0, s);
+        if (A.check_claim && !A.skip1) {
+          const Fe<L> c = ld_fe_cg<L>(A.st.claim);
+          bool eq = true;
+#pragma unroll
+          for (int l = 0; l < L; ++l) eq = eq && s.w[l] == c.w[l];
+          if (!eq) atomicOr(A.st.status, kStatusClaim);
+        }
+      }
     }
   }
-  // 2. challenge r_j
+  if (warp != 0) return;
+  const bool last_round = j == A.num_rounds - 1;
+  const bool claim = A.want_claim || last_round;
+  // What the end of the round reads from global memory, before the hash: the digest's weights
+  // (lanes 0..7) and the Lagrange weights (lanes 8..8 + d); T_{n-1} in the last round (lane k).
+  constexpr int kParts = 8 / L;  // field-sized pieces of the 256-bit digest
+  Fe<L> con = fe_zero<L>();
+  if (lane < kParts)
+    con = fc_get<L>(fc.kdig[lane * L]);
+  else if (claim && lane >= 8 && lane <= 8 + d)
+    con = fc_get<L>(fc.lag[d][lane - 8]);
+  Fe<L> e = fe_zero<L>(), o = fe_zero<L>();
+  if (last_round && lane < E.num_vars) {
+    const uint32_t* tab = A.fold ? A.dst : A.src;  // T_{n-1}: 2 entries per plane
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+      e.w[l] = __ldcg(tab + (lane * L + l) * 2 + 0);
+      o.w[l] = __ldcg(tab + (lane * L + l) * 2 + 1);
+    }
+  }
+  // challenge r_j; lanes 8 + t: g_j(t) times its Lagrange weight, in the same product
+  Fe<L> v = fe_zero<L>();
+  if (A.mode == kChallengeSha3) {
+    // message: domain string (21 bytes) || u32 j || the words of g_j(0..d); word i of j || g
+    // starts at byte 21 + 4 i, so a message word joins two of them
+    const int nwords = 1 + (d + 1) * L;
+    auto tail = [&](int i) -> uint32_t { return i == 0 ? static_cast<uint32_t>(j) : (i < nwords ? g_sm[i - 1] : (i == nwords ? 6u : 0u)); };
+    auto word = [&](int q) -> uint32_t {
+      if (q < 5) return kTranscriptDomain.w[q];
+      return (q == 5 ? kTranscriptDomain.w[5] : tail(q - 6) >> 24) | (tail(q - 5) << 8);
+    };
+    uint32_t lo, hi;
+    sha3_256_warp(word, 21 + 4 * nwords, lo, hi);
+    if (lane < 4) {
+      dig_sm[2 * lane] = lo;
+      dig_sm[2 * lane + 1] = hi;
+    }
+    __syncwarp();
+    // digest (little-endian 256-bit D) -> D R mod p = sum_i D_i (R^2 2^(32 L i)) / R
+    if (lane < kParts) v = ld_fe<L>(dig_sm + lane * L);
+  }
+  if (claim && lane >= 8 && lane <= 8 + d) v = ld_fe<L>(g_sm + (lane - 8) * L);
+  Fe<L> x = fe_mul_any(con, v, F);
   Fe<L> r;
   if (A.mode == kChallengeSha3) {
-    const char dom[] = "zkduel:field-sweep:v1";
-    constexpr int kDom = sizeof(dom) - 1;
-    const int nwords = 1 + (d + 1) * L;
-    if (lane < kDom) msg[lane] = static_cast<uint8_t>(dom[lane]);
-    for (int i = lane; i < nwords; i += 32) {
-      const uint32_t w = i == 0 ? static_cast<uint32_t>(j) : g_sm[i - 1];
-      msg[kDom + 4 * i + 0] = static_cast<uint8_t>(w);
-      msg[kDom + 4 * i + 1] = static_cast<uint8_t>(w >> 8);
-      msg[kDom + 4 * i + 2] = static_cast<uint8_t>(w >> 16);
-      msg[kDom + 4 * i + 3] = static_cast<uint8_t>(w >> 24);
-    }
-    __syncwarp();
-    uint32_t dig[8];
-    sha3_256_warp(msg, kDom + 4 * nwords, dig);
-    // digest (little-endian 256-bit D) -> D R mod p = sum_i (w_i mod p) * R^2 2^(32 i) / R
-    Fe<L> term = fe_zero<L>();
-    if (lane < 8) {
-      uint32_t w = dig[0];
+    Fe<L> y = x;
 #pragma unroll
-      for (int i = 1; i < 8; ++i)
-        if (lane == i) w = dig[i];
-      if (fc.p_small) w %= fc.p_small;
-      Fe<L> wf = fe_zero<L>();
-      wf.w[0] = w;
-      term = fe_mul(wf, fc_get<L>(fc.kdig[lane]), F);
-    }
-#pragma unroll
-    for (int off = 4; off > 0; off >>= 1) term = fe_add(term, fe_shfl_down(term, off), F);
-    r = fe_shfl(term, 0);
-    if (lane == 0) st_fe<L>(A.st.chals + j * L, r);
+    for (int off = kParts / 2; off > 0; off >>= 1) y = fe_add(y, fe_shfl_down(y, off), F);
+    r = fe_shfl(y, 0);
   } else if (A.mode == kChallengeFixed) {
     r = fc_get<L>(fc.one);
-    if (lane == 0) st_fe<L>(A.st.chals + j * L, r);
   } else {
     r = ld_fe_cg<L>(A.st.chals + j * L);
   }
-  // 3. g_j(r_j): the next round's claim, and in the last round the final claim
-  const bool last_round = j == A.num_rounds - 1;
-  if (A.want_claim || last_round) {
-    const Fe<L> gr = lagrange_at<L, K>(g_sm, d, r, fc, F);
-    if (lane == 0) st_fe<L>(last_round ? A.st.finals : A.st.claim, gr);
+  if (lane == 0) {
+    if (A.mode != kChallengeExplicit) st_fe<L>(A.st.chals + j * L, r);
+    st_fe<L>(r_sm, r);
   }
-  // 4. last round: f_k(r) per table
-  if (last_round) {
-    const uint32_t* tab = A.fold ? A.dst : A.src;  // T_{n-1}: 2 entries per plane
-    for (int k = lane; k < E.num_vars; k += 32) {
-      Fe<L> e, o;
+  if (!claim) return;
+  // g_j(r_j), the next round's claim or the final claim: sum_t w_t prod_{s != t} (r - s), the
+  // products of all factors but one by doubling over the lanes of an octet (lane i the factor
+  // r - i, or 1): pairs, then quads beside "all but mine" of a quad, then the other quad's.
+  const int i8 = lane & 7;
+  Fe<L> u = fc_get<L>(fc.one);
+  if (i8 <= d) u = fe_sub(r, fc_get<L>(fc.pts[i8]), F);
+  const Fe<L> u1 = fe_shfl_xor(u, 1);
+  const Fe<L> p2 = fe_mul(u, u1, F);
+  const Fe<L> p2o = fe_shfl_xor(p2, 2);
+  const Fe<L> p4 = fe_mul(lane < 8 ? p2 : u1, p2o, F);  // lanes 0..7 the quad, 8..15 all but mine of it
+  Fe<L> q = p4;
+  if (d >= 4) q = fe_mul(p4, fe_shfl(p4, (lane & 3) | (~lane & 4)), F);  // times the other quad (lanes 0..7)
+  const bool mine = lane >= 8 && lane <= 8 + d;
+  Fe<L> term = fe_mul(q, x, F);
+  if (!mine) term = fe_zero<L>();
 #pragma unroll
-      for (int l = 0; l < L; ++l) {
-        e.w[l] = __ldcg(tab + (k * L + l) * 2 + 0);
-        o.w[l] = __ldcg(tab + (k * L + l) * 2 + 1);
-      }
-      const Fe<L> f = fe_add(e, fe_mul(r, fe_sub(o, e, F), F), F);
-      st_fe<L>(A.st.finals + (1 + k) * L, f);
-    }
+  for (int off = 4; off > 0; off >>= 1) term = fe_add(term, fe_shfl_down(term, off), F);
+  if (lane == 8) st_fe<L>(last_round ? A.st.finals : A.st.claim, term);
+  // last round: f_k(r) per table
+  if (last_round) {
+    const Fe<L> f = fe_add(e, fe_mul(r, fe_sub(o, e, F), F), F);
+    if (lane < E.num_vars) st_fe<L>(A.st.finals + (1 + lane) * L, f);
+  }
+}
+
+// The round's integer sums (s_sm) to g_j and its end; every thread of the block calls.
+template <int L, int K>
+__device__ __forceinline__ void finish_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F,
+                                             const uint64_t* s_sm, uint32_t* g_sm, uint32_t* r_sm) {
+  const int d = E.degree;
+  if (threadIdx.x < 32) {
+    sums_to_points<L, K>(s_sm, d, *A.fc, F, g_sm);
+    if (A.skip1 && !A.ext_out) point1_from_claim<L, K>(A.st.claim, g_sm, F);
+  }
+  __syncthreads();
+  if (A.ext_out) {
+    for (int i = threadIdx.x; i < (d + 1) * L; i += blockDim.x) A.ext_out[i] = g_sm[i];
+  } else {
+    finalize_round<L, K>(A, E, F, g_sm, r_sm);
   }
 }
 
@@ -835,7 +971,8 @@ __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
     round_kernel(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ __align__(16) uint8_t msg[3 * 136];
+  __shared__ uint64_t s_sm[kMaxPoints * L];
+  __shared__ uint32_t r_sm[L];
   __shared__ int is_last;
 
   const int tid = threadIdx.x;
@@ -853,26 +990,11 @@ __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
   process_pairs<L, K, DMAX, SHAPE>(A.src, A.dst, A.src_len, A.fold != 0, r_prev, E, sv, sd,
                                    static_cast<uint64_t>(blockIdx.x) * nthr + tid, A.pairs, stride, A.skip1 != 0, acc, F);
 
-  // block partial -> global; the last block reduces all partials
+  // the block's integer sums to the grid's; the last block finalises the round
   __syncthreads();
-  block_reduce<L, K, DMAX + 1>(acc, d, smem, g_sm, F);
-  for (int i = tid; i < (d + 1) * L; i += nthr) A.partials[static_cast<uint64_t>(blockIdx.x) * kMaxPoints * L + i] = g_sm[i];
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = (atomicAdd(A.st.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  reduce_partials<L, K, DMAX + 1>(A.partials, 0, gridDim.x, d, smem, g_sm, F);
-  if (A.ext_out) {
-    for (int i = tid; i < (d + 1) * L; i += nthr) A.ext_out[i] = g_sm[i];
-  } else if (tid < 32) {
-    finalize_round<L, K>(A, E, F, g_sm, msg);
-  }
-  if (tid == 0) {
-    __threadfence();
-    *A.st.counter = 0;
-  }
+  warp_sums<L, DMAX + 1>(acc, d, smem);
+  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, s_sm, &is_last)) return;
+  finish_round<L, K>(A, E, F, s_sm, g_sm, r_sm);
 }
 
 // ------------------------------------------------------------------------------ resume folds
@@ -911,7 +1033,7 @@ __global__ void __launch_bounds__(256) fold_kernel(const uint32_t* __restrict__ 
 // persistent kernel whose blocks pull (proof round, tile of pairs) items from a device work
 // queue (an atomic counter over the tick's item list). Every item leaves one partial in its
 // round's partial slots; the block that finishes the last item of a proof's round (per-proof
-// atomic ticket) reduces that round's partials and finalises it -- SHA3 challenge included --
+// atomic ticket) reads that round's sums and finalises it -- SHA3 challenge included --
 // while the other blocks go on with other proofs' items. A round's items may be spread over
 // several ticks (the served prover slices large rounds): the ticket counts to the round's
 // item total, whichever tick its last item runs in.
@@ -924,7 +1046,6 @@ __global__ void __launch_bounds__(256) fold_kernel(const uint32_t* __restrict__ 
 struct BatchRound {
   RoundArgs args;        // this proof's round (src/dst/len/pairs/round/fold/mode/flags/fc/state)
   const ExprDev* expr;   // this proof's expression
-  uint32_t* partials;    // the round's partial slots: [round_items][kMaxPoints][L]
   int32_t first_item;    // this tick's items of the round: [first_item, first_item + num_items)
   int32_t num_items;
   int32_t item_base;     // round-relative index of this tick's first item of the round
@@ -957,7 +1078,8 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
     batch_round_kernel(const BatchTickArgs T, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ __align__(16) uint8_t msg[3 * 136];
+  __shared__ uint64_t s_sm[kMaxPoints * L];
+  __shared__ uint32_t r_sm[L];
   __shared__ __align__(16) ExprDev E;
   __shared__ __align__(16) BatchRound R;
   __shared__ const ExprDev* cur_expr;
@@ -999,28 +1121,16 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
 #pragma unroll
       for (int t = 0; t <= DMAX; ++t) acc[t] = fe_zero<L>();
       Fe<L> r_prev = fe_zero<L>();
-      if (R.args.fold) r_prev = ld_fe_cg<L>(R.args.st.chals + (R.args.round - 1) * L);
+      if (R.args.fold) r_prev = k == 0 ? ld_fe_cg<L>(R.args.st.chals + (R.args.round - 1) * L) : ld_fe<L>(r_sm);
       const uint64_t q0 = k == 0 ? I.start : 0, q1 = k == 0 ? I.start + I.count : R.args.pairs;
       process_pairs<L, K, DMAX>(R.args.src, R.args.dst, R.args.src_len, R.args.fold != 0, r_prev, E, sv, sd, q0 + tid,
                                 q1, nthr, R.args.skip1 != 0, acc, F);
       __syncthreads();
-      block_reduce<L, K, DMAX + 1>(acc, d, smem, g_sm, F);
-      if (k == 0) {
-        uint32_t* slot = R.partials + static_cast<uint64_t>(R.item_base + (it - R.first_item)) * kMaxPoints * L;
-        for (int i = tid; i < (d + 1) * L; i += nthr) slot[i] = g_sm[i];
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) is_last = (atomicAdd(R.args.st.counter, 1u) == static_cast<uint32_t>(R.round_items - 1));
-        __syncthreads();
-        if (!is_last) break;
-        __threadfence();
-        reduce_partials<L, K, DMAX + 1>(R.partials, 0, R.round_items, d, smem, g_sm, F);
-      }
-      if (tid < 32) finalize_round<L, K>(R.args, E, F, g_sm, msg);
-      if (k == 0 && tid == 0) {
-        __threadfence();
-        *R.args.st.counter = 0;
-      }
+      warp_sums<L, DMAX + 1>(acc, d, smem);
+      const uint32_t part = k == 0 ? static_cast<uint32_t>(R.item_base + (it - R.first_item)) : 0;
+      const uint32_t parts = k == 0 ? static_cast<uint32_t>(R.round_items) : 1;
+      if (!grid_sums<L>(smem, d, part, parts, R.args.sums, R.args.st.counter, s_sm, &is_last)) break;
+      finish_round<L, K>(R.args, E, F, s_sm, g_sm, r_sm);
       if (k == R.tail_rounds) break;
       __syncthreads();  // the finalisation read R.args; r_j and T_j are visible to the block
       if (tid == 0) {   // round j + 1 of the same proof

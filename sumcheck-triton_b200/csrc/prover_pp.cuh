@@ -49,8 +49,8 @@ __device__ __forceinline__ PointPlan point_plan(int d, bool skip1) {
 // to kmax tables (a slot is 2 kmax L words; a round with 1-lane groups uses the slots it has,
 // the other lanes idle), and at least the reduction scratch, which reuses them.
 __host__ __device__ constexpr int pp_smem_words(int threads, int kmax, int L) {
-  return (threads / 2) * 2 * kmax * L > (threads / 32) * kMaxPoints * L ? (threads / 2) * 2 * kmax * L
-                                                                         : (threads / 32) * kMaxPoints * L;
+  return (threads / 2) * 2 * kmax * L > reduce_scratch_words(threads, L) ? (threads / 2) * 2 * kmax * L
+                                                                         : reduce_scratch_words(threads, L);
 }
 
 // Pairs a block holds at once: one per group, as far as the dynamic shared memory goes.
@@ -170,52 +170,20 @@ __device__ __forceinline__ void pp_process_pairs(const uint32_t* src, uint32_t* 
   }
 }
 
-// Block sum of every point: lane gi of each group holds point pts[gi]. The sums land in
-// red_out[t * L + l] for t = 0..d (zero for point 1 when it was not evaluated).
+// This warp's sum of every point into its row of scratch (prover.cuh: warp_sums): lane gi of
+// each group holds point pts[gi]. Point 1 under skip1 is zero.
 template <int L, int K>
-__device__ __forceinline__ void pp_block_reduce(Fe<L> acc, const PointPlan& P, int d, uint32_t* scratch,
-                                                uint32_t* red_out, const FieldParams<L, K>& F) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+__device__ __forceinline__ void pp_warp_sums(Fe<L> acc, const PointPlan& P, uint32_t* scratch, const FieldParams<L, K>& F) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = P.G;
   // sum over the groups of the warp (lanes with equal lane % G)
   for (int off = 16; off >= G; off >>= 1) acc = fe_add(acc, fe_shfl_down(acc, off), F);
-  __syncthreads();  // the pair slots are free again
-  // zero, then this warp's point sums (point 1 under skip1 and points past d stay zero)
-  if (lane < kMaxPoints) st_fe<L>(scratch + (warp * kMaxPoints + lane) * L, fe_zero<L>());
+  uint64_t* row = reinterpret_cast<uint64_t*>(scratch) + warp * kMaxPoints * L;
+  for (int i = lane; i < kMaxPoints * L; i += 32) row[i] = 0;
   __syncwarp();
-  if (lane < G && lane < P.npts) st_fe<L>(scratch + (warp * kMaxPoints + P.pts[lane]) * L, acc);
-  __syncthreads();
-  if (warp == 0) {
-    for (int t = 0; t <= d; ++t) {
-      Fe<L> v = lane < nwarps ? ld_fe<L>(scratch + (lane * kMaxPoints + t) * L) : fe_zero<L>();
+  if (lane < G && lane < P.npts) {
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = fe_add(v, fe_shfl_down(v, off), F);
-      if (lane == 0) st_fe<L>(red_out + t * L, v);
-    }
-  }
-  __syncthreads();
-}
-
-// Sums partial slots [0, count) into g_sm[t * L + l], one point at a time (one accumulator
-// per lane); block-wide.
-template <int L, int K>
-__device__ __forceinline__ void pp_reduce_partials(const uint32_t* partials, uint64_t count, int d, uint32_t* scratch,
-                                                   uint32_t* g_sm, const FieldParams<L, K>& F) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  for (int t = 0; t <= d; ++t) {
-    Fe<L> acc = fe_zero<L>();
-    for (uint64_t b = tid; b < count; b += blockDim.x) acc = fe_add(acc, ld_fe_cg<L>(partials + (b * kMaxPoints + t) * L), F);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc = fe_add(acc, fe_shfl_down(acc, off), F);
-    if (lane == 0) st_fe<L>(scratch + warp * L, acc);
-    __syncthreads();
-    if (warp == 0) {
-      Fe<L> v = lane < nwarps ? ld_fe<L>(scratch + lane * L) : fe_zero<L>();
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v = fe_add(v, fe_shfl_down(v, off), F);
-      if (lane == 0) st_fe<L>(g_sm + t * L, v);
-    }
-    __syncthreads();
+    for (int l = 0; l < L; ++l) row[P.pts[lane] * L + l] = acc.w[l];
   }
 }
 
@@ -225,9 +193,9 @@ template <int L, int K>
 __global__ void __launch_bounds__(128, 4) round_kernel_pp(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ __align__(16) uint8_t msg[3 * 136];
+  __shared__ uint64_t s_sm[kMaxPoints * L];
+  __shared__ uint32_t r_sm[L];
   __shared__ int is_last;
-  const int tid = threadIdx.x;
   const int d = E.degree;
   const PointPlan P = point_plan(d, A.skip1 != 0);
   Fe<L> acc = fe_zero<L>();
@@ -237,25 +205,10 @@ __global__ void __launch_bounds__(128, 4) round_kernel_pp(const RoundArgs A, con
   pp_process_pairs<L, K>(A.src, A.dst, A.src_len, A.fold != 0, r_prev, E, P, smem, slots,
                          static_cast<uint64_t>(blockIdx.x) * slots, A.pairs,
                          static_cast<uint64_t>(slots) * gridDim.x, acc, F);
-  pp_block_reduce<L, K>(acc, P, d, smem, g_sm, F);
-  for (int i = tid; i < (d + 1) * L; i += blockDim.x)
-    A.partials[static_cast<uint64_t>(blockIdx.x) * kMaxPoints * L + i] = g_sm[i];
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = (atomicAdd(A.st.counter, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  pp_reduce_partials<L, K>(A.partials, gridDim.x, d, smem, g_sm, F);
-  if (A.ext_out) {
-    for (int i = tid; i < (d + 1) * L; i += blockDim.x) A.ext_out[i] = g_sm[i];
-  } else if (tid < 32) {
-    finalize_round<L, K>(A, E, F, g_sm, msg);
-  }
-  if (tid == 0) {
-    __threadfence();
-    *A.st.counter = 0;
-  }
+  __syncthreads();  // the pair slots are free again
+  pp_warp_sums<L, K>(acc, P, smem, F);
+  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, s_sm, &is_last)) return;
+  finish_round<L, K>(A, E, F, s_sm, g_sm, r_sm);
 }
 
 }  // namespace sc

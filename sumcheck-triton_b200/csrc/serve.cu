@@ -98,7 +98,6 @@ struct ServeRequest {
   StateOffsets so{};
   char* block = nullptr;
   uint32_t* state = nullptr;
-  uint32_t* partials = nullptr;
   ExprDev* expr_dev = nullptr;
   uint32_t* tables = nullptr;
   uint32_t* fold_a = nullptr;
@@ -130,18 +129,15 @@ struct TickSlot {
 
 // Layout of one request's device block. Offsets in bytes, every part kAlign-aligned.
 struct BlockLayout {
-  size_t state, partials, expr, rounds, tables, fold_a, fold_b, total;
+  size_t state, expr, rounds, tables, fold_a, fold_b, total;
 };
 
-inline BlockLayout block_layout(int n, int K, int L, int tile_pairs) {
+inline BlockLayout block_layout(int n, int K, int L) {
   const uint64_t N = uint64_t{1} << n;
-  const uint64_t items0 = ((N >> 1) + tile_pairs - 1) / tile_pairs;
   BlockLayout b;
   size_t off = 0;
   b.state = off;
-  off = align_up(off + state_offsets(n, K, L).total_words * 4, kAlign);
-  b.partials = off;
-  off = align_up(off + std::max<uint64_t>(items0, 1) * kMaxPoints * L * 4, kAlign);
+  off = align_up(off + state_and_sums_bytes(state_offsets(n, K, L), L), kAlign);
   b.expr = off;
   off = align_up(off + sizeof(ExprDev), kAlign);
   b.rounds = off;
@@ -257,6 +253,7 @@ void round_args(const sc_server* S, const ServeRequest& R, int t, RoundArgs& A) 
   A.st.finals = s + o.finals;
   A.st.claim0 = s + o.claim0;
   A.st.claim = s + o.claim;
+  A.sums = state_sums(s, o);
 }
 
 // Worker-side completion: results into the request, status published under the lock.
@@ -355,10 +352,9 @@ int retire_ticks(sc_server* S, bool block) {
 // block per tile, so the small requests' higher-priority launches take SMs as these blocks
 // retire), result copy, free, completion event -- all ordered on the lane.
 int issue_large(sc_server* S, ServeRequest* R) {
+  SC_CUDA(cudaMemsetAsync(R->state, 0, state_and_sums_bytes(R->so, S->L), S->lane));
   if (R->first)
     SC_CUDA(cudaMemcpyAsync(R->state, R->resume_state.data(), R->so.total_words * 4, cudaMemcpyHostToDevice, S->lane));
-  else
-    SC_CUDA(cudaMemsetAsync(R->state, 0, R->so.total_words * 4, S->lane));
   ExprDev& E = S->expr_host[R->slot];
   build_expr(S, R->expr, E);
   SC_CUDA(cudaMemcpyAsync(R->expr_dev, &E, sizeof(ExprDev), cudaMemcpyHostToDevice, S->lane));
@@ -389,7 +385,6 @@ int issue_large(sc_server* S, ServeRequest* R) {
     tiles[t] = tile;
     const uint64_t items = (B.args.pairs + tile - 1) / tile;
     B.expr = R->expr_dev;
-    B.partials = R->partials;
     B.first_item = 0;
     B.num_items = static_cast<int32_t>(items);
     B.item_base = 0;
@@ -453,7 +448,7 @@ int admit(sc_server* S) {
     ServeRequest* R = S->waiting.front();
     if (S->admitted_bytes + R->footprint > S->budget) break;  // arrival order: no overtaking
     S->waiting.pop_front();
-    const BlockLayout b = block_layout(R->n, R->K, S->L, S->tile_pairs);
+    const BlockLayout b = block_layout(R->n, R->K, S->L);
     const uint64_t items0 = (((uint64_t{1} << R->n) >> (R->first + 1)) + S->tile_pairs - 1) / S->tile_pairs;
     R->large = static_cast<int64_t>(items0) > S->large_items;
     cudaStream_t st = R->large ? S->lane : S->stream;
@@ -468,7 +463,6 @@ int admit(sc_server* S) {
     }
     R->block = static_cast<char*>(p);
     R->state = reinterpret_cast<uint32_t*>(R->block + b.state);
-    R->partials = reinterpret_cast<uint32_t*>(R->block + b.partials);
     R->expr_dev = reinterpret_cast<ExprDev*>(R->block + b.expr);
     R->rounds_dev = reinterpret_cast<BatchRound*>(R->block + b.rounds);
     R->tables = reinterpret_cast<uint32_t*>(R->block + b.tables);
@@ -485,11 +479,10 @@ int admit(sc_server* S) {
       int rc = issue_large(S, R);
       if (rc) return rc;
     } else {
+      SC_CUDA(cudaMemsetAsync(R->state, 0, state_and_sums_bytes(R->so, S->L), S->stream));
       if (R->first)
         SC_CUDA(cudaMemcpyAsync(R->state, R->resume_state.data(), R->so.total_words * 4, cudaMemcpyHostToDevice,
                                 S->stream));
-      else
-        SC_CUDA(cudaMemsetAsync(R->state, 0, R->so.total_words * 4, S->stream));
       ExprDev& E = S->expr_host[R->slot];
       build_expr(S, R->expr, E);
       SC_CUDA(cudaMemcpyAsync(R->expr_dev, &E, sizeof(ExprDev), cudaMemcpyHostToDevice, S->stream));
@@ -552,7 +545,6 @@ int issue_tick(sc_server* S, bool* issued) {
     std::memset(&B, 0, sizeof(B));
     round_args(S, *R, R->round, B.args);
     B.expr = R->expr_dev;
-    B.partials = R->partials;
     B.first_item = static_cast<int32_t>(items[c].size());
     B.num_items = static_cast<int32_t>(give);
     B.item_base = static_cast<int32_t>(R->issued);
@@ -792,7 +784,7 @@ void worker_main(sc_server* S) {
 
 size_t request_footprint(const sc_server* S, int n, int K) {
   if (S->policy == SC_SERVE_FIFO_PLAIN) return align_up(static_cast<size_t>(K) * S->L * (size_t{1} << n) * 4, kAlign);
-  return block_layout(n, K, S->L, S->tile_pairs).total;
+  return block_layout(n, K, S->L).total;
 }
 
 int check_request(const sc_server* S, const sc_expr* expr, int num_rounds) {

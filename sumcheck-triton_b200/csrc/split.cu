@@ -25,7 +25,7 @@ template <int L, int K>
 __global__ void split_commit_kernel(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F,
                                     const uint32_t* parts, int world) {
   __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ __align__(16) uint8_t msg[3 * 136];
+  __shared__ uint32_t r_sm[L];
   const int lane = threadIdx.x;
   const int d = E.degree;
   if (lane <= d) {
@@ -34,7 +34,8 @@ __global__ void split_commit_kernel(const RoundArgs A, const ExprDev E, const Fi
     st_fe<L>(g_sm + lane * L, acc);
   }
   __syncwarp();
-  finalize_round<L, K>(A, E, F, g_sm, msg);
+  if (A.skip1) point1_from_claim<L, K>(A.st.claim, g_sm, F);
+  finalize_round<L, K>(A, E, F, g_sm, r_sm);
 }
 
 }  // namespace
@@ -52,7 +53,7 @@ struct sc_split {
   int next = 0;                // next round to run
   bool committed = true;       // the last run round was committed
   StateOffsets so{};
-  DevBuf fold_a, fold_b, partials, state, ext, parts, tail, tail_a, tail_b;
+  DevBuf fold_a, fold_b, state, ext, parts, tail, tail_a, tail_b;
   uint32_t* host = nullptr;    // pinned staging
   size_t host_words = 0;
   int threads = 256, grid_max = 1;
@@ -85,7 +86,7 @@ struct SplitSetup {
   static int run(sc_split* S) {
     int threads = kernel_threads(L);
     if (S->E.shape != kShapeGeneric && D == 4) {
-      S->smem = shape_round_smem_bytes(L, K, S->E.shape, threads);  // block_reduce scratch (+ the pair stage)
+      S->smem = shape_round_smem_bytes(L, K, S->E.shape, threads);  // reduction scratch (+ the pair stage)
     } else {
       const int per_thread = round_smem_words_per_thread(S->K, L) * 4;
       while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
@@ -135,8 +136,8 @@ void split_args(const sc_split* S, int j, RoundArgs& A) {
   A.num_rounds = S->n;
   A.mode = S->mode;
   A.fc = S->field->dev;
-  A.partials = static_cast<uint32_t*>(S->partials.p);
   uint32_t* st = static_cast<uint32_t*>(S->state.p);
+  A.sums = state_sums(st, S->so);
   A.st.counter = st + S->so.counter;
   A.st.status = st + S->so.status;
   A.st.checksum = reinterpret_cast<uint64_t*>(st + S->so.checksum);
@@ -225,8 +226,7 @@ int sc_split_create(sc_ctx* ctx, const sc_field* field, const sc_expr* expr, int
   int rc = dispatch<SplitSetup>(S->L, S->kind, S->dclass, S);
   if (!rc) rc = ensure(ctx, S->fold_a, (S->local_rounds >= 2 ? KL * (S->C / 2) : 1) * 4);
   if (!rc) rc = ensure(ctx, S->fold_b, (S->local_rounds >= 3 ? KL * (S->C / 4) : 1) * 4);
-  if (!rc) rc = ensure(ctx, S->partials, static_cast<size_t>(S->grid_max) * kMaxPoints * S->L * 4);
-  if (!rc) rc = ensure(ctx, S->state, S->so.total_words * 4);
+  if (!rc) rc = ensure(ctx, S->state, state_and_sums_bytes(S->so, S->L));
   if (!rc) rc = ensure(ctx, S->ext, kMaxPoints * kMaxLimbs * 4);
   if (!rc) rc = ensure(ctx, S->parts, W * kMaxPoints * kMaxLimbs * 4);
   if (!rc) rc = ensure(ctx, S->tail, KL * std::max<size_t>(W, 2) * 4);
@@ -234,7 +234,7 @@ int sc_split_create(sc_ctx* ctx, const sc_field* field, const sc_expr* expr, int
   if (!rc) rc = ensure(ctx, S->tail_b, KL * std::max<size_t>(W / 4, 2) * 4);
   if (!rc) rc = stage(S, std::max<size_t>({S->so.total_words, W * KL, W * kMaxPoints * kMaxLimbs, 2 * KL + 64}));
   if (!rc) {
-    const cudaError_t e = cudaMemsetAsync(S->state.p, 0, S->so.total_words * 4, ctx->stream);
+    const cudaError_t e = cudaMemsetAsync(S->state.p, 0, state_and_sums_bytes(S->so, S->L), ctx->stream);
     if (e != cudaSuccess) rc = fail(SC_ERR_CUDA, "state: %s", cudaGetErrorString(e));
   }
   if (rc) {
@@ -363,7 +363,7 @@ int sc_split_destroy(sc_split* S) {
   if (!S) return SC_OK;
   cudaSetDevice(S->ctx->device);
   cudaStreamSynchronize(S->ctx->stream);
-  for (DevBuf* b : {&S->fold_a, &S->fold_b, &S->partials, &S->state, &S->ext, &S->parts, &S->tail, &S->tail_a, &S->tail_b})
+  for (DevBuf* b : {&S->fold_a, &S->fold_b, &S->state, &S->ext, &S->parts, &S->tail, &S->tail_a, &S->tail_b})
     if (b->p) cudaFree(b->p);
   if (S->host) cudaFreeHost(S->host);
   delete S;
