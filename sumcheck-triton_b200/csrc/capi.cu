@@ -453,6 +453,7 @@ int sc_field_init(int limbs, const uint32_t* modulus, uint32_t nprime, sc_field*
   std::memcpy(C.one, x, 4 * limbs);
   for (int i = 0; i < 32 * limbs; ++i) hf.dbl(x, x);
   std::memcpy(C.r2, x, 4 * limbs);
+  hf.mul(C.r2, C.r2, C.r3);
   for (int w = 0; w < 8; ++w) {
     std::memcpy(C.kdig[w], x, 4 * limbs);
     for (int i = 0; i < 32; ++i) hf.dbl(x, x);

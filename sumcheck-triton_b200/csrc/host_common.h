@@ -257,12 +257,14 @@ inline int mul_cost(int L, int K) {
 inline int add_cost(int L) { return 3 * L + 4; }
 
 // Whether a term of length len in an expression of degree d is cheaper evaluated at points
-// 0..len and extrapolated by forward differences than evaluated at every point 0..d.
+// 0..len and extrapolated by forward differences than evaluated at every finite point 0..d - 1
+// (a shorter term has no part in the leading coefficient that stands for point d).
 inline bool extrapolate_term(int len, int d, int L, int K) {
-  if (len >= d) return false;
+  const int fin = d - 1;
+  if (len >= fin) return false;
   const int m = mul_cost(L, K), a = add_cost(L);
-  const int direct = (len - 1) * (d + 1) * m + len * d * a;
-  const int extrap = (len - 1) * (len + 1) * m + len * len * a + (len * (len + 1) / 2 + d * len) * a;
+  const int direct = (len - 1) * (fin + 1) * m + len * fin * a;
+  const int extrap = (len - 1) * (len + 1) * m + len * len * a + (len * (len + 1) / 2 + fin * len) * a;
   return extrap < direct;
 }
 

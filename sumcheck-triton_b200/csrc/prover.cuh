@@ -6,10 +6,11 @@
 //      (one 128-bit load per limb plane), folds them with r_{j-1} into the pair
 //      (T_j[2i], T_j[2i+1]) and writes that pair back (the fold of the previous round,
 //      reference field_sumcheck.cu:677-694, fused into this round's read);
-//   2. evaluate: extends every table's pair to t = 0..d (v(t) = v(t-1) + (o - e); reference
+//   2. evaluate: extends every table's pair to t = 0..d - 1 (v(t) = v(t-1) + (o - e); reference
 //      field_sumcheck.cu:326-348) and evaluates the constraint at each point
-//      (field_sumcheck.cu:389-590), accumulating d+1 sums per thread (see eval_pair for the
-//      exact-arithmetic shortcuts: extrapolated low-degree terms, g(1) from the claim);
+//      (field_sumcheck.cu:389-590) and, in the place of point d, its leading coefficient,
+//      accumulating d+1 sums per thread (see eval_pair for the exact-arithmetic shortcuts:
+//      extrapolated low-degree terms, g(1) from the claim);
 //   3. reduce: the point sums are summed word by word as integers -- over the warp, the block
 //      (shared memory) and the grid (64-bit atomic adds) -- with no modular arithmetic until
 //      the last block to finish (atomic ticket) reads (d + 1) L integers and reduces them
@@ -61,6 +62,7 @@ struct FieldConsts {
   uint32_t p_small;                          // p if p < 2^32, else 0
   uint32_t one[kMaxLimbs];                   // R mod p
   uint32_t r2[kMaxLimbs];                    // R^2 mod p
+  uint32_t r3[kMaxLimbs];                    // R^3 mod p
   uint32_t pts[kMaxPoints][kMaxLimbs];       // Montgomery image of t = 0..7
   uint32_t kdig[8][kMaxLimbs];               // R^2 2^(32 i) mod p: digest word i
   uint32_t lag[kMaxPoints][kMaxPoints][kMaxLimbs];  // lag[d][t] = 1 / prod_{s<=d, s!=t} (t - s)
@@ -215,13 +217,14 @@ __device__ __forceinline__ Fe<L> lz_add_or_sub(const Fe<L>& acc, const Fe<L>& x,
   return neg ? lz_sub<LZ>(acc, x, F) : lz_add<LZ>(acc, x, F);
 }
 
-// One pair: acc[t] += expression at point t, for t = 0..d (t = 1 skipped when skip1).
+// One pair: acc[t] += expression at point t, for the finite points t (0..d - 1, or 0 and 1 for
+// d = 1; 1 skipped when skip1), and acc[DMAX] += its coefficient of t^d (make_point_weights).
 // The values and differences of every table are in shared memory (this thread's slots).
 //
 // A term of len factors is a polynomial of degree len in t. Evaluated at points 0..last
-// (last = d, or len when the host marked the term for extrapolation), each point costs len-1
+// (the last finite point, or len when the host marked the term for extrapolation), each point costs len-1
 // products: the factors' values are stepped point to point by one addition of the
-// difference. An extrapolated term's points len+1..d come from its forward differences
+// difference. An extrapolated term's further points come from its forward differences
 // (len(len+1)/2 subtractions, then len additions per step) -- exact, since the term is a
 // polynomial of degree len; the host marks a term only where that is cheaper than the
 // products it replaces. With skip1, point 1 of a directly evaluated term is never formed.
@@ -230,15 +233,17 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, const uint32_t* sv, 
                                           bool skip1, Fe<L> (&acc)[DMAX + 1], const FieldParams<L, K>& F) {
   constexpr bool LZ = lazy_generic<L, K>();
   const int d = E.degree;
+  const int fin = d >= 2 ? d - 1 : 1;  // last finite point
   for (int i = 0; i < E.num_terms; ++i) {
     const int off = E.term_off[i];
     const int len = E.term_len[i];
     const int kind = E.coeff_kind[i];
     const bool extrap = E.term_extrap[i] != 0;
-    const int last = extrap ? len : d;
+    const bool full = len == d && d >= 2;
+    const int last = extrap ? len : fin;
     const bool skip_t1 = skip1 && !extrap;
     const bool neg = kind == kCoeffMinus || (kind == kCoeffSmall && E.coeff_small[i] < 0);
-    Fe<L> prod[DMAX + 1];
+    Fe<L> prod[DMAX], lead;
     {
       const int k0 = E.flat[off];
       Fe<L> v = sm_get<L>(sv, k0, tid, nthr);
@@ -255,8 +260,9 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, const uint32_t* sv, 
         v = fe_mul(v, cm, F);
         df = fe_mul(df, cm, F);
       }
+      lead = df;
 #pragma unroll
-      for (int t = 0; t <= DMAX; ++t) {
+      for (int t = 0; t < DMAX; ++t) {
         if (t > last) break;
         prod[t] = v;
         if (t < last) v = lz_add_c<LZ>(v, df, F);
@@ -266,36 +272,38 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, const uint32_t* sv, 
       const int k = E.flat[off + f];
       Fe<L> v = sm_get<L>(sv, k, tid, nthr);
       const Fe<L> df = sm_get<L>(sd, k, tid, nthr);
+      if (full) lead = lz_mul<LZ>(lead, df, F);
 #pragma unroll
-      for (int t = 0; t <= DMAX; ++t) {
+      for (int t = 0; t < DMAX; ++t) {
         if (t > last) break;
         if (!(skip_t1 && t == 1)) prod[t] = lz_mul<LZ>(prod[t], v, F);
         if (t < last) v = lz_add_c<LZ>(v, df, F);
       }
     }
+    if (full) acc[DMAX] = lz_add_or_sub<LZ>(acc[DMAX], lead, neg, F);
 #pragma unroll
-    for (int t = 0; t <= DMAX; ++t) {
+    for (int t = 0; t < DMAX; ++t) {
       if (t > last) break;
       if (skip1 && t == 1) continue;
       acc[t] = lz_add_or_sub<LZ>(acc[t], prod[t], neg, F);
     }
-    if (extrap && len < d) {
+    if (extrap && len < fin) {
       // forward differences at 0, in place: prod[m] = Delta^m p(0)
 #pragma unroll
-      for (int m = 1; m <= DMAX; ++m) {
+      for (int m = 1; m < DMAX; ++m) {
         if (m > len) break;
 #pragma unroll
-        for (int t = DMAX; t >= 1; --t) {
+        for (int t = DMAX - 1; t >= 1; --t) {
           if (t > len || t < m) continue;
           prod[t] = lz_sub<LZ>(prod[t], prod[t - 1], F);
         }
       }
       // step forward: after s steps prod[0] = p(s)
 #pragma unroll
-      for (int s = 1; s <= DMAX; ++s) {
-        if (s > d) break;
+      for (int s = 1; s < DMAX; ++s) {
+        if (s > fin) break;
 #pragma unroll
-        for (int m = 0; m < DMAX; ++m) {
+        for (int m = 0; m < DMAX - 1; ++m) {
           if (m >= len) break;
           prod[m] = lz_add<LZ>(prod[m], prod[m + 1], F);
         }
@@ -321,6 +329,29 @@ __device__ __forceinline__ Fe<L> shape_value(const Fe<L> (&v)[6], const FieldPar
                                              std::integral_constant<int, kShapeAbcg>) {
   const Fe<L> s = fe_add(fe_mul(fe_mul(v[0], v[1], F), v[2], F), fe_mul(v[4], v[5], F), F);
   return fe_mul(v[3], s, F);
+}
+
+// Their coefficients of t^4 from the tables' differences: the term of full degree alone.
+template <int L, int K>
+__device__ __forceinline__ Fe<L> shape_lead(const Fe<L> (&d)[9], const FieldParams<L, K>& F,
+                                            std::integral_constant<int, kShapeZerocheck>) {
+  return fe_mul(fe_mul(d[2], d[1], F), fe_mul(d[4], d[5], F), F);  // F X1 X2 M
+}
+
+template <int L, int K>
+__device__ __forceinline__ Fe<L> shape_lead(const Fe<L> (&d)[6], const FieldParams<L, K>& F,
+                                            std::integral_constant<int, kShapeAbcg>) {
+  return fe_mul(fe_mul(d[0], d[1], F), fe_mul(d[2], d[3], F), F);  // A B C G
+}
+
+__device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[9], const GoldK k,
+                                                 std::integral_constant<int, kShapeZerocheck>) {
+  return gl_mul(gl_mul(d[2], d[1], k), gl_mul(d[4], d[5], k), k);
+}
+
+__device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[6], const GoldK k,
+                                                 std::integral_constant<int, kShapeAbcg>) {
+  return gl_mul(gl_mul(d[0], d[1], k), gl_mul(d[2], d[3], k), k);
 }
 
 // The same formulas in lazy Goldilocks arithmetic: operands and result in [0, 2^64).
@@ -562,7 +593,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       // as below, in lazy arithmetic: sh_v / sh_d arrive canonical, the differences are
       // canonical, the stepped values and the point sums are any representatives
       constexpr int D = 4;
-      static_assert(DMAX >= D, "shape kernels evaluate degree-4 shapes");
+      static_assert(DMAX == D, "shape kernels evaluate degree-4 shapes");
       const GoldK gk = gold_k(F);
       const std::integral_constant<int, SHAPE> shape{};
       acc[0] = gl_add(acc[0], shape_value_lazy(sh_v, gk, shape), gk);
@@ -575,9 +606,10 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       if constexpr (kAsync) {
         if (!fold && q + stride < last) issue(q + stride);
       }
+      acc[D] = gl_add(acc[D], shape_lead_lazy(sh_d, gk, shape), gk);
       if (!skip1) acc[1] = gl_add(acc[1], shape_value_lazy(sh_v, gk, shape), gk);
 #pragma unroll
-      for (int t = 2; t <= D; ++t) {
+      for (int t = 2; t < D; ++t) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) sh_v[r] = gl_add_c(sh_v[r], sh_d[r], gk);
         acc[t] = gl_add(acc[t], shape_value_lazy(sh_v, gk, shape), gk);
@@ -585,7 +617,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
     } else {
       // point 0: e; point 1: o (skipped when skip1); then v(t) = v(t - 1) + (o - e)
       constexpr int D = 4;
-      static_assert(DMAX >= D, "shape kernels evaluate degree-4 shapes");
+      static_assert(DMAX == D, "shape kernels evaluate degree-4 shapes");
       acc[0] = fe_add(acc[0], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
@@ -596,14 +628,21 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       if constexpr (kAsync) {
         if (!fold && q + stride < last) issue(q + stride);
       }
+      acc[D] = fe_add(acc[D], shape_lead<L, K>(sh_d, F, std::integral_constant<int, SHAPE>{}), F);
       if (!skip1) acc[1] = fe_add(acc[1], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
 #pragma unroll
-      for (int t = 2; t <= D; ++t) {
+      for (int t = 2; t < D; ++t) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) sh_v[r] = fe_add(sh_v[r], sh_d[r], F);
         acc[t] = fe_add(acc[t], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
       }
     }
+  }
+  if constexpr (SHAPE == kShapeGeneric) {  // the leading coefficient belongs in slot d
+    const int d = E.degree;
+#pragma unroll
+    for (int t = 2; t < DMAX; ++t)
+      if (t == d) acc[t] = acc[DMAX];
   }
 }
 
@@ -719,38 +758,107 @@ __device__ __forceinline__ Fe<L> fe_mul_any(const Fe<L>& a, Fe<L> b, const Field
   }
 }
 
-// The round's integer sums to g_j: sum_l s[t L + l] 2^(32 l) mod p for t = 0..d, into
-// g_sm[t L + l]. The low L words times `one` and the word above them times R^2 are one product
-// each, in lanes t and 8 + t of the calling warp.
+// The evaluators' points. For degree d >= 2 they evaluate 0, 1, .. d - 1 (1 is left out when
+// g(1) comes from the claim) and, in the place of point d, the leading coefficient: every factor's
+// value at "infinity" is its difference o - e, so that point needs no stepping and only the
+// terms of full degree. The d-th finite difference of a polynomial of degree d is d! times
+// its leading coefficient, so g(d) = d! lead - sum_{s < d} (-1)^(d - s) C(d, s) g(s): integer
+// weights, applied once a round to the integer sums. Degree 1 evaluates 0 and 1.
+struct PointWeights {
+  int32_t w[kMaxPoints][kMaxPoints];  // [d][s]: weight of slot s in g(d)
+};
+constexpr PointWeights make_point_weights() {
+  PointWeights P{};
+  for (int d = 1; d < kMaxPoints; ++d) {
+    int64_t binom = 1, fact = 1;
+    for (int s = 0; s < d; ++s) {
+      P.w[d][s] = static_cast<int32_t>((d - s) % 2 ? binom : -binom);
+      binom = binom * (d - s) / (s + 1);
+      fact *= s + 1;
+    }
+    P.w[d][d] = static_cast<int32_t>(fact);
+  }
+  P.w[1][0] = 0;  // degree 1: point 1 itself
+  return P;
+}
+static __constant__ PointWeights kPointWeights = make_point_weights();
+
+// The round's integer sums to g_j, into g_sm[t L + l] for t = 0..d (one warp). `claim`, when
+// not null, stands in for point 1: g(1) = claim - g(0). Lane t < 8 turns its slot's sums into
+// words; lane t then forms g(t) as an integer (point d: the weighted sum of the slots; L words
+// and a signed rest) and the rest's words times R^2 (and R^3 at one limb) and the low words
+// times `one` are one product each, in lanes t, 8 + t and 16 + t.
 template <int L, int K>
-__device__ __forceinline__ void sums_to_points(const uint64_t* s_sm, int d, const FieldConsts& fc,
-                                               const FieldParams<L, K>& F, uint32_t* g_sm) {
-  const int lane = threadIdx.x & 31, t = lane & 7;
-  const Fe<L> con = fc_get<L>(lane < 8 ? fc.one : fc.r2);
-  Fe<L> v = fe_zero<L>();
-  if (t <= d && lane < 16) {
+__device__ __forceinline__ void sums_to_points(const uint64_t* s_sm, int d, const uint32_t* claim, bool skip1,
+                                               const FieldConsts& fc, const FieldParams<L, K>& F, uint32_t* g_sm) {
+  __shared__ int64_t slot_sm[kMaxPoints * (L + 1)];
+  const int lane = threadIdx.x & 31, t = lane & 7, part = lane >> 3;
+  const Fe<L> con = fc_get<L>(part == 0 ? fc.one : (part == 1 ? fc.r2 : fc.r3));
+  Fe<L> cl = fe_zero<L>();
+  if (claim && lane == 1) cl = ld_fe_cg<L>(claim);
+  if (lane <= d && !(skip1 && lane == 1)) {
     uint64_t c = 0;
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      c += s_sm[t * L + l];
+      c += s_sm[lane * L + l];
+      slot_sm[lane * (L + 1) + l] = static_cast<int64_t>(c & 0xffffffffu);
+      c >>= 32;
+    }
+    slot_sm[lane * (L + 1) + L] = static_cast<int64_t>(c);
+  }
+  __syncwarp();
+  if (skip1 && lane == 1) {  // claim - g(0); the claim alone is missing from one rank's share
+#pragma unroll
+    for (int l = 0; l <= L; ++l) slot_sm[(L + 1) + l] = (l < L ? static_cast<int64_t>(cl.w[l < L ? l : 0]) : 0) - slot_sm[l];
+  }
+  __syncwarp();
+  Fe<L> v = fe_zero<L>();
+  bool neg = false;
+  if (t <= d && part < (L == 1 ? 3 : 2)) {
+    int64_t a[L + 1];
+#pragma unroll
+    for (int l = 0; l <= L; ++l) a[l] = t < d ? slot_sm[t * (L + 1) + l] : 0;
+    if (t == d)
+      for (int s = 0; s <= d; ++s) {
+        const int64_t w = kPointWeights.w[d][s];
+#pragma unroll
+        for (int l = 0; l <= L; ++l) a[l] += w * slot_sm[s * (L + 1) + l];
+      }
+    int64_t c = 0;
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+      c += a[l];
       v.w[l] = static_cast<uint32_t>(c);
       c >>= 32;
     }
-    if (lane >= 8) {
+    int64_t hi = c + a[L];
+    neg = hi < 0;
+    if (neg) {  // the absolute value; the sign is applied at the end
+      uint64_t k = 1;
+#pragma unroll
+      for (int l = 0; l < L; ++l) {
+        k += static_cast<uint32_t>(~v.w[l]);
+        v.w[l] = static_cast<uint32_t>(k);
+        k >>= 32;
+      }
+      hi = static_cast<int64_t>(~static_cast<uint64_t>(hi) + k);
+    }
+    if (part) {
       v = fe_zero<L>();
-      v.w[0] = static_cast<uint32_t>(c);
+      const uint64_t h = static_cast<uint64_t>(hi);
+      if constexpr (L == 1) {
+        v.w[0] = static_cast<uint32_t>(part == 1 ? h : h >> 32);
+      } else {
+        v.w[0] = static_cast<uint32_t>(h);
+        v.w[1] = static_cast<uint32_t>(h >> 32);
+      }
     }
   }
-  const Fe<L> x = fe_mul_any(con, v, F);
-  const Fe<L> g = fe_add(x, fe_shfl_down(x, 8), F);
+  Fe<L> x = fe_mul_any(con, v, F);
+  if constexpr (L == 1) x = fe_add(x, fe_shfl_down(x, 16), F);
+  Fe<L> g = fe_add(x, fe_shfl_down(x, 8), F);
+  if (neg) g = fe_sub(fe_zero<L>(), g, F);
   if (lane <= d) st_fe<L>(g_sm + lane * L, g);
-  __syncwarp();
-}
-
-// g(1) = claim - g(0), when the round did not evaluate point 1 (one warp).
-template <int L, int K>
-__device__ __forceinline__ void point1_from_claim(const uint32_t* claim, uint32_t* g_sm, const FieldParams<L, K>& F) {
-  if ((threadIdx.x & 31) == 0) st_fe<L>(g_sm + L, fe_sub(ld_fe_cg<L>(claim), ld_fe<L>(g_sm), F));
   __syncwarp();
 }
 
@@ -893,8 +1001,7 @@ __device__ __forceinline__ void finish_round(const RoundArgs& A, const ExprDev& 
                                              const uint64_t* s_sm, uint32_t* g_sm, uint32_t* r_sm) {
   const int d = E.degree;
   if (threadIdx.x < 32) {
-    sums_to_points<L, K>(s_sm, d, *A.fc, F, g_sm);
-    if (A.skip1 && !A.ext_out) point1_from_claim<L, K>(A.st.claim, g_sm, F);
+    sums_to_points<L, K>(s_sm, d, A.skip1 && !A.ext_out ? A.st.claim : nullptr, A.skip1 != 0, *A.fc, F, g_sm);
   }
   __syncthreads();
   if (A.ext_out) {

@@ -12,8 +12,9 @@
 //      fold them with r_{j-1} (two products a table), write T_j, and put every table's value e
 //      and difference o - e into the pair's shared-memory slot;
 //   2. evaluate: each lane computes the expression at its point from the slot: a factor's value
-//      at p is e + p (o - e), p (o - e) by an addition chain (p <= 7), and one product per
-//      factor after the first;
+//      at p is e + p (o - e), p (o - e) by an addition chain (p <= 6), and one product per
+//      factor after the first; the lane of point d takes the differences (the leading
+//      coefficient) instead;
 //   3. reduce: each lane keeps one point sum; lanes with the same point are summed across the
 //      warp (shuffles over the pair index) and across warps (shared memory).
 // A lane holds one sum, one product and one factor, so the 8-limb kernel fits 4 x 128 threads
@@ -79,10 +80,12 @@ __device__ __forceinline__ Fe<L> fe_times_small(const Fe<L>& x, int c, const Fie
   return acc;
 }
 
-// The expression at point p from a pair's slot (e[k], d[k] for every table k).
+// The expression at point p from a pair's slot (e[k], d[k] for every table k); its coefficient
+// of t^d for p = d >= 2 (prover.cuh, make_point_weights).
 template <int L, int K>
 __device__ __forceinline__ Fe<L> pp_eval_point(const ExprDev& E, const uint32_t* slot_e, const uint32_t* slot_d,
                                                int p, const FieldParams<L, K>& F) {
+  const bool lead = p == E.degree && p >= 2;
   auto value = [&](int k) {
     Fe<L> e, d;
 #pragma unroll
@@ -90,12 +93,14 @@ __device__ __forceinline__ Fe<L> pp_eval_point(const ExprDev& E, const uint32_t*
       e.w[l] = slot_e[k * L + l];
       d.w[l] = slot_d[k * L + l];
     }
+    if (lead) return d;
     return p == 0 ? e : fe_add(e, fe_times_small(d, p, F), F);
   };
   Fe<L> acc = fe_zero<L>();
   for (int i = 0; i < E.num_terms; ++i) {
     const int off = E.term_off[i];
     const int len = E.term_len[i];
+    if (lead && len < p) continue;
     const int kind = E.coeff_kind[i];
     Fe<L> prod = value(E.flat[off]);
     if (kind == kCoeffSmall) {

@@ -34,7 +34,19 @@ __global__ void split_commit_kernel(const RoundArgs A, const ExprDev E, const Fi
     st_fe<L>(g_sm + lane * L, acc);
   }
   __syncwarp();
-  if (A.skip1) point1_from_claim<L, K>(A.st.claim, g_sm, F);
+  if (A.skip1 && lane <= d) {
+    // the shares hold -g(0) in the place of g(1); the claim's part of g(1), and of g(d) for
+    // d >= 2 ((-1)^d d claims, make_point_weights), is added here
+    Fe<L> c = ld_fe_cg<L>(A.st.claim);
+    Fe<L> g = ld_fe<L>(g_sm + lane * L);
+    if (lane == 1) g = fe_add(g, c, F);
+    if (lane == d && d >= 2) {
+      c = fe_mul_small(c, static_cast<uint32_t>(d), F);
+      g = d % 2 ? fe_sub(g, c, F) : fe_add(g, c, F);
+    }
+    st_fe<L>(g_sm + lane * L, g);
+  }
+  __syncwarp();
   finalize_round<L, K>(A, E, F, g_sm, r_sm);
 }
 
