@@ -20,54 +20,58 @@ constexpr uint64_t kSkip1MinPairs = uint64_t{1} << 12;
 
 inline bool round_skip1(int n, int j) { return j >= 1 && (uint64_t{1} << (n - j - 1)) >= kSkip1MinPairs; }
 
-// Tail launch: from the first round with at most a few pairs a thread of the batched kernel's
-// block (tail_round), that one block proves the rest of the proof (batch_round_kernel's tail rounds: no
-// grid-wide partials and no launch per round). Generic expressions only: the batched kernel
-// has no compile-time shapes, and the shape kernels' small rounds beat its generic evaluator.
-// Measured on B200 (median of 10 proofs): a b over 2^32 - 5, n = 16, 0.254 -> 0.228 ms,
-// n = 8 0.147 -> 0.110 ms; a degree-3 expression over 2^127 - 1, n = 8..20, 1.09-1.36x;
-// with the zerocheck and g(abc + de) shapes, 0.91-1.0x (so those keep a launch per round).
-#ifndef SC_PLAIN_TAILS
-#define SC_PLAIN_TAILS 1
-#endif
-constexpr bool kPlainTails = SC_PLAIN_TAILS != 0;
-
-struct TailDesc {
-  BatchRound r;
-  ExprDev e;
-};
-
-int tail_shape(sc_ctx* ctx, int L, int kind, int dclass, int tables, int* threads, size_t* smem) {
-  for (const TailShape& t : ctx->tail_shapes)
-    if (t.L == L && t.kind == kind && t.dclass == dclass && t.tables == tables) {
-      *threads = t.threads;
-      *smem = t.smem;
-      return SC_OK;
-    }
-  int grid = 0;
-  int rc = batch_kernel_setup(L, kind, dclass, tables, 0, ctx->sm_count, threads, &grid, smem);
-  if (rc) return rc;
-  ctx->tail_shapes.push_back(TailShape{L, kind, dclass, tables, *threads, *smem});
-  return SC_OK;
+// Rounds of at most tail_pairs() pairs run in one block (tail.cuh): for a generic expression
+// one launch proves the rest of the proof, for the compile-time shapes a launch proves one
+// round. One SM's arithmetic bounds such a round from above, so the line falls with the work of
+// a pair (`units`: products of its folds and of its d + 1 points); a launch, the grid's sums
+// and a thread walking through a whole pair bound the other side, and at 8 limbs the
+// point-parallel kernel takes over earlier. Measured on B200, us a proof at n = 14 by the
+// largest round in one block (0: none):
+//   a b, 1 limb (7 units)               0: 153   32: 137   128: 136   256: 134   1024: 126
+//   permutation check, 2 limbs (80)     0: 286   32: 225   128: 222   256: 220   512: 238
+//   17-term gate, 2 limbs (520)         0: 756   32: 534   64: 513   128: 516   256: 539
+//   aabbc, 4 limbs (30)                 0: 277   32: 227   128: 224   256: 217   1024: 258
+//   17-term gate, 4 limbs (520)         0: 1936  32: 1290  64: 1220  128: 1183  256: 1182
+//   a b, 8 limbs (7)                    0: 225   32: 203   64: 198   256: 197   1024: 239
+//   permutation check, 8 limbs (80)     0: 487   16: 428   32: 425   64: 430   128: 462
+//   12-term gate, 8 limbs (175)         0: 826   16: 661   32: 647   64: 658   256: 850
+//   zerocheck shape, 2 limbs            0: 188   16: 179   32: 179   64: 181   256: 193
+//   g(abc + de) shape, 8 limbs          0: 464   16: 394   32: 383   64: 374   128: 383
+inline uint64_t tail_pairs(const sc_expr& ex, int L, bool shaped) {
+  uint64_t units = 2 * static_cast<uint64_t>(ex.num_vars);
+  for (int32_t len : ex.lens) units += static_cast<uint64_t>(ex.degree + 1) * (len - 1);
+  const uint64_t budget = L >= 8 ? 2600 : 66000;
+  uint64_t p = shaped ? (L >= 8 ? 64 : 32) : 256;
+  const uint64_t least = L >= 8 ? 32 : 64;
+  while (!shaped && p > least && p * units > budget) p >>= 1;
+  while (p && tail_smem_words(p, ex.num_vars, L) * 4 > static_cast<size_t>(kMaxDynSmem)) p >>= 1;
+  return p;
 }
 
-// The round the tail launch starts at (stop: none), for a proof run up to round stop: the
-// first with at most a few pairs a thread of the batched kernel's block.
-int tail_round(sc_ctx* ctx, int L, int kind, int dclass, int tables, int shape, int n, int first, int stop,
-               int* out_round, int* threads, size_t* smem) {
-  *out_round = stop;
-  if (!kPlainTails || stop != n || shape != kShapeGeneric) return SC_OK;
-  int rc = tail_shape(ctx, L, kind, dclass, tables, threads, smem);
-  if (rc) return rc;
-  // pairs a thread at the tail's first round: measured on B200 (1, 2 or 4), 4 was best for
-  // a b over 2^32 - 5 (n = 16: 0.233 -> 0.224 ms), 1-2 for 4 and 8 limbs (4 was 3-7% slower)
-  const uint64_t per_thread = L == 1 ? 4 : (L <= 4 ? 2 : 1);
-  for (int j = first; j < n - 1; ++j)
-    if (((uint64_t{1} << n) >> (j + 1)) <= static_cast<uint64_t>(*threads) * per_thread) {
-      *out_round = j;
-      break;
-    }
-  return SC_OK;
+// The first round of [first, stop) that runs in one block (stop: none).
+int tail_round(const sc_expr& ex, int L, bool shaped, int n, int first, int stop) {
+  const uint64_t p = tail_pairs(ex, L, shaped);
+  for (int j = first; j < stop; ++j)
+    if (((uint64_t{1} << n) >> (j + 1)) <= p) return j;
+  return stop;
+}
+
+// A round's launch; after: it follows another round's launch on the stream and may be set up
+// while that round ends (prover.cuh, pdl_begin).
+template <typename Args, typename Params>
+cudaError_t launch_round(void (*kern)(const Args, const ExprDev, const Params), unsigned grid, int threads, size_t smem,
+                         cudaStream_t stream, bool after, const Args& A, const ExprDev& E, const Params& F) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, A, E, F);
 }
 
 template <int L, int K, int DMAX>
@@ -150,9 +154,7 @@ struct ProveRun {
                            st + so.chals, first, ctx->sm_count, ctx->stream)))
       return rc;
     const uint32_t* prev = first <= 1 ? tables : static_cast<const uint32_t*>(((first - 1) & 1) ? ctx->fold_a.p : ctx->fold_b.p);
-    int tail_j = stop, tail_threads = 0;
-    size_t tail_smem = 0;
-    if ((rc = tail_round(ctx, L, K, DMAX, K_, shape, n, first, stop, &tail_j, &tail_threads, &tail_smem))) return rc;
+    const int tail_j = tail_round(*ex, L, shape != kShapeGeneric, n, first, stop);
     for (int j = first; j < stop; ++j) {
       A.round = j;
       A.pairs = N >> (j + 1);
@@ -177,39 +179,18 @@ struct ProveRun {
         A.dst = static_cast<uint32_t*>((j & 1) ? ctx->fold_a.p : ctx->fold_b.p);
         prev = A.dst;
       }
-      if (j == tail_j) {  // this round and every later one, in one block
-        if ((rc = ensure(ctx, ctx->tail, sizeof(TailDesc)))) return rc;
-        if (!ctx->tail_host) SC_CUDA(cudaMallocHost(&ctx->tail_host, sizeof(TailDesc)));
-        if (!ctx->tail_copied) SC_CUDA(cudaEventCreateWithFlags(&ctx->tail_copied, cudaEventDisableTiming));
-        // the staging's previous copy has landed (a proof ends with a stream synchronisation,
-        // unless it failed part way)
-        SC_CUDA(cudaEventSynchronize(ctx->tail_copied));
-        TailDesc& desc = *static_cast<TailDesc*>(ctx->tail_host);
-        std::memset(&desc, 0, sizeof(desc));
-        TailDesc* dev = static_cast<TailDesc*>(ctx->tail.p);
-        desc.r.args = A;
-        desc.r.expr = &dev->e;
-        desc.r.num_items = 1;
-        desc.r.round_items = 1;
-        desc.r.tail_rounds = n - 1 - j;
-        desc.r.skip1_min_pairs = static_cast<uint32_t>(kSkip1MinPairs);
-        desc.r.fold_a = static_cast<uint32_t*>(ctx->fold_a.p);
-        desc.r.fold_b = static_cast<uint32_t*>(ctx->fold_b.p);
-        desc.e = E;
-        SC_CUDA(cudaMemcpyAsync(dev, &desc, sizeof(desc), cudaMemcpyHostToDevice, ctx->stream));
-        SC_CUDA(cudaEventRecord(ctx->tail_copied, ctx->stream));
-        BatchTickArgs T;
-        T.rounds = &dev->r;
-        T.items = nullptr;
-        T.num_items = 1;
-        T.pad = 0;
-        T.head = nullptr;
-        T.tile = A.pairs;
+      if (j >= tail_j) {  // this round, or this and every later one, in one block
+        TailArgs T;
+        T.first = A;
+        T.rounds = shape == kShapeGeneric ? stop - j : 1;
+        T.store = j + T.rounds < stop ? 1 : 0;
+        const size_t tail_smem = tail_smem_words(A.pairs, K_, L) * 4;
         cudaEvent_t ev;
         if ((rc = timing_begin(ctx, &ev))) return rc;
-        if ((rc = batch_kernel_launch(L, K, DMAX, f, 1, tail_threads, tail_smem, ctx->stream, T))) return rc;
+        SC_CUDA(launch_round(tail_kernel<L, K>, 1, tail_threads(L), tail_smem, ctx->stream, j > first, T, E, F));
         if ((rc = timing_end(ctx))) return rc;
-        break;
+        j += T.rounds - 1;
+        continue;
       }
       uint64_t per_block = static_cast<uint64_t>(threads);
       if (use_point_parallel(L) && shape == kShapeGeneric) {  // pairs a block holds: one per lane group
@@ -221,8 +202,7 @@ struct ProveRun {
       const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(want, grid_max));
       cudaEvent_t ev;
       if ((rc = timing_begin(ctx, &ev))) return rc;
-      kern<<<grid, threads, smem, ctx->stream>>>(A, E, F);
-      SC_CUDA(cudaGetLastError());
+      SC_CUDA(launch_round(kern, grid, threads, smem, ctx->stream, j > first, A, E, F));
       if ((rc = timing_end(ctx))) return rc;
     }
     return finish(ctx, ex, n, stop, st, so, out_polys, out_ch, out_finals, out_claim0, out_checksum, state_io);
@@ -376,12 +356,10 @@ int sc_ctx_destroy(sc_ctx* ctx) {
   if (!ctx) return SC_OK;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  for (DevBuf* b : {&ctx->fold_a, &ctx->fold_b, &ctx->state, &ctx->tail})
+  for (DevBuf* b : {&ctx->fold_a, &ctx->fold_b, &ctx->state})
     if (b->p) cudaFree(b->p);
   for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
   if (ctx->host_state) cudaFreeHost(ctx->host_state);
-  if (ctx->tail_host) cudaFreeHost(ctx->tail_host);
-  if (ctx->tail_copied) cudaEventDestroy(ctx->tail_copied);
   delete ctx;
   return SC_OK;
 }
@@ -693,14 +671,9 @@ int sc_prove_launches(sc_ctx* ctx, const sc_field* field, const sc_expr* expr, i
   if (num_rounds < 1 || num_rounds > kMaxRounds)
     return fail(SC_ERR_INVALID, "num_rounds %d outside 1..%d", num_rounds, kMaxRounds);
   SC_CUDA(cudaSetDevice(ctx->device));
-  int tail = num_rounds, threads = 0;
-  size_t smem = 0;
   uint8_t role[16];
-  const int dclass = degree_class(expr->degree);
-  const int shape = dclass == 4 ? match_shape(*expr, role) : kShapeGeneric;
-  const int rc = tail_round(ctx, field->hf.L, field_kind(field->hf.p, field->hf.L), dclass, expr->num_vars, shape,
-                            num_rounds, 0, num_rounds, &tail, &threads, &smem);
-  if (rc) return rc;
+  const bool shaped = degree_class(expr->degree) == 4 && match_shape(*expr, role) != kShapeGeneric;
+  const int tail = shaped ? num_rounds : tail_round(*expr, field->hf.L, false, num_rounds, 0, num_rounds);
   if (out_launches) *out_launches = tail < num_rounds ? tail + 1 : num_rounds;
   if (out_tail_round) *out_tail_round = tail;
   return SC_OK;

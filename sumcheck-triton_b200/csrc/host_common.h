@@ -13,7 +13,7 @@
 
 #include "../../include/sumcheck_b200.h"
 #include "host_field.h"
-#include "prover.cuh"
+#include "batch.cuh"
 #include "tables.cuh"
 
 using namespace sc;
@@ -60,22 +60,11 @@ int batch_kernel_launch(int L, int K, int dmax, const sc_field* field, unsigned 
 
 using sc_host::DevBuf;
 
-// Launch shape of the batched kernel for one (L, field kind, degree class, tables): the
-// plain path's tail launch (capi.cu) looks it up once per context.
-struct TailShape {
-  int L, kind, dclass, tables, threads;
-  size_t smem;
-};
-
 struct sc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   DevBuf fold_a, fold_b, state;       // state: the proof state's words, then the round's sums
-  DevBuf tail;                        // the tail launch's BatchRound and ExprDev
-  void* tail_host = nullptr;          // pinned staging of the same
-  cudaEvent_t tail_copied = nullptr;  // the staging's last copy to the device
-  std::vector<TailShape> tail_shapes;
   uint32_t* host_state = nullptr;  // pinned staging of the proof state
   size_t host_state_bytes = 0;
   // per-launch timing of the round kernels (off by default)
@@ -203,6 +192,7 @@ template <int L, int K, int D>
 struct SetRoundAttrs {
   static int run() {
     SC_CUDA(cudaFuncSetAttribute(round_kernel<L, K, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+    if constexpr (D == 2) SC_CUDA(cudaFuncSetAttribute(tail_kernel<L, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
     if constexpr (D == 4) {  // the shape kernels (the 2-limb Goldilocks ones stage pairs in shared memory)
       SC_CUDA(cudaFuncSetAttribute(round_kernel<L, K, 4, kShapeZerocheck>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kMaxDynSmem));

@@ -135,9 +135,19 @@ struct RoundArgs {
   ProofState st;
   uint32_t* ext_out;     // non-null: the round's sums g_j(0..d) go here and the round is not
                          // finalised (one rank of a split proof; the commit finalises it)
+  const uint32_t* last;  // non-null: T_{n-1} for the last round's f_k(r) (a tail's, in shared memory)
   int32_t check_claim;   // with skip1 == 0: check g_j(0) + g_j(1) against st.claim (kStatusClaim)
   int32_t pad;
 };
+
+// Rounds are queued with programmatic stream serialisation: a round's launch and its blocks'
+// start overlap the end of the round before, and pdl_begin waits for that round's results
+// (before anything it wrote is read), then lets the next round's launch begin. Without the
+// launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 template <int L>
 __device__ __forceinline__ Fe<L> ld_fe(const uint32_t* p) {
@@ -656,6 +666,22 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
 // limbs and degree 4, 17k at 8 limbs and degree 7, and ran twice a round with a loop over the
 // blocks' partials in between (6.3k / 10.9k).
 
+// Shared memory of a round's end. msg is the hash message preceded by three zero bytes, so that
+// its 21-byte domain string ends on a word and j and the words of g_j follow aligned: message
+// word q is the funnel shift of msg[q] and msg[q + 1].
+constexpr int kMsgG = 7;  // msg[0..5] the domain string, msg[6] = j, msg[7..] the words of g_j
+template <int L>
+struct RoundEnd {
+  static constexpr int kMsgWords = 34 * ((25 + 4 * kMaxPoints * L) / 136 + 1) + 1;
+  uint64_t s[kMaxPoints * L];             // the round's integer sums
+  int64_t slot[kMaxPoints * (L + 1)];     // their words
+  uint32_t msg[kMsgWords];
+  uint32_t r[L];                          // r_j
+  __align__(8) uint32_t dig[8];
+  int is_last;
+  __device__ uint32_t* g() { return msg + kMsgG; }  // g_j(t): words g()[t L + l]
+};
+
 // This warp's integer sums of acc[0..d] into its row of scratch.
 template <int L, int N>
 __device__ __forceinline__ void warp_sums(const Fe<L> (&acc)[N], int d, uint32_t* scratch) {
@@ -699,18 +725,18 @@ __device__ __forceinline__ void block_sums(const uint32_t* scratch, int d, bool 
 }
 
 // Block-wide, after warp_sums: true in the block that completes the round (its `parts`-th block
-// or item), with the round's integer sums in s_sm; every thread calls. Ends with a barrier.
+// or item), with the round's integer sums in end.s; every thread calls. Ends with a barrier.
 template <int L>
 __device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32_t part, uint32_t parts, uint64_t* sums,
-                                          uint32_t* counter, uint64_t* s_sm, int* is_last) {
+                                          uint32_t* counter, RoundEnd<L>& end) {
   __syncthreads();
-  block_sums<L>(scratch, d, parts == 1, s_sm, sums, part);
+  block_sums<L>(scratch, d, parts == 1, end.s, sums, part);
   if (parts > 1) {
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) *is_last = atomicAdd(counter, 1u) == parts - 1;
+    if (threadIdx.x == 0) end.is_last = atomicAdd(counter, 1u) == parts - 1;
     __syncthreads();
-    if (!*is_last) return false;
+    if (!end.is_last) return false;
     __threadfence();
     for (int i = threadIdx.x; i < (d + 1) * L; i += blockDim.x) {
       uint64_t v[kSumCopies], s = 0;
@@ -721,7 +747,7 @@ __device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32
         s += v[c];
         if (c < static_cast<int>(parts)) sums[c * kMaxPoints * L + i] = 0;
       }
-      s_sm[i] = s;
+      end.s[i] = s;
     }
     if (threadIdx.x == 0) *counter = 0;
   }
@@ -783,24 +809,39 @@ constexpr PointWeights make_point_weights() {
 }
 static __constant__ PointWeights kPointWeights = make_point_weights();
 
-// The round's integer sums to g_j, into g_sm[t L + l] for t = 0..d (one warp). `claim`, when
-// not null, stands in for point 1: g(1) = claim - g(0). Lane t < 8 turns its slot's sums into
-// words; lane t then forms g(t) as an integer (point d: the weighted sum of the slots; L words
-// and a signed rest) and the rest's words times R^2 (and R^3 at one limb) and the low words
-// times `one` are one product each, in lanes t, 8 + t and 16 + t.
-template <int L, int K>
-__device__ __forceinline__ void sums_to_points(const uint64_t* s_sm, int d, const uint32_t* claim, bool skip1,
-                                               const FieldConsts& fc, const FieldParams<L, K>& F, uint32_t* g_sm) {
-  __shared__ int64_t slot_sm[kMaxPoints * (L + 1)];
+// Field constants of a round's end, by lane of warp 0 (they depend on nothing else, so a block
+// that proves several rounds loads them once).
+template <int L>
+struct EndConsts {
+  Fe<L> con;  // sums_to_points
+  Fe<L> dig;  // lanes 0..8 / L - 1: the digest's weights
+};
+template <int L>
+__device__ __forceinline__ EndConsts<L> load_end_consts(const FieldConsts& fc) {
+  const int lane = threadIdx.x & 31, part = lane >> 3;
+  EndConsts<L> c;
+  c.con = fc_get<L>(part == 0 ? fc.one : (part == 1 ? fc.r2 : fc.r3));
+  c.dig = lane < 8 / L ? fc_get<L>(fc.kdig[lane * L]) : fe_zero<L>();
+  return c;
+}
+
+// The round's integer sums (sum(t L + l)) to g_j, into end.g() (warp 0). `claim`, when not null,
+// stands in for point 1: g(1) = claim - g(0). Lane t < 8 turns its slot's sums into words; lane
+// t then forms g(t) as an integer (point d: the weighted sum of the slots; L words and a signed
+// rest) and the rest's words times R^2 (and R^3 at one limb) and the low words times `one` are
+// one product each, in lanes t, 8 + t and 16 + t.
+template <int L, int K, typename Sum>
+__device__ __forceinline__ void sums_to_points(Sum sum, int d, const uint32_t* claim, bool skip1, const Fe<L>& con,
+                                               const FieldParams<L, K>& F, RoundEnd<L>& end) {
+  int64_t* const slot_sm = end.slot;
   const int lane = threadIdx.x & 31, t = lane & 7, part = lane >> 3;
-  const Fe<L> con = fc_get<L>(part == 0 ? fc.one : (part == 1 ? fc.r2 : fc.r3));
   Fe<L> cl = fe_zero<L>();
   if (claim && lane == 1) cl = ld_fe_cg<L>(claim);
   if (lane <= d && !(skip1 && lane == 1)) {
     uint64_t c = 0;
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      c += s_sm[lane * L + l];
+      c += sum(lane * L + l);
       slot_sm[lane * (L + 1) + l] = static_cast<int64_t>(c & 0xffffffffu);
       c >>= 32;
     }
@@ -858,30 +899,40 @@ __device__ __forceinline__ void sums_to_points(const uint64_t* s_sm, int d, cons
   if constexpr (L == 1) x = fe_add(x, fe_shfl_down(x, 16), F);
   Fe<L> g = fe_add(x, fe_shfl_down(x, 8), F);
   if (neg) g = fe_sub(fe_zero<L>(), g, F);
-  if (lane <= d) st_fe<L>(g_sm + lane * L, g);
+  if (lane <= d) st_fe<L>(end.g() + lane * L, g);
   __syncwarp();
 }
 
-// The transcript's domain string as little-endian words; word 5 holds its last byte.
+// The transcript's 21-byte domain string behind three zero bytes, as little-endian words.
 struct TranscriptDomain {
   uint32_t w[6];
 };
 constexpr TranscriptDomain make_transcript_domain() {
   const char dom[] = "zkduel:field-sweep:v1";
   TranscriptDomain t{};
-  for (int i = 0; i < 21; ++i) t.w[i / 4] |= static_cast<uint32_t>(static_cast<unsigned char>(dom[i])) << (8 * (i % 4));
+  for (int i = 0; i < 21; ++i)
+    t.w[(i + 3) / 4] |= static_cast<uint32_t>(static_cast<unsigned char>(dom[i])) << (8 * ((i + 3) % 4));
   return t;
 }
 static __constant__ TranscriptDomain kTranscriptDomain = make_transcript_domain();
 
-// The end of round j, with g_j complete in g_sm[t * L + l]; every thread of the block calls,
-// after a barrier. Warp 0 derives r_j (into r_sm[L] too, for a caller that goes on with the
-// next round in this block, after a barrier of its own); the next warp, if there is one,
-// stores the round polynomial, the checksum and the claim of round 0 meanwhile.
+// The parts of round j's hash message that are known before g_j (threads first, first + step, ..).
+template <int L>
+__device__ __forceinline__ void begin_message(RoundEnd<L>& end, int d, int j, int first, int step) {
+  const int past = kMsgG + (d + 1) * L;  // the word after g_j: the padding's first byte
+  for (int i = first; i < RoundEnd<L>::kMsgWords; i += step)
+    if (i < kMsgG || i >= past)
+      end.msg[i] = i < 6 ? kTranscriptDomain.w[i] : (i == 6 ? static_cast<uint32_t>(j) : (i == past ? 6u : 0u));
+}
+
+// The end of round j, with g_j complete in end.g() and begin_message done; every thread of the
+// block calls, after a barrier. Warp 0 derives r_j (into end.r too, for a caller that goes on
+// with the next round in this block, after a barrier of its own); the next warp, if there is
+// one, stores the round polynomial, the checksum and the claim of round 0 meanwhile.
 template <int L, int K>
-__device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F, const uint32_t* g_sm,
-                               uint32_t* r_sm) {
-  __shared__ __align__(8) uint32_t dig_sm[8];
+__device__ __forceinline__ void finalize_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F,
+                                               const EndConsts<L>& consts, RoundEnd<L>& end) {
+  const uint32_t* const g_sm = end.g();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int d = E.degree;
   const int j = A.round;
@@ -917,40 +968,30 @@ __device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const Field
   // What the end of the round reads from global memory, before the hash: the digest's weights
   // (lanes 0..7) and the Lagrange weights (lanes 8..8 + d); T_{n-1} in the last round (lane k).
   constexpr int kParts = 8 / L;  // field-sized pieces of the 256-bit digest
-  Fe<L> con = fe_zero<L>();
-  if (lane < kParts)
-    con = fc_get<L>(fc.kdig[lane * L]);
-  else if (claim && lane >= 8 && lane <= 8 + d)
-    con = fc_get<L>(fc.lag[d][lane - 8]);
+  Fe<L> con = consts.dig;
+  if (claim && lane >= 8 && lane <= 8 + d) con = fc_get<L>(fc.lag[d][lane - 8]);
   Fe<L> e = fe_zero<L>(), o = fe_zero<L>();
   if (last_round && lane < E.num_vars) {
-    const uint32_t* tab = A.fold ? A.dst : A.src;  // T_{n-1}: 2 entries per plane
+    const uint32_t* tab = A.last ? A.last : (A.fold ? A.dst : A.src);  // T_{n-1}: 2 entries per plane
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      e.w[l] = __ldcg(tab + (lane * L + l) * 2 + 0);
-      o.w[l] = __ldcg(tab + (lane * L + l) * 2 + 1);
+      e.w[l] = tab[(lane * L + l) * 2 + 0];
+      o.w[l] = tab[(lane * L + l) * 2 + 1];
     }
   }
   // challenge r_j; lanes 8 + t: g_j(t) times its Lagrange weight, in the same product
   Fe<L> v = fe_zero<L>();
   if (A.mode == kChallengeSha3) {
-    // message: domain string (21 bytes) || u32 j || the words of g_j(0..d); word i of j || g
-    // starts at byte 21 + 4 i, so a message word joins two of them
-    const int nwords = 1 + (d + 1) * L;
-    auto tail = [&](int i) -> uint32_t { return i == 0 ? static_cast<uint32_t>(j) : (i < nwords ? g_sm[i - 1] : (i == nwords ? 6u : 0u)); };
-    auto word = [&](int q) -> uint32_t {
-      if (q < 5) return kTranscriptDomain.w[q];
-      return (q == 5 ? kTranscriptDomain.w[5] : tail(q - 6) >> 24) | (tail(q - 5) << 8);
-    };
+    auto word = [&](int q) -> uint32_t { return __funnelshift_l(end.msg[q], end.msg[q + 1], 8); };
     uint32_t lo, hi;
-    sha3_256_warp(word, 21 + 4 * nwords, lo, hi);
+    sha3_256_warp(word, 25 + 4 * (d + 1) * L, lo, hi);
     if (lane < 4) {
-      dig_sm[2 * lane] = lo;
-      dig_sm[2 * lane + 1] = hi;
+      end.dig[2 * lane] = lo;
+      end.dig[2 * lane + 1] = hi;
     }
     __syncwarp();
     // digest (little-endian 256-bit D) -> D R mod p = sum_i D_i (R^2 2^(32 L i)) / R
-    if (lane < kParts) v = ld_fe<L>(dig_sm + lane * L);
+    if (lane < kParts) v = ld_fe<L>(end.dig + lane * L);
   }
   if (claim && lane >= 8 && lane <= 8 + d) v = ld_fe<L>(g_sm + (lane - 8) * L);
   Fe<L> x = fe_mul_any(con, v, F);
@@ -967,7 +1008,7 @@ __device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const Field
   }
   if (lane == 0) {
     if (A.mode != kChallengeExplicit) st_fe<L>(A.st.chals + j * L, r);
-    st_fe<L>(r_sm, r);
+    st_fe<L>(end.r, r);
   }
   if (!claim) return;
   // g_j(r_j), the next round's claim or the final claim: sum_t w_t prod_{s != t} (r - s), the
@@ -995,20 +1036,25 @@ __device__ void finalize_round(const RoundArgs& A, const ExprDev& E, const Field
   }
 }
 
-// The round's integer sums (s_sm) to g_j and its end; every thread of the block calls.
-template <int L, int K>
+// The round's integer sums to g_j and its end; every thread of the block calls, after a barrier.
+template <int L, int K, typename Sum>
 __device__ __forceinline__ void finish_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F,
-                                             const uint64_t* s_sm, uint32_t* g_sm, uint32_t* r_sm) {
-  const int d = E.degree;
-  if (threadIdx.x < 32) {
-    sums_to_points<L, K>(s_sm, d, A.skip1 && !A.ext_out ? A.st.claim : nullptr, A.skip1 != 0, *A.fc, F, g_sm);
-  }
+                                             const EndConsts<L>& consts, Sum sum, RoundEnd<L>& end) {
+  const int d = E.degree, tid = threadIdx.x, nthr = blockDim.x;
+  if (tid < 32)
+    sums_to_points<L, K>(sum, d, A.skip1 && !A.ext_out ? A.st.claim : nullptr, A.skip1 != 0, consts.con, F, end);
+  if (tid >= 32 || nthr == 32) begin_message<L>(end, d, A.round, nthr == 32 ? tid : tid - 32, nthr == 32 ? 32 : nthr - 32);
   __syncthreads();
   if (A.ext_out) {
-    for (int i = threadIdx.x; i < (d + 1) * L; i += blockDim.x) A.ext_out[i] = g_sm[i];
+    for (int i = tid; i < (d + 1) * L; i += nthr) A.ext_out[i] = end.g()[i];
   } else {
-    finalize_round<L, K>(A, E, F, g_sm, r_sm);
+    finalize_round<L, K>(A, E, F, consts, end);
   }
+}
+template <int L, int K>
+__device__ __forceinline__ void finish_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F,
+                                             RoundEnd<L>& end) {
+  finish_round<L, K>(A, E, F, load_end_consts<L>(*A.fc), [&](int i) { return end.s[i]; }, end);
 }
 
 // Dynamic shared memory per thread: values and differences of every table.
@@ -1077,10 +1123,7 @@ template <int L, int K, int DMAX, int SHAPE = kShapeGeneric>
 __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
     round_kernel(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ uint64_t s_sm[kMaxPoints * L];
-  __shared__ uint32_t r_sm[L];
-  __shared__ int is_last;
+  __shared__ RoundEnd<L> end;
 
   const int tid = threadIdx.x;
   const int nthr = blockDim.x;
@@ -1088,6 +1131,7 @@ __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
   uint32_t* sv = smem;                           // [K][L][nthr] values at the current point
   uint32_t* sd = smem + E.num_vars * L * nthr;   // [K][L][nthr] differences o - e
 
+  pdl_begin();
   Fe<L> acc[DMAX + 1];
 #pragma unroll
   for (int t = 0; t <= DMAX; ++t) acc[t] = fe_zero<L>();
@@ -1100,8 +1144,8 @@ __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
   // the block's integer sums to the grid's; the last block finalises the round
   __syncthreads();
   warp_sums<L, DMAX + 1>(acc, d, smem);
-  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, s_sm, &is_last)) return;
-  finish_round<L, K>(A, E, F, s_sm, g_sm, r_sm);
+  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, end)) return;
+  finish_round<L, K>(A, E, F, end);
 }
 
 // ------------------------------------------------------------------------------ resume folds
@@ -1131,130 +1175,6 @@ __global__ void __launch_bounds__(256) fold_kernel(const uint32_t* __restrict__ 
     const Fe<L> o = fe_add(x2, fe_mul(r, fe_sub(x3, x2, F), F), F);
 #pragma unroll
     for (int l = 0; l < L; ++l) reinterpret_cast<uint2*>(dst + (k * L + l) * dst_len)[q] = make_uint2(e.w[l], o.w[l]);
-  }
-}
-
-// ------------------------------------------------------------------------------ batched
-//
-// Many independent proofs advance together, one launch per "tick" and degree class: a
-// persistent kernel whose blocks pull (proof round, tile of pairs) items from a device work
-// queue (an atomic counter over the tick's item list). Every item leaves one partial in its
-// round's partial slots; the block that finishes the last item of a proof's round (per-proof
-// atomic ticket) reads that round's sums and finalises it -- SHA3 challenge included --
-// while the other blocks go on with other proofs' items. A round's items may be spread over
-// several ticks (the served prover slices large rounds): the ticket counts to the round's
-// item total, whichever tick its last item runs in.
-//
-// Tail rounds: once a proof's round fits in one item, the block that proves it also proves
-// every later round of that proof (tail_rounds of them), one after another with block
-// barriers in between -- a few microseconds a round instead of one tick each. Round j + 1
-// reads T_j, which this block wrote itself, and r_j, which its warp 0 just derived.
-
-struct BatchRound {
-  RoundArgs args;        // this proof's round (src/dst/len/pairs/round/fold/mode/flags/fc/state)
-  const ExprDev* expr;   // this proof's expression
-  int32_t first_item;    // this tick's items of the round: [first_item, first_item + num_items)
-  int32_t num_items;
-  int32_t item_base;     // round-relative index of this tick's first item of the round
-  int32_t round_items;   // items of the whole round, over all ticks
-  int32_t tail_rounds;   // > 0: the block that finalises this round proves the next tail_rounds too
-  uint32_t skip1_min_pairs;  // tail rounds: g(1) from the claim when a round has this many pairs
-  uint32_t* fold_a;      // tail rounds: T_i for odd i
-  uint32_t* fold_b;      //              T_i for even i >= 2
-};
-
-struct BatchItem {
-  int32_t round;       // index into the tick's BatchRound array
-  int32_t pad;
-  uint64_t start;      // pairs [start, start + count)
-  uint64_t count;
-};
-
-struct BatchTickArgs {
-  const BatchRound* rounds;
-  const BatchItem* items;  // nullptr: one round, item i = pairs [i tile, (i + 1) tile)
-  int32_t num_items;
-  int32_t pad;
-  uint32_t* head;          // queue counter of this tick (zero before the launch); nullptr:
-                           // block b does item b alone (grid = num_items)
-  uint64_t tile;           // pairs per item when items is nullptr
-};
-
-template <int L, int K, int DMAX>
-__global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
-    batch_round_kernel(const BatchTickArgs T, const FieldParams<L, K> F) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ uint64_t s_sm[kMaxPoints * L];
-  __shared__ uint32_t r_sm[L];
-  __shared__ __align__(16) ExprDev E;
-  __shared__ __align__(16) BatchRound R;
-  __shared__ const ExprDev* cur_expr;
-  __shared__ int item_sm, is_last;
-
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  if (tid == 0) cur_expr = nullptr;
-  for (int pass = 0;; ++pass) {
-    __syncthreads();
-    if (tid == 0)
-      item_sm = T.head ? static_cast<int>(atomicAdd(T.head, 1u)) : (pass == 0 ? static_cast<int>(blockIdx.x) : T.num_items);
-    __syncthreads();
-    const int it = item_sm;
-    if (it >= T.num_items) break;
-    BatchItem I;
-    if (T.items) {
-      I = T.items[it];
-    } else {
-      I.round = 0;
-      I.start = static_cast<uint64_t>(it) * T.tile;
-    }
-    if (tid == 0) R = T.rounds[I.round];
-    __syncthreads();
-    if (!T.items) I.count = R.args.pairs - I.start < T.tile ? R.args.pairs - I.start : T.tile;
-    if (R.expr != cur_expr) {
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(R.expr);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&E);
-      for (int i = tid; i < static_cast<int>(sizeof(ExprDev) / 4); i += nthr) dst[i] = src[i];
-      __syncthreads();
-      if (tid == 0) cur_expr = R.expr;
-    }
-    const int d = E.degree;
-    uint32_t* sv = smem;
-    uint32_t* sd = smem + E.num_vars * L * nthr;
-    // k = 0: this item of the proof's round; k >= 1: the proof's tail rounds (only in the
-    // block that finalised round k - 1; R.args then describes round R.args.round)
-    for (int k = 0;; ++k) {
-      Fe<L> acc[DMAX + 1];
-#pragma unroll
-      for (int t = 0; t <= DMAX; ++t) acc[t] = fe_zero<L>();
-      Fe<L> r_prev = fe_zero<L>();
-      if (R.args.fold) r_prev = k == 0 ? ld_fe_cg<L>(R.args.st.chals + (R.args.round - 1) * L) : ld_fe<L>(r_sm);
-      const uint64_t q0 = k == 0 ? I.start : 0, q1 = k == 0 ? I.start + I.count : R.args.pairs;
-      process_pairs<L, K, DMAX>(R.args.src, R.args.dst, R.args.src_len, R.args.fold != 0, r_prev, E, sv, sd, q0 + tid,
-                                q1, nthr, R.args.skip1 != 0, acc, F);
-      __syncthreads();
-      warp_sums<L, DMAX + 1>(acc, d, smem);
-      const uint32_t part = k == 0 ? static_cast<uint32_t>(R.item_base + (it - R.first_item)) : 0;
-      const uint32_t parts = k == 0 ? static_cast<uint32_t>(R.round_items) : 1;
-      if (!grid_sums<L>(smem, d, part, parts, R.args.sums, R.args.st.counter, s_sm, &is_last)) break;
-      finish_round<L, K>(R.args, E, F, s_sm, g_sm, r_sm);
-      if (k == R.tail_rounds) break;
-      __syncthreads();  // the finalisation read R.args; r_j and T_j are visible to the block
-      if (tid == 0) {   // round j + 1 of the same proof
-        RoundArgs& A = R.args;
-        const int j = A.round + 1;
-        if (j >= 2) A.src = A.dst;  // T_j (round 1 folds the tables themselves)
-        A.dst = (j & 1) ? R.fold_a : R.fold_b;
-        A.round = j;
-        A.pairs >>= 1;
-        A.src_len = A.pairs * 4;
-        A.fold = 1;
-        A.skip1 = A.pairs >= R.skip1_min_pairs ? 1 : 0;
-        A.want_claim = (j + 1 < A.num_rounds && (A.pairs >> 1) >= R.skip1_min_pairs) ? 1 : 0;
-        A.check_claim = 0;
-      }
-      __syncthreads();
-    }
   }
 }
 

@@ -197,12 +197,10 @@ __device__ __forceinline__ void pp_warp_sums(Fe<L> acc, const PointPlan& P, uint
 template <int L, int K>
 __global__ void __launch_bounds__(128, 4) round_kernel_pp(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
-  __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ uint64_t s_sm[kMaxPoints * L];
-  __shared__ uint32_t r_sm[L];
-  __shared__ int is_last;
+  __shared__ RoundEnd<L> end;
   const int d = E.degree;
   const PointPlan P = point_plan(d, A.skip1 != 0);
+  pdl_begin();
   Fe<L> acc = fe_zero<L>();
   Fe<L> r_prev = fe_zero<L>();
   if (A.fold) r_prev = ld_fe_cg<L>(A.st.chals + (A.round - 1) * L);
@@ -212,8 +210,8 @@ __global__ void __launch_bounds__(128, 4) round_kernel_pp(const RoundArgs A, con
                          static_cast<uint64_t>(slots) * gridDim.x, acc, F);
   __syncthreads();  // the pair slots are free again
   pp_warp_sums<L, K>(acc, P, smem, F);
-  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, s_sm, &is_last)) return;
-  finish_round<L, K>(A, E, F, s_sm, g_sm, r_sm);
+  if (!grid_sums<L>(smem, d, blockIdx.x, gridDim.x, A.sums, A.st.counter, end)) return;
+  finish_round<L, K>(A, E, F, end);
 }
 
 }  // namespace sc

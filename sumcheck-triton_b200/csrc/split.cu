@@ -24,8 +24,8 @@ constexpr uint64_t kSplitSkip1MinPairs = uint64_t{1} << 12;
 template <int L, int K>
 __global__ void split_commit_kernel(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F,
                                     const uint32_t* parts, int world) {
-  __shared__ __align__(16) uint32_t g_sm[kMaxPoints * kMaxLimbs];
-  __shared__ uint32_t r_sm[L];
+  __shared__ RoundEnd<L> end;
+  uint32_t* const g_sm = end.g();
   const int lane = threadIdx.x;
   const int d = E.degree;
   if (lane <= d) {
@@ -47,7 +47,9 @@ __global__ void split_commit_kernel(const RoundArgs A, const ExprDev E, const Fi
     st_fe<L>(g_sm + lane * L, g);
   }
   __syncwarp();
-  finalize_round<L, K>(A, E, F, g_sm, r_sm);
+  begin_message<L>(end, d, A.round, lane, 32);
+  __syncwarp();
+  finalize_round<L, K>(A, E, F, load_end_consts<L>(*A.fc), end);
 }
 
 }  // namespace
