@@ -93,7 +93,7 @@ struct KernelSetup {
   static int run(int kmax, int threads_req, int sm_count, int* threads_out, int* grid_out, size_t* smem_out) {
 
     int threads = std::min(threads_req ? threads_req : kernel_threads(L), kernel_threads(L));
-    const int per_thread = round_smem_words_per_thread(kmax, L) * 4;
+    const int per_thread = round_smem_words_per_thread(kmax, L, D) * 4;
     while (threads > 32 && static_cast<size_t>(threads) * per_thread > static_cast<size_t>(kMaxDynSmem)) threads -= 32;
     const size_t smem = static_cast<size_t>(threads) * per_thread;
     SC_CUDA(cudaFuncSetAttribute(batch_round_kernel<L, K, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
@@ -144,7 +144,9 @@ inline int dispatch_dmax(int L, int K, int dmax, Args&&... args) {
     case 4:
       return K == kFieldMersenne127 ? dispatch_dmax_l<Fn, 4, kFieldMersenne127>(dmax, args...)
                                     : dispatch_dmax_l<Fn, 4, kFieldGeneric>(dmax, args...);
-    default: return dispatch_dmax_l<Fn, 8, kFieldGeneric>(dmax, args...);
+    default:
+      return K == kFieldBls381 ? dispatch_dmax_l<Fn, 8, kFieldBls381>(dmax, args...)
+                               : dispatch_dmax_l<Fn, 8, kFieldGeneric>(dmax, args...);
   }
 }
 

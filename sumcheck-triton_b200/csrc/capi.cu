@@ -111,7 +111,7 @@ struct ProveRun {
       smem = static_cast<size_t>(pp_smem_words(threads, K_, L)) * 4;
       SC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
     } else if (shape == kShapeGeneric) {
-      const int per_thread = round_smem_words_per_thread(K_, L) * 4;
+      const int per_thread = round_smem_words_per_thread(K_, L, DMAX) * 4;
       while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
       smem = static_cast<size_t>(threads) * per_thread;
     } else {
@@ -648,7 +648,10 @@ int resume_folds(const sc_field* f, int n, int num_tables, const uint32_t* table
       return field_kind(f->hf.p, L) == kFieldMersenne127
                  ? fold_prefix<4, kFieldMersenne127>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream)
                  : fold_prefix<4, kFieldGeneric>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream);
-    default: return fold_prefix<8, kFieldGeneric>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream);
+    default:
+      return field_kind(f->hf.p, L) == kFieldBls381
+                 ? fold_prefix<8, kFieldBls381>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream)
+                 : fold_prefix<8, kFieldGeneric>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream);
   }
 }
 

@@ -148,6 +148,8 @@ inline int field_kind(const uint32_t* p, int L) {
   if (L == 2 && p[0] == 1u && p[1] == 0xFFFFFFFFu) return kFieldGoldilocks;
   if (L == 4 && p[0] == 0xFFFFFFFFu && p[1] == 0xFFFFFFFFu && p[2] == 0xFFFFFFFFu && p[3] == 0x7FFFFFFFu)
     return kFieldMersenne127;
+  constexpr Words8 bls = bls381_p();
+  if (L == 8 && std::equal(bls.w, bls.w + 8, p)) return kFieldBls381;
   return kFieldGeneric;
 }
 
@@ -171,15 +173,17 @@ inline int dispatch(int L, int K, int dclass, Args&&... args) {
     case 4:
       return K == kFieldMersenne127 ? dispatch_degree<Fn, 4, kFieldMersenne127>(dclass, args...)
                                     : dispatch_degree<Fn, 4, kFieldGeneric>(dclass, args...);
-    default: return dispatch_degree<Fn, 8, kFieldGeneric>(dclass, args...);
+    default:
+      return K == kFieldBls381 ? dispatch_degree<Fn, 8, kFieldBls381>(dclass, args...)
+                               : dispatch_degree<Fn, 8, kFieldGeneric>(dclass, args...);
   }
 }
 
 // Calls Fn for every instantiation (set-up of kernel attributes).
 template <template <int, int, int> class Fn>
 inline int for_each_instance() {
-  const int combos[6][2] = {{1, kFieldGeneric}, {2, kFieldGeneric}, {2, kFieldGoldilocks},
-                            {4, kFieldGeneric}, {4, kFieldMersenne127}, {8, kFieldGeneric}};
+  const int combos[7][2] = {{1, kFieldGeneric}, {2, kFieldGeneric}, {2, kFieldGoldilocks}, {4, kFieldGeneric},
+                            {4, kFieldMersenne127}, {8, kFieldGeneric}, {8, kFieldBls381}};
   for (const auto& c : combos)
     for (int dc : {2, 4, 7}) {
       const int rc = dispatch<Fn>(c[0], c[1], dc);
@@ -245,18 +249,6 @@ inline int mul_cost(int L, int K) {
   return K == kFieldGoldilocks ? 16 : (K == kFieldMersenne127 ? 60 : (L == 1 ? 10 : 4 * L * L + 8 * L));
 }
 inline int add_cost(int L) { return 3 * L + 4; }
-
-// Whether a term of length len in an expression of degree d is cheaper evaluated at points
-// 0..len and extrapolated by forward differences than evaluated at every finite point 0..d - 1
-// (a shorter term has no part in the leading coefficient that stands for point d).
-inline bool extrapolate_term(int len, int d, int L, int K) {
-  const int fin = d - 1;
-  if (len >= fin) return false;
-  const int m = mul_cost(L, K), a = add_cost(L);
-  const int direct = (len - 1) * (fin + 1) * m + len * fin * a;
-  const int extrap = (len - 1) * (len + 1) * m + len * len * a + (len * (len + 1) / 2 + fin * len) * a;
-  return extrap < direct;
-}
 
 // Matches the expression against the compile-time shapes (prover.cuh: Shape). Returns the
 // shape (kShapeGeneric when none matches) and fills role[] with the table of every role.
@@ -346,7 +338,6 @@ inline void build_expr_dev(const sc_expr& ex, const sc_field& f, ExprDev& E) {
   E.degree = ex.degree;
   const HostField& hf = f.hf;
   const int K = field_kind(hf.p, L);
-  for (int i = 0; i < ex.num_terms; ++i) E.term_extrap[i] = extrapolate_term(ex.lens[i], ex.degree, L, K) ? 1 : 0;
   const int mul_cost = ::sc_host::mul_cost(L, K), add_cost = ::sc_host::add_cost(L);
   for (int i = 0; i < ex.num_terms; ++i) {
     E.term_len[i] = static_cast<uint8_t>(ex.lens[i]);

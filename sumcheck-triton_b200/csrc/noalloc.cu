@@ -76,7 +76,7 @@ static int run(sc_ctx* ctx, const sc_field* f, const sc_expr* ex, int n, const u
   int rc;
   if ((rc = noalloc_scratch(ctx->device, &base))) return rc;  // first call on a device: set-up
   int threads = kernel_threads(L);
-  const int per_thread = round_smem_words_per_thread(K_, L) * 4;
+  const int per_thread = round_smem_words_per_thread(K_, L, DMAX) * 4;
   while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
   const size_t smem = static_cast<size_t>(threads) * per_thread;
   int bps = 0;

@@ -10,7 +10,7 @@
 //      field_sumcheck.cu:326-348) and evaluates the constraint at each point
 //      (field_sumcheck.cu:389-590) and, in the place of point d, its leading coefficient,
 //      accumulating d+1 sums per thread (see eval_pair for the exact-arithmetic shortcuts:
-//      extrapolated low-degree terms, g(1) from the claim);
+//      factors taken in pairs, g(1) from the claim);
 //   3. reduce: the point sums are summed word by word as integers -- over the warp, the block
 //      (shared memory) and the grid (64-bit atomic adds) -- with no modular arithmetic until
 //      the last block to finish (atomic ticket) reads (d + 1) L integers and reduces them
@@ -78,7 +78,6 @@ struct ExprDev {
   uint8_t term_off[kMaxTerms];
   uint8_t flat[kMaxFlat];
   uint8_t coeff_kind[kMaxTerms];
-  uint8_t term_extrap[kMaxTerms];   // 1: evaluate points 0..len only, extrapolate the rest
   int32_t coeff_small[kMaxTerms];
   uint32_t coeff_mont[kMaxTerms][kMaxLimbs];
   int32_t shape;                    // Shape the host matched (kShapeGeneric: none)
@@ -223,24 +222,33 @@ __device__ __forceinline__ Fe<L> lz_mul(const Fe<L>& a, const Fe<L>& b, const Fi
   else return fe_mul(a, b, F);
 }
 template <bool LZ, int L, int K>
+__device__ __forceinline__ void lz_mul2(Fe<L>& r0, const Fe<L>& a0, const Fe<L>& b0, Fe<L>& r1, const Fe<L>& a1,
+                                        const Fe<L>& b1, const FieldParams<L, K>& F) {
+  if constexpr (LZ) {
+    const Fe<L> x = gl_mul(a0, b0, gold_k(F));
+    r1 = gl_mul(a1, b1, gold_k(F));
+    r0 = x;
+  } else {
+    fe_mul2(r0, a0, b0, r1, a1, b1, F);
+  }
+}
+template <bool LZ, int L, int K>
 __device__ __forceinline__ Fe<L> lz_add_or_sub(const Fe<L>& acc, const Fe<L>& x, bool neg, const FieldParams<L, K>& F) {
   return neg ? lz_sub<LZ>(acc, x, F) : lz_add<LZ>(acc, x, F);
 }
 
 // One pair: acc[t] += expression at point t, for the finite points t (0..d - 1, or 0 and 1 for
 // d = 1; 1 skipped when skip1), and acc[DMAX] += its coefficient of t^d (make_point_weights).
-// The values and differences of every table are in shared memory (this thread's slots).
+// get(k, e, o) gives table k's values at 0 and 1; add(slot, x, neg) adds to a sum.
 //
-// A term of len factors is a polynomial of degree len in t. Evaluated at points 0..last
-// (the last finite point, or len when the host marked the term for extrapolation), each point costs len-1
-// products: the factors' values are stepped point to point by one addition of the
-// difference. An extrapolated term's further points come from its forward differences
-// (len(len+1)/2 subtractions, then len additions per step) -- exact, since the term is a
-// polynomial of degree len; the host marks a term only where that is cheaper than the
-// products it replaces. With skip1, point 1 of a directly evaluated term is never formed.
-template <int L, int K, int DMAX>
-__device__ __forceinline__ void eval_pair(const ExprDev& E, const uint32_t* sv, const uint32_t* sd, int tid, int nthr,
-                                          bool skip1, Fe<L> (&acc)[DMAX + 1], const FieldParams<L, K>& F) {
+// A term's factors are taken two at a time where that saves products (more than three points):
+// the product of two is a quadratic, known from its values at 0 and 1 and its leading
+// coefficient (three products) and stepped from point to point by two additions, so each
+// further point costs one product for the two factors instead of two. Six factors at six points take
+// 21 products instead of 30, four at four points 10 instead of 12.
+template <int L, int K, int DMAX, typename Get, typename Add, typename Prod>
+__device__ __forceinline__ void eval_pair(const ExprDev& E, Get get, Add add, Prod& prod, bool skip1,
+                                          const FieldParams<L, K>& F) {
   constexpr bool LZ = lazy_generic<L, K>();
   const int d = E.degree;
   const int fin = d >= 2 ? d - 1 : 1;  // last finite point
@@ -248,110 +256,160 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, const uint32_t* sv, 
     const int off = E.term_off[i];
     const int len = E.term_len[i];
     const int kind = E.coeff_kind[i];
-    const bool extrap = E.term_extrap[i] != 0;
     const bool full = len == d && d >= 2;
-    const int last = extrap ? len : fin;
-    const bool skip_t1 = skip1 && !extrap;
+    const bool paired = fin + 1 - (skip1 ? 1 : 0) + (full ? 1 : 0) > 3;  // points the term is needed at
     const bool neg = kind == kCoeffMinus || (kind == kCoeffSmall && E.coeff_small[i] < 0);
-    Fe<L> prod[DMAX], lead;
-    {
-      const int k0 = E.flat[off];
-      Fe<L> v = sm_get<L>(sv, k0, tid, nthr);
-      Fe<L> df = sm_get<L>(sd, k0, tid, nthr);
-      if (kind == kCoeffSmall) {
-        const int32_t c = E.coeff_small[i];
-        const uint32_t m = c < 0 ? static_cast<uint32_t>(-static_cast<int64_t>(c)) : static_cast<uint32_t>(c);
-        v = fe_mul_small(v, m, F);
-        df = fe_mul_small(df, m, F);
-      } else if (kind == kCoeffMont) {
-        Fe<L> cm;
+    Fe<L> prod0, lead;
+    for (int f = 0; f < len;) {
+      // this step's factor, or the product of two: v(0), v(1) - v(0), the step's step, and the
+      // leading coefficient
+      Fe<L> v, v1;
+      get(E.flat[off + f], v, v1);
+      if (f == 0) {
+        if (kind == kCoeffSmall) {
+          const int32_t c = E.coeff_small[i];
+          const uint32_t m = c < 0 ? static_cast<uint32_t>(-static_cast<int64_t>(c)) : static_cast<uint32_t>(c);
+          v = fe_mul_small(v, m, F);
+          v1 = fe_mul_small(v1, m, F);
+        } else if (kind == kCoeffMont) {
+          Fe<L> cm;
 #pragma unroll
-        for (int l = 0; l < L; ++l) cm.w[l] = E.coeff_mont[i][l];
-        v = fe_mul(v, cm, F);
-        df = fe_mul(df, cm, F);
+          for (int l = 0; l < L; ++l) cm.w[l] = E.coeff_mont[i][l];
+          fe_mul2(v, v, cm, v1, v1, cm, F);
+        }
       }
-      lead = df;
+      Fe<L> li = fe_sub(v1, v, F), df = li, dd = fe_zero<L>();
+      const bool two = paired && f + 1 < len;
+      if (two) {
+        Fe<L> w, w1;
+        get(E.flat[off + f + 1], w, w1);
+        li = fe_mul(li, fe_sub(w1, w, F), F);
+        fe_mul2(v, v, w, v1, v1, w1, F);
+        df = fe_sub(v1, v, F);
+        dd = fe_add(li, li, F);
+      }
+      // products two points at a time: the leading coefficient with point 0, then 1 | 2, 3 | ..
+      if (f == 0) {
+        if (full) lead = li;
+        prod0 = v;
+      } else if (full) {
+        lz_mul2<LZ>(lead, lead, li, prod0, prod0, v, F);
+      } else {
+        prod0 = lz_mul<LZ>(prod0, v, F);
+      }
+      auto step = [&]() {
+        v = lz_add_c<LZ>(v, df, F);
+        if (two) df = fe_add(df, dd, F);
+      };
 #pragma unroll
-      for (int t = 0; t < DMAX; ++t) {
-        if (t > last) break;
-        prod[t] = v;
-        if (t < last) v = lz_add_c<LZ>(v, df, F);
+      for (int t = 1; t < DMAX; t += 2) {  // t odd, then t + 1
+        if (t > fin) break;
+        step();
+        const Fe<L> va = v;
+        const bool odd = !(skip1 && t == 1), even = t + 1 < DMAX && t + 1 <= fin;
+        const int u = t + 1 < DMAX ? t + 1 : t;
+        if (even) step();
+        if (f == 0) {
+          prod.set(t, va);
+          if (even) prod.set(u, v);
+        } else if (odd && even) {
+          Fe<L> x, y;
+          lz_mul2<LZ>(x, prod.get(t), va, y, prod.get(u), v, F);
+          prod.set(t, x);
+          prod.set(u, y);
+        } else if (odd) {
+          prod.set(t, lz_mul<LZ>(prod.get(t), va, F));
+        } else if (even) {
+          prod.set(u, lz_mul<LZ>(prod.get(u), v, F));
+        }
       }
+      f += two ? 2 : 1;
     }
-    for (int f = 1; f < len; ++f) {
-      const int k = E.flat[off + f];
-      Fe<L> v = sm_get<L>(sv, k, tid, nthr);
-      const Fe<L> df = sm_get<L>(sd, k, tid, nthr);
-      if (full) lead = lz_mul<LZ>(lead, df, F);
+    if (full) add(DMAX, lead, neg);
+    add(0, prod0, neg);
 #pragma unroll
-      for (int t = 0; t < DMAX; ++t) {
-        if (t > last) break;
-        if (!(skip_t1 && t == 1)) prod[t] = lz_mul<LZ>(prod[t], v, F);
-        if (t < last) v = lz_add_c<LZ>(v, df, F);
-      }
-    }
-    if (full) acc[DMAX] = lz_add_or_sub<LZ>(acc[DMAX], lead, neg, F);
-#pragma unroll
-    for (int t = 0; t < DMAX; ++t) {
-      if (t > last) break;
+    for (int t = 1; t < DMAX; ++t) {
+      if (t > fin) break;
       if (skip1 && t == 1) continue;
-      acc[t] = lz_add_or_sub<LZ>(acc[t], prod[t], neg, F);
-    }
-    if (extrap && len < fin) {
-      // forward differences at 0, in place: prod[m] = Delta^m p(0)
-#pragma unroll
-      for (int m = 1; m < DMAX; ++m) {
-        if (m > len) break;
-#pragma unroll
-        for (int t = DMAX - 1; t >= 1; --t) {
-          if (t > len || t < m) continue;
-          prod[t] = lz_sub<LZ>(prod[t], prod[t - 1], F);
-        }
-      }
-      // step forward: after s steps prod[0] = p(s)
-#pragma unroll
-      for (int s = 1; s < DMAX; ++s) {
-        if (s > fin) break;
-#pragma unroll
-        for (int m = 0; m < DMAX - 1; ++m) {
-          if (m >= len) break;
-          prod[m] = lz_add<LZ>(prod[m], prod[m + 1], F);
-        }
-        if (s > len && !(skip1 && s == 1)) acc[s] = lz_add_or_sub<LZ>(acc[s], prod[0], neg, F);
-      }
+      add(t, prod.get(t), neg);
     }
   }
 }
 
-template <int L, int K>
-__device__ __forceinline__ Fe<L> shape_value(const Fe<L> (&v)[9], const FieldParams<L, K>& F,
-                                             std::integral_constant<int, kShapeZerocheck>) {
-  const Fe<L> u = fe_add(v[0], fe_mul(v[5], v[4], F), F);  // S1 + M X2
-  Fe<L> s = fe_mul(v[1], u, F);                            // X1 (S1 + M X2)
-  s = fe_add(s, fe_mul(v[3], v[4], F), F);                 // + S2 X2
-  s = fe_sub(s, fe_mul(v[6], v[7], F), F);                 // - S4 X3
-  s = fe_add(s, v[8], F);                                  // + S5
-  return fe_mul(v[2], s, F);                               // F (...)
-}
+// A term's products at points 1..DMAX - 1: in registers, or in this thread's shared-memory slots.
+template <int L, int DMAX>
+struct RegProducts {
+  Fe<L> a[DMAX];
+  __device__ __forceinline__ Fe<L> get(int t) const { return a[t]; }
+  __device__ __forceinline__ void set(int t, const Fe<L>& x) { a[t] = x; }
+};
+template <int L>
+struct SmProducts {
+  uint32_t* sm;
+  int tid, nthr;
+  __device__ __forceinline__ Fe<L> get(int t) const { return sm_get<L>(sm, t - 1, tid, nthr); }
+  __device__ __forceinline__ void set(int t, const Fe<L>& x) { sm_put<L>(sm, t - 1, tid, nthr, x); }
+};
 
-template <int L, int K>
-__device__ __forceinline__ Fe<L> shape_value(const Fe<L> (&v)[6], const FieldParams<L, K>& F,
+// Where the generic evaluator keeps a pair's tables, a term's products and a thread's point sums.
+// Fields of up to 4 limbs stage the tables' values in shared memory and hold products and sums
+// in registers. At 8 limbs those are 8 words each: the tables are read from memory at every use
+// (T_j from L2, where this thread has just written it) and shared memory takes the products and
+// sums instead, which leaves 128 registers and 4 blocks an SM up to degree 4. Measured on B200, 64 mixed
+// proofs: 4.84 ms, against 4.99 with the products in registers (3 blocks) and 5.10 with the
+// tables staged and both in registers; at 4 limbs 40 served requests took 7.18 ms staged, 7.30
+// from memory.
+__host__ __device__ constexpr bool streamed_tables(int L) { return L >= 8; }
+
+// Shape kernels hold a pair's tables in role order. shape_value is the formula at one point,
+// shape_value2 at two points, their products side by side; value(i) and value2(i) give role
+// i's value. shape_ends is point 0 and the leading coefficient (from the tables' differences,
+// the term of full degree alone).
+template <int L, int K, typename V>
+__device__ __forceinline__ Fe<L> shape_value(V v, const FieldParams<L, K>& F, std::integral_constant<int, kShapeZerocheck>) {
+  const Fe<L> u = fe_add(v(0), fe_mul(v(5), v(4), F), F);  // S1 + M X2
+  Fe<L> s = fe_mul(v(1), u, F);                            // X1 (S1 + M X2)
+  s = fe_add(s, fe_mul(v(3), v(4), F), F);                 // + S2 X2
+  s = fe_sub(s, fe_mul(v(6), v(7), F), F);                 // - S4 X3
+  s = fe_add(s, v(8), F);                                  // + S5
+  return fe_mul(v(2), s, F);                               // F (...)
+}
+template <int L, int K, typename V>
+__device__ __forceinline__ Fe<L> shape_value(V v, const FieldParams<L, K>& F, std::integral_constant<int, kShapeAbcg>) {
+  Fe<L> ab, de;
+  fe_mul2(ab, v(0), v(1), de, v(4), v(5), F);
+  return fe_mul(v(3), fe_add(fe_mul(ab, v(2), F), de, F), F);
+}
+template <int L, int K, typename V, typename W>
+__device__ __forceinline__ void shape_value2(V v, W w, Fe<L>& x, Fe<L>& y, const FieldParams<L, K>& F,
+                                             std::integral_constant<int, kShapeZerocheck> shape) {
+  x = shape_value<L, K>(v, F, shape);
+  y = shape_value<L, K>(w, F, shape);
+}
+template <int L, int K, typename V, typename W>
+__device__ __forceinline__ void shape_value2(V v, W w, Fe<L>& x, Fe<L>& y, const FieldParams<L, K>& F,
                                              std::integral_constant<int, kShapeAbcg>) {
-  const Fe<L> s = fe_add(fe_mul(fe_mul(v[0], v[1], F), v[2], F), fe_mul(v[4], v[5], F), F);
-  return fe_mul(v[3], s, F);
+  Fe<L> p, q;
+  fe_mul2(x, v(0), v(1), y, w(0), w(1), F);
+  fe_mul2(x, x, v(2), y, y, w(2), F);
+  fe_mul2(p, v(4), v(5), q, w(4), w(5), F);
+  x = fe_add(x, p, F);
+  y = fe_add(y, q, F);
+  fe_mul2(x, x, v(3), y, y, w(3), F);
 }
-
-// Their coefficients of t^4 from the tables' differences: the term of full degree alone.
-template <int L, int K>
-__device__ __forceinline__ Fe<L> shape_lead(const Fe<L> (&d)[9], const FieldParams<L, K>& F,
-                                            std::integral_constant<int, kShapeZerocheck>) {
-  return fe_mul(fe_mul(d[2], d[1], F), fe_mul(d[4], d[5], F), F);  // F X1 X2 M
+template <int L, int K, typename V, typename D>
+__device__ __forceinline__ void shape_ends(V v, D d, Fe<L>& x, Fe<L>& lead, const FieldParams<L, K>& F,
+                                           std::integral_constant<int, kShapeZerocheck> shape) {
+  x = shape_value<L, K>(v, F, shape);
+  lead = fe_mul(fe_mul(d(2), d(1), F), fe_mul(d(4), d(5), F), F);  // F X1 X2 M
 }
-
-template <int L, int K>
-__device__ __forceinline__ Fe<L> shape_lead(const Fe<L> (&d)[6], const FieldParams<L, K>& F,
-                                            std::integral_constant<int, kShapeAbcg>) {
-  return fe_mul(fe_mul(d[0], d[1], F), fe_mul(d[2], d[3], F), F);  // A B C G
+template <int L, int K, typename V, typename D>
+__device__ __forceinline__ void shape_ends(V v, D d, Fe<L>& x, Fe<L>& lead, const FieldParams<L, K>& F,
+                                           std::integral_constant<int, kShapeAbcg>) {
+  fe_mul2(x, v(0), v(1), lead, d(0), d(1), F);
+  fe_mul2(x, x, v(2), lead, lead, d(2), F);
+  x = fe_add(x, fe_mul(v(4), v(5), F), F);
+  fe_mul2(x, x, v(3), lead, lead, d(3), F);  // G (A B C + D E); A B C G
 }
 
 __device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[9], const GoldK k,
@@ -461,6 +519,11 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
     return;
   }
   const int tid = threadIdx.x, nthr = blockDim.x;
+  constexpr bool kStream = SHAPE == kShapeGeneric && streamed_tables(L);
+  if constexpr (kStream) {
+#pragma unroll
+    for (int t = 0; t <= DMAX; ++t) sm_put<L>(sv, t, tid, nthr, fe_zero<L>());
+  }
   constexpr int NR = SHAPE == kShapeGeneric ? 1 : shape_tables(SHAPE);
   constexpr bool kGoldLazy = SHAPE != kShapeGeneric && L == 2 && K == kFieldGoldilocksFma && SC_GOLD_LAZY;
   constexpr bool kAsync = (kGoldLazy && SC_GOLD_ASYNC) || l8_async_stage(L, SHAPE);
@@ -566,7 +629,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
     } else
 #endif
 #pragma unroll (SHAPE == kShapeGeneric ? 1 : NR)
-    for (int i = 0; i < nv; ++i) {
+    for (int i = 0; i < (kStream && !fold ? 0 : nv); ++i) {
       const int k = SHAPE == kShapeGeneric ? i : E.role[i];
       Fe<L> e, o;
       if (fold) {
@@ -576,8 +639,9 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
           const uint4 v = __ldcs(reinterpret_cast<const uint4*>(src + (static_cast<uint64_t>(k) * L + l) * src_len) + q);
           x0.w[l] = v.x; x1.w[l] = v.y; x2.w[l] = v.z; x3.w[l] = v.w;
         }
-        e = fe_add(x0, fe_mul(r_prev, fe_sub(x1, x0, F), F), F);
-        o = fe_add(x2, fe_mul(r_prev, fe_sub(x3, x2, F), F), F);
+        fe_mul2(e, r_prev, fe_sub(x1, x0, F), o, r_prev, fe_sub(x3, x2, F), F);
+        e = fe_add(x0, e, F);
+        o = fe_add(x2, o, F);
         const uint64_t dst_len = src_len >> 1;
 #pragma unroll
         for (int l = 0; l < L; ++l)
@@ -590,15 +654,43 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
         }
       }
       if constexpr (SHAPE == kShapeGeneric) {
-        sm_put<L>(sv, k, tid, nthr, e);
-        sm_put<L>(sd, k, tid, nthr, fe_sub(o, e, F));
+        if constexpr (!kStream) {
+          sm_put<L>(sv, k, tid, nthr, e);
+          sm_put<L>(sd, k, tid, nthr, o);
+        }
       } else {
         sh_v[i] = e;
         sh_d[i] = o;  // o for now: the difference is formed below
       }
     }
-    if constexpr (SHAPE == kShapeGeneric) {
-      eval_pair<L, K, DMAX>(E, sv, sd, tid, nthr, skip1, acc, F);
+    if constexpr (kStream) {
+      SmProducts<L> products{sv + (DMAX + 1) * L * nthr, tid, nthr};
+      const uint32_t* const tab = fold ? dst : src;
+      const uint64_t len = fold ? src_len >> 1 : src_len;
+      eval_pair<L, K, DMAX>(
+          E,
+          [&](int k, Fe<L>& e, Fe<L>& o) {
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+              const uint2 w = reinterpret_cast<const uint2*>(tab + (static_cast<uint64_t>(k) * L + l) * len)[q];
+              e.w[l] = w.x;
+              o.w[l] = w.y;
+            }
+          },
+          [&](int t, const Fe<L>& x, bool neg) {
+            sm_put<L>(sv, t, tid, nthr, add_or_sub(sm_get<L>(sv, t, tid, nthr), x, neg, F));
+          },
+          products, skip1, F);
+    } else if constexpr (SHAPE == kShapeGeneric) {
+      RegProducts<L, DMAX> products;
+      eval_pair<L, K, DMAX>(
+          E,
+          [&](int k, Fe<L>& e, Fe<L>& o) {
+            e = sm_get<L>(sv, k, tid, nthr);
+            o = sm_get<L>(sd, k, tid, nthr);
+          },
+          [&](int t, const Fe<L>& x, bool neg) { acc[t] = lz_add_or_sub<lazy_generic<L, K>()>(acc[t], x, neg, F); },
+          products, skip1, F);
     } else if constexpr (kGoldLazy) {
       // as below, in lazy arithmetic: sh_v / sh_d arrive canonical, the differences are
       // canonical, the stepped values and the point sums are any representatives
@@ -625,10 +717,13 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
         acc[t] = gl_add(acc[t], shape_value_lazy(sh_v, gk, shape), gk);
       }
     } else {
-      // point 0: e; point 1: o (skipped when skip1); then v(t) = v(t - 1) + (o - e)
-      constexpr int D = 4;
-      static_assert(DMAX == D, "shape kernels evaluate degree-4 shapes");
-      acc[0] = fe_add(acc[0], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
+      // sh_v: the values at 0, sh_d: at 1; then the values at 1 and the differences
+      static_assert(DMAX == 4, "shape kernels evaluate degree-4 shapes");
+      const std::integral_constant<int, SHAPE> shape{};
+      Fe<L> x, y;
+      shape_ends<L, K>([&](int i) { return sh_v[i]; }, [&](int i) { return fe_sub(sh_d[i], sh_v[i], F); }, x, y, F, shape);
+      acc[0] = fe_add(acc[0], x, F);
+      acc[4] = fe_add(acc[4], y, F);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const Fe<L> o = sh_d[r];
@@ -638,15 +733,16 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       if constexpr (kAsync) {
         if (!fold && q + stride < last) issue(q + stride);
       }
-      acc[D] = fe_add(acc[D], shape_lead<L, K>(sh_d, F, std::integral_constant<int, SHAPE>{}), F);
-      if (!skip1) acc[1] = fe_add(acc[1], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
-#pragma unroll
-      for (int t = 2; t < D; ++t) {
-#pragma unroll
-        for (int r = 0; r < NR; ++r) sh_v[r] = fe_add(sh_v[r], sh_d[r], F);
-        acc[t] = fe_add(acc[t], shape_value<L, K>(sh_v, F, std::integral_constant<int, SHAPE>{}), F);
-      }
+      if (!skip1) acc[1] = fe_add(acc[1], shape_value<L, K>([&](int i) { return sh_v[i]; }, F, shape), F);
+      shape_value2<L, K>([&](int i) { return fe_add(sh_v[i], sh_d[i], F); },
+                         [&](int i) { return fe_add(fe_add(sh_v[i], sh_d[i], F), sh_d[i], F); }, x, y, F, shape);
+      acc[2] = fe_add(acc[2], x, F);
+      acc[3] = fe_add(acc[3], y, F);
     }
+  }
+  if constexpr (kStream) {
+#pragma unroll
+    for (int t = 0; t <= DMAX; ++t) acc[t] = sm_get<L>(sv, t, tid, nthr);
   }
   if constexpr (SHAPE == kShapeGeneric) {  // the leading coefficient belongs in slot d
     const int d = E.degree;
@@ -1057,8 +1153,11 @@ __device__ __forceinline__ void finish_round(const RoundArgs& A, const ExprDev& 
   finish_round<L, K>(A, E, F, load_end_consts<L>(*A.fc), [&](int i) { return end.s[i]; }, end);
 }
 
-// Dynamic shared memory per thread: values and differences of every table.
-__host__ __device__ constexpr int round_smem_words_per_thread(int K, int L) { return 2 * K * L; }
+// Dynamic shared memory per thread of the generic evaluator: both values of every table, or the
+// point sums.
+__host__ __device__ constexpr int round_smem_words_per_thread(int K, int L, int dmax) {
+  return streamed_tables(L) ? 2 * dmax * L : 2 * K * L;
+}
 
 // Launch shape per limb count: 8-limb kernels hold (DMAX + 1) x 8-word point arrays per
 // thread, so they run 128-thread blocks and ask the compiler for at least 3 blocks per SM
@@ -1103,16 +1202,11 @@ __host__ __device__ constexpr int kernel_min_blocks(int L) {
 #ifndef SC_SHAPE_L8_MIN_BLOCKS
 #define SC_SHAPE_L8_MIN_BLOCKS 2
 #endif
-// The batched kernel per limb count and degree class: the 8-limb classes of degree 6-7 hold
-// 7-8 points of 8-limb accumulators and products in registers.
-#ifndef SC_BATCH_L8_HIGH_MIN_BLOCKS
-#define SC_BATCH_L8_HIGH_MIN_BLOCKS SC_L8_MIN_BLOCKS
-#endif
-#ifndef SC_BATCH_L8_HIGH_DMAX
-#define SC_BATCH_L8_HIGH_DMAX 6
-#endif
+// The batched kernel per limb count and degree class: at 8 limbs 4 blocks/SM up to degree 4
+// (128 registers), 3 above (shared memory for 7-8 points' products and sums). 5 and 4 blocks
+// spilled more than they hid (64 mixed proofs 5.09 ms against 4.84; 3 and 3 blocks 4.99).
 __host__ __device__ constexpr int batch_min_blocks(int L, int dmax) {
-  return (L >= 8 && dmax >= SC_BATCH_L8_HIGH_DMAX) ? SC_BATCH_L8_HIGH_MIN_BLOCKS : kernel_min_blocks(L);
+  return L >= 8 && dmax <= 4 ? 4 : kernel_min_blocks(L);
 }
 __host__ __device__ constexpr int round_min_blocks(int L, int shape) {
   return (shape != 0 && L <= 2) ? SC_SHAPE_MIN_BLOCKS
@@ -1128,8 +1222,8 @@ __global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
   const int tid = threadIdx.x;
   const int nthr = blockDim.x;
   const int d = E.degree;
-  uint32_t* sv = smem;                           // [K][L][nthr] values at the current point
-  uint32_t* sd = smem + E.num_vars * L * nthr;   // [K][L][nthr] differences o - e
+  uint32_t* sv = smem;                           // [K][L][nthr] values at 0 (or the point sums)
+  uint32_t* sd = smem + E.num_vars * L * nthr;   // [K][L][nthr] values at 1
 
   pdl_begin();
   Fe<L> acc[DMAX + 1];

@@ -886,7 +886,7 @@ int sc_server_create(int device, const sc_field* field, int policy, uint64_t hbm
   // one tile size for every class (a request's partial slots are sized by it)
   int cls_threads = kernel_threads(S->L);
   if (threads) cls_threads = std::min(threads, cls_threads);
-  const int per_thread = round_smem_words_per_thread(max_tables, S->L) * 4;
+  const int per_thread = round_smem_words_per_thread(max_tables, S->L, 7) * 4;
   while (cls_threads > 32 && static_cast<size_t>(cls_threads) * per_thread > static_cast<size_t>(kMaxDynSmem)) cls_threads -= 32;
   S->tile_pairs = cls_threads * S->ppt;
   int max_grid = 1;

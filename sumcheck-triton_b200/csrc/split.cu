@@ -102,7 +102,7 @@ struct SplitSetup {
     if (S->E.shape != kShapeGeneric && D == 4) {
       S->smem = shape_round_smem_bytes(L, K, S->E.shape, threads);  // reduction scratch (+ the pair stage)
     } else {
-      const int per_thread = round_smem_words_per_thread(S->K, L) * 4;
+      const int per_thread = round_smem_words_per_thread(S->K, L, D) * 4;
       while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
       S->smem = static_cast<size_t>(threads) * per_thread;
     }
