@@ -36,7 +36,7 @@ struct BatchRound {
 
 struct BatchItem {
   int32_t round;       // index into the tick's BatchRound array
-  int32_t pad;
+  int32_t lgP;         // >= 0: a small part of 2^lgP pairs, spread over the block (tail.cuh); -1: not
   uint64_t start;      // pairs [start, start + count)
   uint64_t count;
 };
@@ -54,16 +54,15 @@ struct BatchTickArgs {
 // prove_tail out of line: the tick's own register budget does not see it.
 template <int L, int K>
 __device__ __noinline__ void batch_tail(RoundArgs* A, const ExprDev* E, const FieldParams<L, K> F, int rounds,
-                                        bool r_ready, bool store, uint32_t* smem, RoundEnd<L>* end) {
-  prove_tail<L, K>(*A, *E, F, rounds, r_ready, store, smem, *end);
+                                        uint32_t* smem, RoundEnd<L>* end) {
+  prove_tail<L, K>(*A, *E, F, rounds, true, false, smem, *end);
 }
 
-// Whole rounds of at most this many pairs are spread over their block's threads (tail.cuh)
-// instead of a thread walking through each pair. TICK_FIGURES
-#ifndef SC_TICK_SMALL
-#define SC_TICK_SMALL 32
-#endif
-constexpr uint64_t kSmallRoundPairs = SC_TICK_SMALL;
+template <int L, int K>
+__device__ __noinline__ void batch_part(const RoundArgs* A, const ExprDev* E, const FieldParams<L, K> F, int lgP,
+                                        uint32_t part, uint32_t parts, uint32_t* smem, RoundEnd<L>* end) {
+  prove_part<L, K>(*A, *E, F, lgP, part, parts, smem, *end);
+}
 
 // finish_round out of line, for the same reason.
 template <int L, int K>
@@ -114,11 +113,14 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
     uint32_t* sd = smem + E.num_vars * L * nthr;
     // k = 0: this item of the proof's round; k >= 1: the proof's tail rounds (only in the
     // block that finalised round k - 1; R.args then describes round R.args.round)
+    if (T.items && I.lgP >= 0) {
+      batch_part<L, K>(&R.args, &E, F, I.lgP, static_cast<uint32_t>(R.item_base + (it - R.first_item)),
+                       static_cast<uint32_t>(R.round_items), smem, &end);
+      continue;
+    }
     for (int k = 0;; ++k) {
-      const bool small = k > 0 || (R.round_items == 1 && R.args.pairs <= kSmallRoundPairs);
-      if (small && tail_smem_words(R.args.pairs, E.num_vars, L) * 4 <= dyn_bytes) {
-        batch_tail<L, K>(&R.args, &E, F, R.tail_rounds - k + 1, k > 0,
-                         R.tail_rounds == 0 && R.args.fold && R.args.round + 1 < R.args.num_rounds, smem, &end);
+      if (k > 0 && tail_smem_words(R.args.pairs, E.num_vars, L) * 4 <= dyn_bytes) {
+        batch_tail<L, K>(&R.args, &E, F, R.tail_rounds - k + 1, smem, &end);
         break;
       }
       Fe<L> acc[DMAX + 1];

@@ -6,7 +6,6 @@
 // (cuda/src/field_sumcheck.cu:1012-1088); here a proof is num_rounds launches of one
 // fused round kernel on the caller's stream and a single copy of the results at the end.
 #include "host_common.h"
-#include "prover_pp.cuh"
 
 using namespace sc;
 using namespace sc_host;
@@ -23,9 +22,8 @@ inline bool round_skip1(int n, int j) { return j >= 1 && (uint64_t{1} << (n - j 
 // Rounds of at most tail_pairs() pairs run in one block (tail.cuh): for a generic expression
 // one launch proves the rest of the proof, for the compile-time shapes a launch proves one
 // round. One SM's arithmetic bounds such a round from above, so the line falls with the work of
-// a pair (`units`: products of its folds and of its d + 1 points); a launch, the grid's sums
-// and a thread walking through a whole pair bound the other side, and at 8 limbs the
-// point-parallel kernel takes over earlier. Measured on B200, us a proof at n = 14 by the
+// a pair (`units`: products of its folds and of its d + 1 points); a launch and the grid's sums
+// bound the other side, and at 8 limbs several blocks are worth them earlier. Measured on B200, us a proof at n = 14 by the
 // largest round in one block (0: none):
 //   a b, 1 limb (7 units)               0: 153   32: 137   128: 136   256: 134   1024: 126
 //   permutation check, 2 limbs (80)     0: 286   32: 225   128: 222   256: 220   512: 238
@@ -46,6 +44,25 @@ inline uint64_t tail_pairs(const sc_expr& ex, int L, bool shaped) {
   while (!shaped && p > least && p * units > budget) p >>= 1;
   while (p && tail_smem_words(p, ex.num_vars, L) * 4 > static_cast<size_t>(kMaxDynSmem)) p >>= 1;
   return p;
+}
+
+// Rounds of more pairs than that, up to part_pairs(), are cut into parts of 32 to 128 pairs, a
+// block each (part_kernel): below a pair a thread on every SM, spreading a pair over threads is
+// faster than the register evaluator's sparing use of products. The 2-limb zerocheck shape's 5
+// products a point are never beaten. Measured on B200, us a proof by the largest round in parts
+// (0: none):
+//   n = 16  permutation check, 2 limbs   0: 261   2048: 244   4096: 236   8192: 227   32768: 227
+//           17-term gate, 4 limbs        0: 1265  2048: 942   4096: 884   8192: 843   32768: 931
+//           aabbc, 4 limbs               0: 251   2048: 238   4096: 230   8192: 226   32768: 225
+//           zerocheck shape, 2 limbs     0: 210   2048: 215   4096: 213   8192: 211   32768: 222
+//           g(abc + de) shape, 8 limbs   0: 442   2048: 389   4096: 384   8192: 382   32768: 382
+//   n = 18  12-term gate, 8 limbs        4096: 1677   16384: 1589   32768: 1546   131072: 1602
+//           17-term gate, 8 limbs        4096: 3789   16384: 3489   32768: 3547   131072: 4542
+//           a b, 8 limbs                 4096: 299    16384: 299    32768: 300    131072: 312
+//           g(abc + de) shape, 8 limbs   4096: 533    16384: 543    32768: 552    131072: 595
+inline uint64_t part_pairs(int L, bool shaped) {
+  if (L >= 8) return shaped ? 8192 : 32768;
+  return shaped ? 0 : 8192;
 }
 
 // The first round of [first, stop) that runs in one block (stop: none).
@@ -105,12 +122,7 @@ struct ProveRun {
     }
     int threads = kernel_threads(L);
     size_t smem;
-    if (use_point_parallel(L) && shape == kShapeGeneric) {
-      kern = round_kernel_pp<L, K>;
-      threads = kPointParallelThreads;
-      smem = static_cast<size_t>(pp_smem_words(threads, K_, L)) * 4;
-      SC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
-    } else if (shape == kShapeGeneric) {
+    if (shape == kShapeGeneric) {
       const int per_thread = round_smem_words_per_thread(K_, L, DMAX) * 4;
       while (threads > 32 && threads * per_thread > kMaxDynSmem) threads -= 32;
       smem = static_cast<size_t>(threads) * per_thread;
@@ -154,6 +166,7 @@ struct ProveRun {
                            st + so.chals, first, ctx->sm_count, ctx->stream)))
       return rc;
     const uint32_t* prev = first <= 1 ? tables : static_cast<const uint32_t*>(((first - 1) & 1) ? ctx->fold_a.p : ctx->fold_b.p);
+    const uint64_t part_max = part_pairs(L, shape != kShapeGeneric);
     const int tail_j = tail_round(*ex, L, shape != kShapeGeneric, n, first, stop);
     for (int j = first; j < stop; ++j) {
       A.round = j;
@@ -192,13 +205,23 @@ struct ProveRun {
         j += T.rounds - 1;
         continue;
       }
-      uint64_t per_block = static_cast<uint64_t>(threads);
-      if (use_point_parallel(L) && shape == kShapeGeneric) {  // pairs a block holds: one per lane group
-        const int npts = ex->degree + 1 - (A.skip1 ? 1 : 0);
-        const int G = npts <= 2 ? 2 : (npts <= 4 ? 4 : 8);
-        per_block = static_cast<uint64_t>(threads / G);
+      if (A.pairs <= part_max) {  // small parts, one a block
+        PartArgs T;
+        T.round = A;
+        T.lgP = 5;
+        while ((A.pairs >> T.lgP) > static_cast<uint64_t>(ctx->sm_count) && T.lgP < 7 &&
+               (size_t{4} << T.lgP) * K_ * L * 4 <= static_cast<size_t>(kMaxDynSmem))
+          ++T.lgP;
+        T.pad = 0;
+        const size_t part_smem = (size_t{2} << T.lgP) * K_ * L * 4;
+        cudaEvent_t ev;
+        if ((rc = timing_begin(ctx, &ev))) return rc;
+        SC_CUDA(launch_round(part_kernel<L, K>, static_cast<unsigned>(A.pairs >> T.lgP), tail_threads(L), part_smem,
+                             ctx->stream, j > first, T, E, F));
+        if ((rc = timing_end(ctx))) return rc;
+        continue;
       }
-      const uint64_t want = (A.pairs + per_block - 1) / per_block;
+      const uint64_t want = (A.pairs + threads - 1) / threads;
       const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(want, grid_max));
       cudaEvent_t ev;
       if ((rc = timing_begin(ctx, &ev))) return rc;

@@ -771,10 +771,12 @@ struct RoundEnd {
   static constexpr int kMsgWords = 34 * ((25 + 4 * kMaxPoints * L) / 136 + 1) + 1;
   uint64_t s[kMaxPoints * L];             // the round's integer sums
   int64_t slot[kMaxPoints * (L + 1)];     // their words
+  uint32_t half[kMaxPoints * L * 2];      // a block's sums as 16-bit halves (tail.cuh)
   uint32_t msg[kMsgWords];
   uint32_t r[L];                          // r_j
   __align__(8) uint32_t dig[8];
   int is_last;
+  __device__ uint64_t half_sum(int i) const { return half[2 * i] + (static_cast<uint64_t>(half[2 * i + 1]) << 16); }
   __device__ uint32_t* g() { return msg + kMsgG; }  // g_j(t): words g()[t L + l]
 };
 
@@ -820,13 +822,11 @@ __device__ __forceinline__ void block_sums(const uint32_t* scratch, int d, bool 
   }
 }
 
-// Block-wide, after warp_sums: true in the block that completes the round (its `parts`-th block
-// or item), with the round's integer sums in end.s; every thread calls. Ends with a barrier.
+// Block-wide, after the block added its sums (or, alone, put them into end.s): true in the block
+// that completes the round (its `parts`-th block or item), with the round's integer sums in
+// end.s; every thread calls. Ends with a barrier.
 template <int L>
-__device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32_t part, uint32_t parts, uint64_t* sums,
-                                          uint32_t* counter, RoundEnd<L>& end) {
-  __syncthreads();
-  block_sums<L>(scratch, d, parts == 1, end.s, sums, part);
+__device__ __forceinline__ bool grid_end(int d, uint32_t parts, uint64_t* sums, uint32_t* counter, RoundEnd<L>& end) {
   if (parts > 1) {
     __threadfence();
     __syncthreads();
@@ -849,6 +849,14 @@ __device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32
   }
   __syncthreads();
   return true;
+}
+// After warp_sums: the block's sums to the round's, then grid_end.
+template <int L>
+__device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32_t part, uint32_t parts, uint64_t* sums,
+                                          uint32_t* counter, RoundEnd<L>& end) {
+  __syncthreads();
+  block_sums<L>(scratch, d, parts == 1, end.s, sums, part);
+  return grid_end<L>(d, parts, sums, counter, end);
 }
 
 template <int L>
@@ -1165,13 +1173,6 @@ __host__ __device__ constexpr int round_smem_words_per_thread(int K, int L, int 
 // with the C++ product, 5% and 4% slower with the even/odd product); smaller fields run
 // 256-thread blocks.
 __host__ __device__ constexpr int kernel_threads(int L) { return L >= 8 ? 128 : 256; }
-#ifndef SC_PP_MIN_LIMBS
-#define SC_PP_MIN_LIMBS 8
-#endif
-// Fields of at least this many limbs evaluate generic expressions point-parallel
-// (prover_pp.cuh) in the plain round kernel.
-__host__ __device__ constexpr bool use_point_parallel(int L) { return L >= SC_PP_MIN_LIMBS; }
-constexpr int kPointParallelThreads = 128;
 #ifndef SC_L8_MIN_BLOCKS
 #define SC_L8_MIN_BLOCKS 3
 #endif
@@ -1214,7 +1215,7 @@ __host__ __device__ constexpr int round_min_blocks(int L, int shape) {
 }
 
 template <int L, int K, int DMAX, int SHAPE = kShapeGeneric>
-__global__ void __launch_bounds__(kernel_threads(L), round_min_blocks(L, SHAPE))
+__global__ void __launch_bounds__(kernel_threads(L), SHAPE ? round_min_blocks(L, SHAPE) : batch_min_blocks(L, DMAX))
     round_kernel(const RoundArgs A, const ExprDev E, const FieldParams<L, K> F) {
   extern __shared__ __align__(16) uint32_t smem[];
   __shared__ RoundEnd<L> end;

@@ -555,7 +555,7 @@ int issue_tick(sc_server* S, bool* issued) {
     for (uint64_t i = R->issued; i < R->issued + give; ++i) {
       BatchItem I;
       I.round = ridx;
-      I.pad = 0;
+      I.lgP = -1;
       I.start = i * tile;
       I.count = std::min<uint64_t>(tile, pairs - i * tile);
       items[c].push_back(I);
