@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "field_gold.cuh"
+#include "field_m127.cuh"
 #include "field_ptx.cuh"
 
 namespace sc {
@@ -252,65 +253,6 @@ static __device__ __noinline__ Fe8x2 bls381_mul2_call(const Fe<8> a0, const Fe<8
   return r;
 }
 
-// Montgomery product for p = 2^127 - 1 and R = 2^128 (x, y < p): R = 2 (mod p), so
-// x y R^-1 = (x y mod p) 2^126, and multiplying a 127-bit residue by 2^126 = 2^-1 is a
-// rotation right by one bit. x y < 2^254 = h 2^127 + l reduces to h + l < 2^128, then
-// (s mod 2^127) + (s >> 127) <= p, then one conditional subtraction of p.
-__device__ __forceinline__ void m127_mul(uint32_t (&r)[4], const uint32_t (&x)[4], const uint32_t (&y)[4]) {
-  uint32_t t[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) t[i] = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint64_t c = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint64_t uv = static_cast<uint64_t>(x[j]) * y[i] + t[i + j] + c;
-      t[i + j] = static_cast<uint32_t>(uv);
-      c = uv >> 32;
-    }
-    t[i + 4] = static_cast<uint32_t>(c);
-  }
-  // l = t mod 2^127, h = t >> 127 (both < 2^127); s = l + h
-  uint32_t h[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = (t[i + 3] >> 31) | (t[i + 4] << 1);
-  t[3] &= 0x7fffffffu;
-  uint32_t sw[4];
-  uint64_t c = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint64_t v = static_cast<uint64_t>(t[i]) + h[i] + c;
-    sw[i] = static_cast<uint32_t>(v);
-    c = v >> 32;
-  }
-  // s < 2^128: fold bit 127 back in (2^127 = 1)
-  const uint32_t top = sw[3] >> 31;
-  sw[3] &= 0x7fffffffu;
-  c = top;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint64_t v = static_cast<uint64_t>(sw[i]) + c;
-    sw[i] = static_cast<uint32_t>(v);
-    c = v >> 32;
-  }
-  // now s <= p; s == p means 0
-  const bool is_p = sw[0] == 0xffffffffu && sw[1] == 0xffffffffu && sw[2] == 0xffffffffu && sw[3] == 0x7fffffffu;
-  if (is_p) sw[0] = sw[1] = sw[2] = sw[3] = 0;
-  // times 2^126 = 2^-1: rotate the 127-bit value right by one
-  const uint32_t low = sw[0] & 1u;
-  r[0] = (sw[0] >> 1) | (sw[1] << 31);
-  r[1] = (sw[1] >> 1) | (sw[2] << 31);
-  r[2] = (sw[2] >> 1) | (sw[3] << 31);
-  r[3] = (sw[3] >> 1) | (low << 30);
-}
-
-static __device__ __noinline__ Fe<4> m127_mul_call(const Fe<4> a, const Fe<4> b) {
-  Fe<4> r;
-  m127_mul(r.w, a.w, b.w);
-  return r;
-}
-
 template <int L, int K>
 __device__ __forceinline__ Fe<L> fe_mul(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
   Fe<L> r;
@@ -319,7 +261,8 @@ __device__ __forceinline__ Fe<L> fe_mul(const Fe<L>& a, const Fe<L>& b, const Fi
   } else if constexpr (K == kFieldGoldilocks && L == 2) {
     gold_mul(r.w, a.w, b.w);
   } else if constexpr (K == kFieldMersenne127 && L == 4) {
-    r = m127_mul_call(a, b);
+    m127_mul_lazy(r.w, a.w, b.w);
+    m127_canon(r.w, r.w);
   } else if constexpr (K == kFieldBls381 && L == 8) {
     r = bls381_mul_call(a, b);
   } else if constexpr (L == 1) {
@@ -392,6 +335,80 @@ __device__ __forceinline__ Fe<2> gl_mul(const Fe<2>& a, const Fe<2>& b, const Go
 #endif
   return r;
 }
+// Arithmetic on any representative where the field has it in every operand (2^127 - 1: below
+// 2^128, field_m127.cuh), the canonical forms elsewhere.
+template <int L, int K>
+__host__ __device__ constexpr bool any_rep() {
+  return L == 4 && K == kFieldMersenne127;
+}
+template <int L, int K>
+__device__ __forceinline__ Fe<L> fa_add(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    Fe<L> r;
+    m127_add_lazy(r.w, a.w, b.w);
+    return r;
+  } else {
+    return fe_add(a, b, F);
+  }
+}
+template <int L, int K>
+__device__ __forceinline__ Fe<L> fa_sub(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    Fe<L> r;
+    m127_sub_lazy(r.w, a.w, b.w);
+    return r;
+  } else {
+    return fe_sub(a, b, F);
+  }
+}
+template <int L, int K>
+__device__ __forceinline__ Fe<L> fa_mul(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    Fe<L> r;
+    m127_mul_lazy(r.w, a.w, b.w);
+    return r;
+  } else {
+    return fe_mul(a, b, F);
+  }
+}
+template <int L, int K>
+__device__ __forceinline__ void fa_mul2(Fe<L>& r0, const Fe<L>& a0, const Fe<L>& b0, Fe<L>& r1, const Fe<L>& a1,
+                                        const Fe<L>& b1, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    const Fe<L> x = fa_mul(a0, b0, F);
+    r1 = fa_mul(a1, b1, F);
+    r0 = x;
+  } else {
+    fe_mul2(r0, a0, b0, r1, a1, b1, F);
+  }
+}
+
+// Two folds by one challenge, canonical: e = x0 + r (x1 - x0), o = x2 + r (x3 - x2).
+template <int L, int K>
+__device__ __forceinline__ void fe_fold2(Fe<L>& e, Fe<L>& o, const Fe<L>& x0, const Fe<L>& x1, const Fe<L>& x2,
+                                         const Fe<L>& x3, const Fe<L>& r, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    e = fa_add(x0, fa_mul(r, fa_sub(x1, x0, F), F), F);
+    o = fa_add(x2, fa_mul(r, fa_sub(x3, x2, F), F), F);
+    m127_canon(e.w, e.w);
+    m127_canon(o.w, o.w);
+  } else {
+    fe_mul2(e, r, fe_sub(x1, x0, F), o, r, fe_sub(x3, x2, F), F);
+    e = fe_add(x0, e, F);
+    o = fe_add(x2, o, F);
+  }
+}
+template <int L, int K>
+__device__ __forceinline__ Fe<L> fe_fold(const Fe<L>& x0, const Fe<L>& x1, const Fe<L>& r, const FieldParams<L, K>& F) {
+  if constexpr (any_rep<L, K>()) {
+    Fe<L> e = fa_add(x0, fa_mul(r, fa_sub(x1, x0, F), F), F);
+    m127_canon(e.w, e.w);
+    return e;
+  } else {
+    return fe_add(x0, fe_mul(r, fe_sub(x1, x0, F), F), F);
+  }
+}
+
 template <int L>
 __device__ __forceinline__ bool fe_is_zero(const Fe<L>& a) {
   uint32_t o = 0;

@@ -204,22 +204,22 @@ __host__ __device__ constexpr bool lazy_generic() {
 template <bool LZ, int L, int K>
 __device__ __forceinline__ Fe<L> lz_add(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
   if constexpr (LZ) return gl_add(a, b, gold_k(F));
-  else return fe_add(a, b, F);
+  else return fa_add(a, b, F);
 }
 template <bool LZ, int L, int K>  // b canonical
 __device__ __forceinline__ Fe<L> lz_add_c(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
   if constexpr (LZ) return gl_add_c(a, b, gold_k(F));
-  else return fe_add(a, b, F);
+  else return fa_add(a, b, F);
 }
 template <bool LZ, int L, int K>
 __device__ __forceinline__ Fe<L> lz_sub(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
   if constexpr (LZ) return gl_sub(a, b, gold_k(F));
-  else return fe_sub(a, b, F);
+  else return fa_sub(a, b, F);
 }
 template <bool LZ, int L, int K>
 __device__ __forceinline__ Fe<L> lz_mul(const Fe<L>& a, const Fe<L>& b, const FieldParams<L, K>& F) {
   if constexpr (LZ) return gl_mul(a, b, gold_k(F));
-  else return fe_mul(a, b, F);
+  else return fa_mul(a, b, F);
 }
 template <bool LZ, int L, int K>
 __device__ __forceinline__ void lz_mul2(Fe<L>& r0, const Fe<L>& a0, const Fe<L>& b0, Fe<L>& r1, const Fe<L>& a1,
@@ -229,7 +229,7 @@ __device__ __forceinline__ void lz_mul2(Fe<L>& r0, const Fe<L>& a0, const Fe<L>&
     r1 = gl_mul(a1, b1, gold_k(F));
     r0 = x;
   } else {
-    fe_mul2(r0, a0, b0, r1, a1, b1, F);
+    fa_mul2(r0, a0, b0, r1, a1, b1, F);
   }
 }
 template <bool LZ, int L, int K>
@@ -283,10 +283,10 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, Get get, Add add, Pr
       if (two) {
         Fe<L> w, w1;
         get(E.flat[off + f + 1], w, w1);
-        li = fe_mul(li, fe_sub(w1, w, F), F);
-        fe_mul2(v, v, w, v1, v1, w1, F);
-        df = fe_sub(v1, v, F);
-        dd = fe_add(li, li, F);
+        li = fa_mul(li, fe_sub(w1, w, F), F);
+        fa_mul2(v, v, w, v1, v1, w1, F);
+        df = fa_sub(v1, v, F);
+        dd = fa_add(li, li, F);
       }
       // products two points at a time: the leading coefficient with point 0, then 1 | 2, 3 | ..
       if (f == 0) {
@@ -299,7 +299,7 @@ __device__ __forceinline__ void eval_pair(const ExprDev& E, Get get, Add add, Pr
       }
       auto step = [&]() {
         v = lz_add_c<LZ>(v, df, F);
-        if (two) df = fe_add(df, dd, F);
+        if (two) df = fa_add(df, dd, F);
       };
 #pragma unroll
       for (int t = 1; t < DMAX; t += 2) {  // t odd, then t + 1
@@ -367,18 +367,18 @@ __host__ __device__ constexpr bool streamed_tables(int L) { return L >= 8; }
 // the term of full degree alone).
 template <int L, int K, typename V>
 __device__ __forceinline__ Fe<L> shape_value(V v, const FieldParams<L, K>& F, std::integral_constant<int, kShapeZerocheck>) {
-  const Fe<L> u = fe_add(v(0), fe_mul(v(5), v(4), F), F);  // S1 + M X2
-  Fe<L> s = fe_mul(v(1), u, F);                            // X1 (S1 + M X2)
-  s = fe_add(s, fe_mul(v(3), v(4), F), F);                 // + S2 X2
-  s = fe_sub(s, fe_mul(v(6), v(7), F), F);                 // - S4 X3
-  s = fe_add(s, v(8), F);                                  // + S5
-  return fe_mul(v(2), s, F);                               // F (...)
+  const Fe<L> u = fa_add(v(0), fa_mul(v(5), v(4), F), F);  // S1 + M X2
+  Fe<L> s = fa_mul(v(1), u, F);                            // X1 (S1 + M X2)
+  s = fa_add(s, fa_mul(v(3), v(4), F), F);                 // + S2 X2
+  s = fa_sub(s, fa_mul(v(6), v(7), F), F);                 // - S4 X3
+  s = fa_add(s, v(8), F);                                  // + S5
+  return fa_mul(v(2), s, F);                               // F (...)
 }
 template <int L, int K, typename V>
 __device__ __forceinline__ Fe<L> shape_value(V v, const FieldParams<L, K>& F, std::integral_constant<int, kShapeAbcg>) {
   Fe<L> ab, de;
-  fe_mul2(ab, v(0), v(1), de, v(4), v(5), F);
-  return fe_mul(v(3), fe_add(fe_mul(ab, v(2), F), de, F), F);
+  fa_mul2(ab, v(0), v(1), de, v(4), v(5), F);
+  return fa_mul(v(3), fa_add(fa_mul(ab, v(2), F), de, F), F);
 }
 template <int L, int K, typename V, typename W>
 __device__ __forceinline__ void shape_value2(V v, W w, Fe<L>& x, Fe<L>& y, const FieldParams<L, K>& F,
@@ -390,26 +390,26 @@ template <int L, int K, typename V, typename W>
 __device__ __forceinline__ void shape_value2(V v, W w, Fe<L>& x, Fe<L>& y, const FieldParams<L, K>& F,
                                              std::integral_constant<int, kShapeAbcg>) {
   Fe<L> p, q;
-  fe_mul2(x, v(0), v(1), y, w(0), w(1), F);
-  fe_mul2(x, x, v(2), y, y, w(2), F);
-  fe_mul2(p, v(4), v(5), q, w(4), w(5), F);
-  x = fe_add(x, p, F);
-  y = fe_add(y, q, F);
-  fe_mul2(x, x, v(3), y, y, w(3), F);
+  fa_mul2(x, v(0), v(1), y, w(0), w(1), F);
+  fa_mul2(x, x, v(2), y, y, w(2), F);
+  fa_mul2(p, v(4), v(5), q, w(4), w(5), F);
+  x = fa_add(x, p, F);
+  y = fa_add(y, q, F);
+  fa_mul2(x, x, v(3), y, y, w(3), F);
 }
 template <int L, int K, typename V, typename D>
 __device__ __forceinline__ void shape_ends(V v, D d, Fe<L>& x, Fe<L>& lead, const FieldParams<L, K>& F,
                                            std::integral_constant<int, kShapeZerocheck> shape) {
   x = shape_value<L, K>(v, F, shape);
-  lead = fe_mul(fe_mul(d(2), d(1), F), fe_mul(d(4), d(5), F), F);  // F X1 X2 M
+  lead = fa_mul(fa_mul(d(2), d(1), F), fa_mul(d(4), d(5), F), F);  // F X1 X2 M
 }
 template <int L, int K, typename V, typename D>
 __device__ __forceinline__ void shape_ends(V v, D d, Fe<L>& x, Fe<L>& lead, const FieldParams<L, K>& F,
                                            std::integral_constant<int, kShapeAbcg>) {
-  fe_mul2(x, v(0), v(1), lead, d(0), d(1), F);
-  fe_mul2(x, x, v(2), lead, lead, d(2), F);
-  x = fe_add(x, fe_mul(v(4), v(5), F), F);
-  fe_mul2(x, x, v(3), lead, lead, d(3), F);  // G (A B C + D E); A B C G
+  fa_mul2(x, v(0), v(1), lead, d(0), d(1), F);
+  fa_mul2(x, x, v(2), lead, lead, d(2), F);
+  x = fa_add(x, fa_mul(v(4), v(5), F), F);
+  fa_mul2(x, x, v(3), lead, lead, d(3), F);  // G (A B C + D E); A B C G
 }
 
 __device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[9], const GoldK k,
@@ -562,8 +562,8 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
             const uint4 v = reinterpret_cast<const uint4*>(stage)[(i * L + l) * nthr + tid];
             x0.w[l] = v.x; x1.w[l] = v.y; x2.w[l] = v.z; x3.w[l] = v.w;
           }
-          const Fe<L> e = fe_add(x0, fe_mul(r_prev, fe_sub(x1, x0, F), F), F);
-          const Fe<L> o = fe_add(x2, fe_mul(r_prev, fe_sub(x3, x2, F), F), F);
+          Fe<L> e, o;
+          fe_fold2(e, o, x0, x1, x2, x3, r_prev, F);
 #pragma unroll
           for (int l = 0; l < L; ++l)
             reinterpret_cast<uint2*>(dst + (static_cast<uint64_t>(E.role[i]) * L + l) * dst_len)[q] = make_uint2(e.w[l], o.w[l]);
@@ -603,8 +603,8 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
           for (int l = 0; l < L; ++l) {
             x0.w[l] = raw[i][l].x; x1.w[l] = raw[i][l].y; x2.w[l] = raw[i][l].z; x3.w[l] = raw[i][l].w;
           }
-          const Fe<L> e = fe_add(x0, fe_mul(r_prev, fe_sub(x1, x0, F), F), F);
-          const Fe<L> o = fe_add(x2, fe_mul(r_prev, fe_sub(x3, x2, F), F), F);
+          Fe<L> e, o;
+          fe_fold2(e, o, x0, x1, x2, x3, r_prev, F);
 #pragma unroll
           for (int l = 0; l < L; ++l)
             reinterpret_cast<uint2*>(dst + (static_cast<uint64_t>(E.role[i]) * L + l) * dst_len)[q] = make_uint2(e.w[l], o.w[l]);
@@ -639,9 +639,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
           const uint4 v = __ldcs(reinterpret_cast<const uint4*>(src + (static_cast<uint64_t>(k) * L + l) * src_len) + q);
           x0.w[l] = v.x; x1.w[l] = v.y; x2.w[l] = v.z; x3.w[l] = v.w;
         }
-        fe_mul2(e, r_prev, fe_sub(x1, x0, F), o, r_prev, fe_sub(x3, x2, F), F);
-        e = fe_add(x0, e, F);
-        o = fe_add(x2, o, F);
+        fe_fold2(e, o, x0, x1, x2, x3, r_prev, F);
         const uint64_t dst_len = src_len >> 1;
 #pragma unroll
         for (int l = 0; l < L; ++l)
@@ -722,8 +720,8 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       const std::integral_constant<int, SHAPE> shape{};
       Fe<L> x, y;
       shape_ends<L, K>([&](int i) { return sh_v[i]; }, [&](int i) { return fe_sub(sh_d[i], sh_v[i], F); }, x, y, F, shape);
-      acc[0] = fe_add(acc[0], x, F);
-      acc[4] = fe_add(acc[4], y, F);
+      acc[0] = fa_add(acc[0], x, F);
+      acc[4] = fa_add(acc[4], y, F);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const Fe<L> o = sh_d[r];
@@ -733,11 +731,11 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       if constexpr (kAsync) {
         if (!fold && q + stride < last) issue(q + stride);
       }
-      if (!skip1) acc[1] = fe_add(acc[1], shape_value<L, K>([&](int i) { return sh_v[i]; }, F, shape), F);
-      shape_value2<L, K>([&](int i) { return fe_add(sh_v[i], sh_d[i], F); },
-                         [&](int i) { return fe_add(fe_add(sh_v[i], sh_d[i], F), sh_d[i], F); }, x, y, F, shape);
-      acc[2] = fe_add(acc[2], x, F);
-      acc[3] = fe_add(acc[3], y, F);
+      if (!skip1) acc[1] = fa_add(acc[1], shape_value<L, K>([&](int i) { return sh_v[i]; }, F, shape), F);
+      shape_value2<L, K>([&](int i) { return fa_add(sh_v[i], sh_d[i], F); },
+                         [&](int i) { return fa_add(fa_add(sh_v[i], sh_d[i], F), sh_d[i], F); }, x, y, F, shape);
+      acc[2] = fa_add(acc[2], x, F);
+      acc[3] = fa_add(acc[3], y, F);
     }
   }
   if constexpr (kStream) {
@@ -867,24 +865,12 @@ __device__ __forceinline__ Fe<L> fc_get(const uint32_t* row) {
 // a b R^-1 mod p, fully reduced, for a < p and any b < 2^(32 L).
 template <int L, int K>
 __device__ __forceinline__ Fe<L> fe_mul_any(const Fe<L>& a, Fe<L> b, const FieldParams<L, K>& F) {
-  if constexpr (K == kFieldMersenne127 && L == 4) {
-    // the product wants operands <= p = 2^127 - 1: bit 127 is worth 1
-    const uint32_t top = b.w[3] >> 31;
-    b.w[3] &= 0x7fffffffu;
-    uint64_t c = top;
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      c += b.w[l];
-      b.w[l] = static_cast<uint32_t>(c);
-      c >>= 32;
-    }
-    return fe_mul(a, b, F);
-  } else if constexpr (K == kFieldGoldilocks && L == 2) {
+  if constexpr (K == kFieldGoldilocks && L == 2) {
     Fe<2> r;
     gold_mul(r.w, a.w, b.w);  // h < p and b' < p below, whatever b is
     return r;
   } else {
-    return fe_mul(a, b, F);  // the rows scan b's words against a: t < a + p throughout
+    return fe_mul(a, b, F);  // the rows scan b's words against a: t < a + p throughout; or any operands
   }
 }
 
@@ -1266,8 +1252,8 @@ __global__ void __launch_bounds__(256) fold_kernel(const uint32_t* __restrict__ 
       const uint4 v = __ldcs(reinterpret_cast<const uint4*>(src + (k * L + l) * src_len) + q);
       x0.w[l] = v.x; x1.w[l] = v.y; x2.w[l] = v.z; x3.w[l] = v.w;
     }
-    const Fe<L> e = fe_add(x0, fe_mul(r, fe_sub(x1, x0, F), F), F);
-    const Fe<L> o = fe_add(x2, fe_mul(r, fe_sub(x3, x2, F), F), F);
+    Fe<L> e, o;
+    fe_fold2(e, o, x0, x1, x2, x3, r, F);
 #pragma unroll
     for (int l = 0; l < L; ++l) reinterpret_cast<uint2*>(dst + (k * L + l) * dst_len)[q] = make_uint2(e.w[l], o.w[l]);
   }

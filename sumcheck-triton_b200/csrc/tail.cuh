@@ -37,10 +37,11 @@ template <int L, int K>
 __device__ __forceinline__ Fe<L> tail_value(const Fe<L>& e, const Fe<L>& o, int point, bool lead,
                                             const FieldParams<L, K>& F) {
   if (!lead && point < 2) return point == 0 ? e : o;
+  constexpr bool LZ = lazy_generic<L, K>();
   const Fe<L> d = fe_sub(o, e, F);
   if (lead) return d;
-  Fe<L> v = fe_add(o, d, F);
-  for (int t = 2; t < point; ++t) v = fe_add(v, d, F);
+  Fe<L> v = lz_add_c<LZ>(o, d, F);
+  for (int t = 2; t < point; ++t) v = lz_add_c<LZ>(v, d, F);
   return v;
 }
 
@@ -69,7 +70,7 @@ __device__ __forceinline__ void tail_fold(const RoundArgs& A, int nv, const Fiel
         a.w[l] = w.x;
         b.w[l] = w.y;
       }
-      f = fe_add(a, fe_mul(r, fe_sub(b, a, F), F), F);
+      f = fe_fold(a, b, r, F);
       if (store) {
 #pragma unroll
         for (int l = 0; l < L; ++l) A.dst[static_cast<uint64_t>(v * L + l) * (A.src_len >> 1) + 2 * q0 + x] = f.w[l];
@@ -86,6 +87,7 @@ __device__ __forceinline__ void tail_fold(const RoundArgs& A, int nv, const Fiel
 template <int L, int K>
 __device__ __forceinline__ void tail_eval(const ExprDev& E, const FieldParams<L, K>& F, const uint32_t* cur, int lgP,
                                           bool skip1, uint32_t* cnt) {
+  constexpr bool LZ = lazy_generic<L, K>();
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
   const int d = E.degree, S = d + 1 - (skip1 ? 1 : 0), P = 1 << lgP, lg2P = lgP + 1;
   const uint32_t s_inv = 65536u / S + 1;  // combo / S below, for combo < 2^13
@@ -118,16 +120,22 @@ __device__ __forceinline__ void tail_eval(const ExprDev& E, const FieldParams<L,
         bool neg = kind == kCoeffMinus;
         if (kind == kCoeffSmall) {
           const int32_t c = E.coeff_small[t];
-          prod = fe_mul_small(prod, c < 0 ? static_cast<uint32_t>(-static_cast<int64_t>(c)) : static_cast<uint32_t>(c), F);
+          const uint32_t m = c < 0 ? static_cast<uint32_t>(-static_cast<int64_t>(c)) : static_cast<uint32_t>(c);
+          Fe<L> base = prod;  // double and add
+          prod = fe_zero<L>();
+          for (uint32_t k = m; k; k >>= 1) {
+            if (k & 1u) prod = lz_add<LZ>(prod, base, F);
+            if (k > 1u) base = lz_add<LZ>(base, base, F);
+          }
           neg = c < 0;
         } else if (kind == kCoeffMont) {
           Fe<L> cm;
 #pragma unroll
           for (int l = 0; l < L; ++l) cm.w[l] = E.coeff_mont[t][l];
-          prod = fe_mul(prod, cm, F);
+          prod = lz_mul<LZ>(prod, cm, F);
         }
-        for (int f = 1; f < len; ++f) prod = fe_mul(prod, value(E.flat[off + f]), F);
-        sum = add_or_sub(sum, prod, neg, F);
+        for (int f = 1; f < len; ++f) prod = lz_mul<LZ>(prod, value(E.flat[off + f]), F);
+        sum = lz_add_or_sub<LZ>(sum, prod, neg, F);
       }
     // a warp's lanes share the point when P >= 32
     if (P >= 32) {

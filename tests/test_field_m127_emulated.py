@@ -1,0 +1,97 @@
+"""The inline-PTX arithmetic of csrc/field_m127.cuh (any representatives of residues mod
+2^127 - 1 below 2^128), run on the CPU statement by statement against big integers: random
+operands and the edges of the representation (0, p, 2^127, 2^128 - 1, and their neighbours)."""
+
+from __future__ import annotations
+
+import random
+import re
+from pathlib import Path
+
+import pytest
+
+HEADER = Path(__file__).resolve().parents[1] / "sumcheck-triton_b200" / "csrc" / "field_m127.cuh"
+M32 = (1 << 32) - 1
+P = (1 << 127) - 1
+EDGES = [0, 1, 2, P - 1, P, P + 1, P + 2, (1 << 127) + 5, (1 << 128) - 3, (1 << 128) - 2, (1 << 128) - 1, 2 * P, 2 * P + 1]
+
+
+def _programs():
+    out = {}
+    for name, body in re.findall(r"void (m127_\w+)\((.*?)\n\}\n", HEADER.read_text(), re.S):
+        text = "".join(re.findall(r'"((?:[^"\\]|\\.)*)"', body.split("asm(")[1].split('\n      : "=&r"')[0]))
+        lines = [ln.strip().rstrip(";") for ln in text.replace("\\n", "\n").replace("\\t", "").split("\n")]
+        ins = re.findall(r'"r"\((\w)\[(\d)\]\)', body)
+        out[name] = ([ln for ln in lines if ln and ln not in "{}" and not ln.startswith(".reg")], ins)
+    return out
+
+
+PROGRAMS = _programs()
+
+
+def run(name, **operands):
+    """The value (four words) the statement leaves in %0..%3."""
+    lines, ins = PROGRAMS[name]
+    regs = {f"%{4 + i}": operands[v] >> (32 * int(k)) & M32 for i, (v, k) in enumerate(ins)}
+    flag = family = None
+    val = lambda x: regs[x] if x in regs else int(x, 0) & M32  # noqa: E731
+    for ln in lines:
+        op, rest = ln.split(None, 1)
+        args = [a.strip() for a in rest.split(",")]
+        kind, d, a = op.split(".")[0], args[0], [val(x) for x in args[1:]]
+        if kind in ("addc", "madc", "subc"):
+            assert family == ("sub" if kind == "subc" else "add"), f"{name}: {ln} reads the other family's flag"
+        cin = flag if kind in ("addc", "madc", "subc") else 0
+        if kind in ("mul", "mad", "madc"):
+            prod = a[0] * a[1]
+            s = (prod & M32 if ".lo" in op else prod >> 32) + (a[2] + cin if kind != "mul" else 0)
+        elif kind in ("add", "addc"):
+            s = a[0] + a[1] + cin
+        elif kind in ("sub", "subc"):
+            s = a[0] - a[1] - cin
+        elif kind == "and":
+            s = a[0] & a[1]
+        elif kind == "shl":
+            s = a[0] << a[1] & M32
+        elif kind == "shr":
+            s = a[0] >> a[1]
+        elif kind == "shf":
+            s = ((a[1] << 32 | a[0]) >> a[2]) & M32
+        else:
+            raise ValueError(ln)
+        if ".cc" in op:
+            flag, family = int(s < 0 or s > M32), "sub" if kind.startswith("sub") else "add"
+        elif kind in ("mad", "madc", "add", "addc"):
+            assert s <= M32 or name == "m127_canon" or "s0, c" in ln, f"{name}: {ln} drops a carry"
+        regs[d] = s & M32
+    return sum(regs[f"%{k}"] << (32 * k) for k in range(4))
+
+
+def pairs(seed, count):
+    rng = random.Random(seed)
+    out = [(a, b) for a in EDGES for b in EDGES]
+    for _ in range(count):
+        a, b = rng.getrandbits(128), rng.getrandbits(128)
+        if rng.random() < 0.3:
+            a = (1 << 128) - 1 - rng.getrandbits(rng.randrange(1, 100))
+        if rng.random() < 0.3:
+            b = rng.getrandbits(rng.randrange(1, 128))
+        out.append((a, b))
+    return out
+
+
+@pytest.mark.parametrize("name,want", [
+    ("m127_mul_lazy", lambda a, b: a * b * pow(1 << 128, -1, P)),
+    ("m127_add_lazy", lambda a, b: a + b),
+    ("m127_sub_lazy", lambda a, b: a - b),
+])
+def test_lazy_forms_match_big_integers(name, want):
+    for a, b in pairs(7, 3000):
+        got = run(name, x=a, y=b) if name == "m127_mul_lazy" else run(name, a=a, b=b)
+        assert got % P == want(a, b) % P, (hex(a), hex(b))
+
+
+def test_canonical_form():
+    for a, b in pairs(9, 1500):
+        for x in (a, b):
+            assert run("m127_canon", a=x) == x % P, hex(x)
