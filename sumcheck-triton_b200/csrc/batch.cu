@@ -108,6 +108,8 @@ struct KernelSetup {
     while (threads > 32 && static_cast<size_t>(threads) * per_thread > static_cast<size_t>(kMaxDynSmem)) threads -= 32;
     const size_t smem = static_cast<size_t>(threads) * per_thread;
     SC_CUDA(cudaFuncSetAttribute(batch_round_kernel<L, K, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+    cudaFuncAttributes loaded;  // loads the kernel now: a first launch would stop to do it
+    SC_CUDA(cudaFuncGetAttributes(&loaded, batch_round_kernel<L, K, D>));
     int bps = 0;
     SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, batch_round_kernel<L, K, D>, threads, smem));
     if (bps < 1) return fail(SC_ERR_UNSUPPORTED, "batch kernel does not fit on an SM (tables=%d, L=%d)", kmax, L);
@@ -121,12 +123,11 @@ struct KernelSetup {
 template <int L, int K, int D>
 struct KernelLaunch {
   static int run(const sc_field* field, unsigned grid, int threads, size_t smem, cudaStream_t stream,
-                 const BatchTickArgs& T) {
+                 const BatchTickArgs& T, bool after) {
     FieldParams<L, K> F;
     for (int l = 0; l < L; ++l) F.p[l] = field->hf.p[l];
     F.np = field->hf.np;
-    batch_round_kernel<L, K, D><<<grid, threads, smem, stream>>>(T, F);
-    SC_CUDA(cudaGetLastError());
+    SC_CUDA(launch_after(batch_round_kernel<L, K, D>, grid, threads, smem, stream, after, T, F));
     return SC_OK;
   }
 };
@@ -171,8 +172,8 @@ int batch_kernel_setup(int L, int K, int dmax, int kmax, int threads_req, int sm
 }
 
 int batch_kernel_launch(int L, int K, int dmax, const sc_field* field, unsigned grid, int threads, size_t smem,
-                        cudaStream_t stream, const BatchTickArgs& T) {
-  return dispatch_dmax<KernelLaunch>(L, K, dmax, field, grid, threads, smem, stream, T);
+                        cudaStream_t stream, const BatchTickArgs& T, bool after) {
+  return dispatch_dmax<KernelLaunch>(L, K, dmax, field, grid, threads, smem, stream, T, after);
 }
 
 }  // namespace sc_host
@@ -351,7 +352,7 @@ int batch_issue(sc_batch* B) {
       T.rounds = static_cast<const BatchRound*>(B->rounds.p) + C.tick_round0[t];
       T.items = static_cast<const BatchItem*>(B->items.p) + C.tick_item0[t];
       T.num_items = C.tick_items[t];
-      T.pad = 0;
+      T.lgP = -1;
       T.head = static_cast<uint32_t*>(B->heads.p) + C.head0 + t;
       T.tile = 0;
       const int rc = batch_tick(B, C, t, T);

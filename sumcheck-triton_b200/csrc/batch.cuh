@@ -45,7 +45,7 @@ struct BatchTickArgs {
   const BatchRound* rounds;
   const BatchItem* items;  // nullptr: one round, item i = pairs [i tile, (i + 1) tile)
   int32_t num_items;
-  int32_t pad;
+  int32_t lgP;             // with items nullptr: >= 0 for parts of 2^lgP pairs (BatchItem::lgP)
   uint32_t* head;          // queue counter of this tick (zero before the launch); nullptr:
                            // block b does item b alone (grid = num_items)
   uint64_t tile;           // pairs per item when items is nullptr
@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
   uint32_t dyn_bytes;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
   if (tid == 0) cur_expr = nullptr;
+  pdl_begin();
   for (int pass = 0;; ++pass) {
     __syncthreads();
     if (tid == 0)
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
       I = T.items[it];
     } else {
       I.round = 0;
+      I.lgP = T.lgP;
       I.start = static_cast<uint64_t>(it) * T.tile;
     }
     if (tid == 0) R = T.rounds[I.round];
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
     uint32_t* sd = smem + E.num_vars * L * nthr;
     // k = 0: this item of the proof's round; k >= 1: the proof's tail rounds (only in the
     // block that finalised round k - 1; R.args then describes round R.args.round)
-    if (T.items && I.lgP >= 0) {
+    if (I.lgP >= 0) {
       batch_part<L, K>(&R.args, &E, F, I.lgP, static_cast<uint32_t>(R.item_base + (it - R.first_item)),
                        static_cast<uint32_t>(R.round_items), smem, &end);
       continue;

@@ -73,24 +73,6 @@ int tail_round(const sc_expr& ex, int L, bool shaped, int n, int first, int stop
   return stop;
 }
 
-// A round's launch; after: it follows another round's launch on the stream and may be set up
-// while that round ends (prover.cuh, pdl_begin).
-template <typename Args, typename Params>
-cudaError_t launch_round(void (*kern)(const Args, const ExprDev, const Params), unsigned grid, int threads, size_t smem,
-                         cudaStream_t stream, bool after, const Args& A, const ExprDev& E, const Params& F) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(static_cast<unsigned>(threads));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = after ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, A, E, F);
-}
-
 template <int L, int K, int DMAX>
 struct ProveRun {
   // Rounds [first, stop) of the proof. state_io (host, state words; NULL for a whole proof
@@ -200,7 +182,7 @@ struct ProveRun {
         const size_t tail_smem = tail_smem_words(A.pairs, K_, L) * 4;
         cudaEvent_t ev;
         if ((rc = timing_begin(ctx, &ev))) return rc;
-        SC_CUDA(launch_round(tail_kernel<L, K>, 1, tail_threads(L), tail_smem, ctx->stream, j > first, T, E, F));
+        SC_CUDA(launch_after(tail_kernel<L, K>, 1, tail_threads(L), tail_smem, ctx->stream, j > first, T, E, F));
         if ((rc = timing_end(ctx))) return rc;
         j += T.rounds - 1;
         continue;
@@ -216,7 +198,7 @@ struct ProveRun {
         const size_t part_smem = (size_t{2} << T.lgP) * K_ * L * 4;
         cudaEvent_t ev;
         if ((rc = timing_begin(ctx, &ev))) return rc;
-        SC_CUDA(launch_round(part_kernel<L, K>, static_cast<unsigned>(A.pairs >> T.lgP), tail_threads(L), part_smem,
+        SC_CUDA(launch_after(part_kernel<L, K>, static_cast<unsigned>(A.pairs >> T.lgP), tail_threads(L), part_smem,
                              ctx->stream, j > first, T, E, F));
         if ((rc = timing_end(ctx))) return rc;
         continue;
@@ -225,7 +207,7 @@ struct ProveRun {
       const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(want, grid_max));
       cudaEvent_t ev;
       if ((rc = timing_begin(ctx, &ev))) return rc;
-      SC_CUDA(launch_round(kern, grid, threads, smem, ctx->stream, j > first, A, E, F));
+      SC_CUDA(launch_after(kern, grid, threads, smem, ctx->stream, j > first, A, E, F));
       if ((rc = timing_end(ctx))) return rc;
     }
     return finish(ctx, ex, n, stop, st, so, out_polys, out_ch, out_finals, out_claim0, out_checksum, state_io);
@@ -676,6 +658,17 @@ int resume_folds(const sc_field* f, int n, int num_tables, const uint32_t* table
                  ? fold_prefix<8, kFieldBls381>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream)
                  : fold_prefix<8, kFieldGeneric>(f, n, num_tables, tables, fold_a, fold_b, chals_dev, j, sm_count, stream);
   }
+}
+
+int preload_tables(int L) {
+  cudaFuncAttributes loaded;
+  switch (L) {
+    case 1: SC_CUDA(cudaFuncGetAttributes(&loaded, generate_tables_kernel<1>)); break;
+    case 2: SC_CUDA(cudaFuncGetAttributes(&loaded, generate_tables_kernel<2>)); break;
+    case 4: SC_CUDA(cudaFuncGetAttributes(&loaded, generate_tables_kernel<4>)); break;
+    default: SC_CUDA(cudaFuncGetAttributes(&loaded, generate_tables_kernel<8>)); break;
+  }
+  return SC_OK;
 }
 
 int prove_segment(sc_ctx* ctx, const sc_field* field, const sc_expr* expr, int n, const uint32_t* tables, int mode,

@@ -47,14 +47,34 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+// A round kernel's launch; after: it follows another round's launch on the stream and may be set
+// up while that round ends (prover.cuh, pdl_begin).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_after(void (*kern)(Params...), unsigned grid, int threads, size_t smem, cudaStream_t stream,
+                                bool after, const Args&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // The batched round kernel's launch shape and launch (instantiated once, in batch.cu):
 // threads per block, grid (resident blocks on every SM) and dynamic shared memory for
 // requests of up to kmax tables. dmax is the largest degree the instance proves: a degree
 // class (2, 4, 7) or 6.
 int batch_kernel_setup(int L, int K, int dmax, int kmax, int threads_req, int sm_count, int* threads, int* grid,
                        size_t* smem);
+// after: the launch follows another one of this kernel on the stream and may be set up while
+// that one ends (prover.cuh, pdl_begin).
 int batch_kernel_launch(int L, int K, int dmax, const sc_field* field, unsigned grid, int threads, size_t smem,
-                        cudaStream_t stream, const BatchTickArgs& T);
+                        cudaStream_t stream, const BatchTickArgs& T, bool after = false);
 
 }  // namespace sc_host
 
@@ -533,6 +553,9 @@ inline int transcript_match(const TranscriptInfo& I, const HostField& hf, const 
     return fail(SC_ERR_INVALID, "transcript is of another expression");
   return SC_OK;
 }
+
+// Loads the table generator's kernel for this limb count. Defined in capi.cu.
+int preload_tables(int L);
 
 // Proves rounds [first, stop) of a proof on the context's stream. state_io (host,
 // state_offsets words) is uploaded before -- the state after round first - 1, zeros for

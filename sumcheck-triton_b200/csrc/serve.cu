@@ -2,7 +2,7 @@
 //
 // One worker thread per server owns two streams, a device memory pool and the request state.
 // Requests whose round 0 fills more than one wave of the GPU ("large") run whole on the
-// large-proof lane, a low-priority stream: one launch per round, one block per tile, issued
+// two large-proof lanes, low-priority streams: one launch per round, one block per tile, issued
 // at admission. All others are batched continuously in ticks on high-priority streams, so
 // their blocks are dispatched ahead of the lane's as the lane's blocks retire: small proofs
 // overtake large ones on the device instead of queueing behind them, while a large proof
@@ -52,6 +52,14 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 constexpr int kSlots = 2;                       // ticks in flight at most
+// Large proofs run on two lanes (pick_lane). Measured on B200, a burst of 40 requests with n from
+// 12 to 20: 6.05 ms on one lane, 3.98 ms on two.
+constexpr int kLanes = 2;
+// Rounds of at most this many pairs are cut into parts of 32 pairs, spread over their blocks'
+// threads (tail.cuh), as on the plain path.
+constexpr uint64_t kPartRoundPairs = 8192;
+constexpr int kPartLg = 5;
+inline size_t part_smem(int K, int L) { return (size_t{2} << kPartLg) * K * L * 4; }
 constexpr uint64_t kServeSkip1MinPairs = uint64_t{1} << 12;
 // Once a request's round fits one tile, that item's block proves the rest of the proof
 // (tail rounds, batch_round_kernel): one tick instead of one per remaining round. Measured
@@ -103,7 +111,8 @@ struct ServeRequest {
   uint32_t* fold_a = nullptr;
   uint32_t* fold_b = nullptr;
   BatchRound* rounds_dev = nullptr;  // large requests: every round's descriptor
-  bool large = false;    // runs whole on the large-proof lane
+  bool large = false;    // runs whole on a large-proof lane
+  int lane = 0;          // which one
   int slot = -1;         // pinned staging slot
   int round = 0;         // current round
   uint64_t issued = 0;   // items of the current round issued so far
@@ -172,10 +181,13 @@ struct sc_server {
   ExprDev* expr_host = nullptr;    // pinned [max_inflight] expression staging
   BatchRound* rounds_host = nullptr;  // pinned [max_inflight][kMaxRounds] (large requests)
   std::vector<cudaEvent_t> stage_events;  // per staging slot: a large request's completion
-  // large-proof lane: a low-priority stream of its own, with a context for table generation
-  cudaStream_t lane = nullptr;
-  sc_ctx* lane_ctx = nullptr;
-  std::deque<ServeRequest*> lane_inflight;
+  // large-proof lanes: low-priority streams of their own, with contexts for table generation. A
+  // large proof's last ten rounds or so leave the GPU nearly idle; with two lanes another large proof's
+  // first rounds run beside them.
+  cudaStream_t lane[kLanes] = {};
+  sc_ctx* lane_ctx[kLanes] = {};
+  int lane_load[kLanes] = {};
+  std::deque<ServeRequest*> lane_inflight;  // of all lanes, in admission order
   int64_t large_items = 1;         // round-0 tiles above which a request takes the lane
   size_t stage_words = 0;
   std::vector<int> free_stage;
@@ -328,11 +340,14 @@ int retire_ticks(sc_server* S, bool block) {
     T.busy = false;
     S->slots_in_flight.pop_front();
   }
-  // the large-proof lane completes in admission order
-  while (!S->lane_inflight.empty()) {
-    ServeRequest* R = S->lane_inflight.front();
+  // a lane completes in its admission order
+  for (auto it = S->lane_inflight.begin(); it != S->lane_inflight.end();) {
+    ServeRequest* R = *it;
     const cudaError_t q = cudaEventQuery(S->stage_events[R->slot]);
-    if (q == cudaErrorNotReady) break;
+    if (q == cudaErrorNotReady) {
+      ++it;
+      continue;
+    }
     if (q != cudaSuccess) return fail(SC_ERR_CUDA, "large request: %s", cudaGetErrorString(q));
     const double t = S->now();
     const uint32_t* hs = S->stage_host + static_cast<size_t>(R->slot) * S->stage_words;
@@ -341,7 +356,8 @@ int retire_ticks(sc_server* S, bool block) {
     S->free_stage.push_back(R->slot);
     R->slot = -1;
     S->admitted_bytes -= R->footprint;  // its block went back to the pool before the event
-    S->lane_inflight.pop_front();
+    --S->lane_load[R->lane];
+    it = S->lane_inflight.erase(it);
     publish(S, R, dev_status ? SC_ERR_DEVICE : SC_OK, t);
   }
   mark_idle_if_done(S);
@@ -352,12 +368,14 @@ int retire_ticks(sc_server* S, bool block) {
 // block per tile, so the small requests' higher-priority launches take SMs as these blocks
 // retire), result copy, free, completion event -- all ordered on the lane.
 int issue_large(sc_server* S, ServeRequest* R) {
-  SC_CUDA(cudaMemsetAsync(R->state, 0, state_and_sums_bytes(R->so, S->L), S->lane));
+  const cudaStream_t lane = S->lane[R->lane];
+  sc_ctx* const lane_ctx = S->lane_ctx[R->lane];
+  SC_CUDA(cudaMemsetAsync(R->state, 0, state_and_sums_bytes(R->so, S->L), lane));
   if (R->first)
-    SC_CUDA(cudaMemcpyAsync(R->state, R->resume_state.data(), R->so.total_words * 4, cudaMemcpyHostToDevice, S->lane));
+    SC_CUDA(cudaMemcpyAsync(R->state, R->resume_state.data(), R->so.total_words * 4, cudaMemcpyHostToDevice, lane));
   ExprDev& E = S->expr_host[R->slot];
   build_expr(S, R->expr, E);
-  SC_CUDA(cudaMemcpyAsync(R->expr_dev, &E, sizeof(ExprDev), cudaMemcpyHostToDevice, S->lane));
+  SC_CUDA(cudaMemcpyAsync(R->expr_dev, &E, sizeof(ExprDev), cudaMemcpyHostToDevice, lane));
   BatchRound* rh = S->rounds_host + static_cast<size_t>(R->slot) * kMaxRounds;
   int c = 0;
   while (S->classes[c].dclass != R->dclass) ++c;
@@ -374,6 +392,7 @@ int issue_large(sc_server* S, ServeRequest* R) {
 #endif
   constexpr uint64_t kLaneWaves = SC_LANE_WAVES;
   std::vector<uint64_t> tiles(R->n);
+  std::vector<int> part(R->n);
   int last = R->n;  // rounds [first, last) are launched; a tail covers the rest
   for (int t = R->first; t < last; ++t) {
     BatchRound& B = rh[t];
@@ -383,7 +402,10 @@ int issue_large(sc_server* S, ServeRequest* R) {
     const uint64_t thr = static_cast<uint64_t>(C.threads);
     const uint64_t tile = std::max<uint64_t>(S->tile_pairs, (want + thr - 1) / thr * thr);
     tiles[t] = tile;
-    const uint64_t items = (B.args.pairs + tile - 1) / tile;
+    const bool parts = B.args.pairs > static_cast<uint64_t>(S->tile_pairs) && B.args.pairs <= kPartRoundPairs &&
+                       part_smem(R->K, S->L) <= C.smem;
+    part[t] = parts ? kPartLg : -1;
+    const uint64_t items = parts ? B.args.pairs >> kPartLg : (B.args.pairs + tile - 1) / tile;
     B.expr = R->expr_dev;
     B.first_item = 0;
     B.num_items = static_cast<int32_t>(items);
@@ -395,29 +417,30 @@ int issue_large(sc_server* S, ServeRequest* R) {
     }
   }
   SC_CUDA(cudaMemcpyAsync(R->rounds_dev + R->first, rh + R->first,
-                          static_cast<size_t>(last - R->first) * sizeof(BatchRound), cudaMemcpyHostToDevice, S->lane));
-  int rc = sc_tables_generate(S->lane_ctx, S->field, R->K, R->n, R->kinds.data(), R->seed, R->tables);
+                          static_cast<size_t>(last - R->first) * sizeof(BatchRound), cudaMemcpyHostToDevice, lane));
+  int rc = sc_tables_generate(lane_ctx, S->field, R->K, R->n, R->kinds.data(), R->seed, R->tables);
   if (!rc)
     rc = resume_folds(S->field, R->n, R->K, R->tables, R->fold_a, R->fold_b, R->state + R->so.chals, R->first,
-                      S->lane_ctx->sm_count, S->lane);
+                      lane_ctx->sm_count, lane);
   if (rc) return rc;
   for (int t = R->first; t < last; ++t) {
     BatchTickArgs A;
     A.rounds = R->rounds_dev + t;
     A.items = nullptr;
     A.num_items = rh[t].num_items;
-    A.pad = 0;
+    A.lgP = part[t];
     A.head = nullptr;
     A.tile = tiles[t];
     rc = batch_kernel_launch(S->L, S->kind, C.dclass, S->field, static_cast<unsigned>(A.num_items), C.threads, C.smem,
-                             S->lane, A);
+                             lane, A, t > R->first);
     if (rc) return rc;
   }
   SC_CUDA(cudaMemcpyAsync(S->stage_host + static_cast<size_t>(R->slot) * S->stage_words, R->state,
-                          R->so.total_words * 4, cudaMemcpyDeviceToHost, S->lane));
-  SC_CUDA(cudaFreeAsync(R->block, S->lane));
+                          R->so.total_words * 4, cudaMemcpyDeviceToHost, lane));
+  SC_CUDA(cudaFreeAsync(R->block, lane));
   R->block = nullptr;
-  SC_CUDA(cudaEventRecord(S->stage_events[R->slot], S->lane));
+  SC_CUDA(cudaEventRecord(S->stage_events[R->slot], lane));
+  ++S->lane_load[R->lane];
   S->lane_inflight.push_back(R);
   return SC_OK;
 }
@@ -442,6 +465,19 @@ void suspend_waiting(sc_server* S) {
   }
 }
 
+// The lane a large request goes to: the less loaded one. The second lane cannot reuse a block
+// of the first before that lane has come to its free, and growing the pool holds the worker for
+// milliseconds, so it is taken only while the mapped pool has room for every admitted request.
+int pick_lane(sc_server* S, uint64_t footprint) {
+  if (S->lane_load[0] <= S->lane_load[1]) return 0;
+  uint64_t mapped = 0;
+  if (cudaMemPoolGetAttribute(S->pool, cudaMemPoolAttrReservedMemCurrent, &mapped) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return mapped >= S->admitted_bytes + footprint ? 1 : 0;
+}
+
 int admit(sc_server* S) {
   while (!S->waiting.empty() && static_cast<int>(S->active.size() + S->lane_inflight.size()) < S->max_inflight &&
          !S->free_stage.empty()) {
@@ -451,7 +487,8 @@ int admit(sc_server* S) {
     const BlockLayout b = block_layout(R->n, R->K, S->L);
     const uint64_t items0 = (((uint64_t{1} << R->n) >> (R->first + 1)) + S->tile_pairs - 1) / S->tile_pairs;
     R->large = static_cast<int64_t>(items0) > S->large_items;
-    cudaStream_t st = R->large ? S->lane : S->stream;
+    R->lane = R->large ? pick_lane(S, R->footprint) : 0;
+    cudaStream_t st = R->large ? S->lane[R->lane] : S->stream;
     void* p = nullptr;
     const double a0 = S->now();
     const cudaError_t e = cudaMallocFromPoolAsync(&p, b.total, S->pool, st);
@@ -540,7 +577,14 @@ int issue_tick(sc_server* S, bool* issued) {
     int c = 0;
     while (S->classes[c].dclass != R->dclass) ++c;
     const uint64_t pairs = (uint64_t{1} << R->n) >> (R->round + 1);
-    const uint64_t round_items = (pairs + tile - 1) / tile;
+    uint64_t round_items = (pairs + tile - 1) / tile;
+    // a whole round in this tick: in small parts while they fit one wave of the grid
+    const uint64_t parts = pairs >> kPartLg;
+    const bool split = round_items > 1 && give == round_items && pairs <= kPartRoundPairs &&
+                       part_smem(R->K, S->L) <= S->classes[c].smem &&
+                       static_cast<int64_t>(total_items + parts) <= std::min<int64_t>(S->wave_items, S->tick_item_cap);
+    if (split) give = round_items = parts;
+    const uint64_t step = split ? uint64_t{1} << kPartLg : tile;
     BatchRound B;
     std::memset(&B, 0, sizeof(B));
     round_args(S, *R, R->round, B.args);
@@ -555,9 +599,9 @@ int issue_tick(sc_server* S, bool* issued) {
     for (uint64_t i = R->issued; i < R->issued + give; ++i) {
       BatchItem I;
       I.round = ridx;
-      I.lgP = -1;
-      I.start = i * tile;
-      I.count = std::min<uint64_t>(tile, pairs - i * tile);
+      I.lgP = split ? kPartLg : -1;
+      I.start = i * step;
+      I.count = std::min<uint64_t>(step, pairs - i * step);
       items[c].push_back(I);
     }
     rounds[c].push_back(B);
@@ -611,7 +655,7 @@ int issue_tick(sc_server* S, bool* issued) {
     A.rounds = reinterpret_cast<const BatchRound*>(T.dev + r_off[c]);
     A.items = reinterpret_cast<const BatchItem*>(T.dev + i_off[c]);
     A.num_items = static_cast<int32_t>(items[c].size());
-    A.pad = 0;
+    A.lgP = -1;
     A.head = reinterpret_cast<uint32_t*>(T.dev) + c;
     A.tile = 0;
     SC_CUDA(cudaStreamWaitEvent(C.stream, S->fork, 0));
@@ -708,7 +752,8 @@ void loop_continuous(sc_server* S) {
     if (rc) {
       fail_all(S, rc);
       cudaStreamSynchronize(S->stream);
-      cudaStreamSynchronize(S->lane);
+      for (cudaStream_t st : S->lane) cudaStreamSynchronize(st);
+      std::fill(S->lane_load, S->lane_load + kLanes, 0);
       cudaGetLastError();
     }
   }
@@ -808,17 +853,20 @@ void destroy_resources(sc_server* S) {
     if (T.dev) cudaFree(T.dev);
     if (T.done) cudaEventDestroy(T.done);
   }
-  if (S->lane) cudaStreamSynchronize(S->lane);
+  for (cudaStream_t st : S->lane)
+    if (st) cudaStreamSynchronize(st);
   if (S->fork) cudaEventDestroy(S->fork);
   for (cudaEvent_t e : S->stage_events) cudaEventDestroy(e);
   if (S->stage_host) cudaFreeHost(S->stage_host);
   if (S->expr_host) cudaFreeHost(S->expr_host);
   if (S->rounds_host) cudaFreeHost(S->rounds_host);
   if (S->ctx) sc_ctx_destroy(S->ctx);
-  if (S->lane_ctx) sc_ctx_destroy(S->lane_ctx);
+  for (sc_ctx* c : S->lane_ctx)
+    if (c) sc_ctx_destroy(c);
   if (S->pool) cudaMemPoolDestroy(S->pool);
   if (S->stream) cudaStreamDestroy(S->stream);
-  if (S->lane) cudaStreamDestroy(S->lane);
+  for (cudaStream_t st : S->lane)
+    if (st) cudaStreamDestroy(st);
 }
 
 }  // namespace
@@ -864,10 +912,12 @@ int sc_server_create(int device, const sc_field* field, int policy, uint64_t hbm
   int prio_low = 0, prio_high = 0;
   cudaError_t e = cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
   if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&S->stream, cudaStreamNonBlocking, prio_high);
-  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&S->lane, cudaStreamNonBlocking, prio_low);
+  for (cudaStream_t& st : S->lane)
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, prio_low);
   if (e != cudaSuccess) return bail(fail(SC_ERR_CUDA, "stream: %s", cudaGetErrorString(e)));
   int rc = sc_ctx_create(device, S->stream, &S->ctx);
-  if (!rc) rc = sc_ctx_create(device, S->lane, &S->lane_ctx);
+  for (int i = 0; i < kLanes; ++i)
+    if (!rc) rc = sc_ctx_create(device, S->lane[i], &S->lane_ctx[i]);
   if (rc) return bail(rc);
   cudaMemPoolProps props;
   std::memset(&props, 0, sizeof(props));
@@ -902,6 +952,7 @@ int sc_server_create(int device, const sc_field* field, int policy, uint64_t hbm
     S->classes.push_back(C);
     if (e != cudaSuccess) return bail(fail(SC_ERR_CUDA, "class stream: %s", cudaGetErrorString(e)));
   }
+  if ((rc = preload_tables(S->L))) return bail(rc);
   S->wave_items = max_grid;
   S->large_items = max_grid;
   S->tick_budget = chunk_items ? chunk_items : 2 * max_grid;
