@@ -112,7 +112,12 @@ struct ProveRun {
       smem = shape_round_smem_bytes(L, K, shape, threads);  // reduction scratch (+ the pair stage)
     }
     int blocks_per_sm = 0;
-    SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, threads, smem));
+    for (const Occupancy& o : ctx->occupancy)
+      if (o.kern == reinterpret_cast<const void*>(kern) && o.threads == threads && o.smem == smem) blocks_per_sm = o.blocks;
+    if (!blocks_per_sm) {
+      SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, threads, smem));
+      ctx->occupancy.push_back(Occupancy{reinterpret_cast<const void*>(kern), threads, smem, blocks_per_sm});
+    }
     if (blocks_per_sm < 1) return fail(SC_ERR_UNSUPPORTED, "round kernel does not fit on an SM (K=%d, L=%d)", K_, L);
     const uint64_t grid_max = static_cast<uint64_t>(blocks_per_sm) * ctx->sm_count;
 

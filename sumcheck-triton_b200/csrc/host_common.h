@@ -80,11 +80,20 @@ int batch_kernel_launch(int L, int K, int dmax, const sc_field* field, unsigned 
 
 using sc_host::DevBuf;
 
+// Resident blocks per SM of a kernel at a launch shape, looked up once per context.
+struct Occupancy {
+  const void* kern;
+  int threads;
+  size_t smem;
+  int blocks;
+};
+
 struct sc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int sm_count = 0;
   DevBuf fold_a, fold_b, state;       // state: the proof state's words, then the round's sums
+  std::vector<Occupancy> occupancy;
   uint32_t* host_state = nullptr;  // pinned staging of the proof state
   size_t host_state_bytes = 0;
   // per-launch timing of the round kernels (off by default)

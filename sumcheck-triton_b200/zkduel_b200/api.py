@@ -204,28 +204,26 @@ class Proof:
     checksum: int
     extras: dict = dc_field(default_factory=dict)
 
-    def _dec(self, limbs) -> int:
-        return self.field.decode_limbs([int(x) for x in limbs])
-
     @property
     def round_polys(self) -> list[list[int]]:
-        return [[self._dec(v) for v in row] for row in self.round_polys_mont]
+        values, d1 = self.field.decode_array(self.round_polys_mont), self.degree + 1
+        return [values[i:i + d1] for i in range(0, len(values), d1)]
 
     @property
     def challenges(self) -> list[int]:
-        return [self._dec(v) for v in self.challenges_mont]
+        return self.field.decode_array(self.challenges_mont)
 
     @property
     def claim0(self) -> int:
-        return self._dec(self.claim0_mont)
+        return self.field.decode_array(self.claim0_mont)[0]
 
     @property
     def final_claim(self) -> int:
-        return self._dec(self.finals_mont[0])
+        return self.field.decode_array(self.finals_mont[0])[0]
 
     @property
     def final_values(self) -> list[int]:
-        return [self._dec(v) for v in self.finals_mont[1:]]
+        return self.field.decode_array(self.finals_mont[1:])
 
 
 # --------------------------------------------------------------------------------------
@@ -260,12 +258,12 @@ def host_tables_to_limbs(values: Sequence[Sequence[int]] | np.ndarray, spec: Fie
         if values.dtype.kind == "i" and (values < 0).any():
             arr = (values.astype(object) % q).astype(np.uint64)
         else:
-            arr = values.astype(np.uint64) % np.uint64(q)
-        out = np.empty((arr.shape[0], L, arr.shape[1]), dtype=np.uint32)
-        out[:, 0, :] = (arr & np.uint64(0xFFFFFFFF)).astype(np.uint32)
-        if L == 2:
-            out[:, 1, :] = (arr >> np.uint64(32)).astype(np.uint32)
-        return out
+            arr = np.ascontiguousarray(values, dtype=np.uint64)
+            if arr.size and int(arr.max()) >= q:
+                arr = arr % np.uint64(q)
+        K, N = arr.shape
+        words = np.ascontiguousarray(arr).view(np.dtype("<u4")).reshape(K, N, 2)
+        return np.ascontiguousarray(words[:, :, :L].transpose(0, 2, 1))
     rows = [np.array([int(x) % q for x in row], dtype=object) for row in values]
     K, N = len(rows), len(rows[0]) if rows else 0
     out = np.empty((K, L, N), dtype=np.uint32)
@@ -329,16 +327,18 @@ def prove_device(tables, expr: CompiledExpression | Expression, spec: FieldSpec,
             c = int(challenges[j]) if j < len(challenges) else 0
             words.extend(spec.montgomery_limbs(c))
         explicit = _lib.u32_array(words)
-    polys = np.zeros((n, d + 1, L), dtype=np.uint32)
-    chals = np.zeros((n, L), dtype=np.uint32)
-    finals = np.zeros((1 + K, L), dtype=np.uint32)
-    claim0 = np.zeros((L,), dtype=np.uint32)
+    # every output in one buffer: round polynomials, challenges, finals, claim
+    o1 = n * (d + 1) * L
+    o2 = o1 + n * L
+    o3 = o2 + (1 + K) * L
+    out = np.zeros(o3 + L, dtype=np.uint32)
     checksum = ctypes.c_uint64(0)
-    p = lambda a: a.ctypes.data_as(_lib.U32P)  # noqa: E731
+    at = lambda words: ctypes.byref(ctypes.c_uint32.from_buffer(out, 4 * words))  # noqa: E731
     rc = _lib.load().sc_prove(ctx.handle, fld.handle, expr.handle, n, ctypes.c_void_p(tables.data_ptr()), mode,
-                              explicit, p(polys), p(chals), p(finals), p(claim0), ctypes.byref(checksum))
+                              explicit, at(0), at(o1), at(o2), at(o3), ctypes.byref(checksum))
     _lib.check(rc, "sc_prove")
-    return Proof(spec, n, d, tuple(var_names or enc.var_names), polys, chals, finals, claim0, int(checksum.value))
+    return Proof(spec, n, d, tuple(var_names or enc.var_names), out[:o1].reshape(n, d + 1, L),
+                 out[o1:o2].reshape(n, L), out[o2:o3].reshape(1 + K, L), out[o3:], int(checksum.value))
 
 
 def prove_host(host_tables, expr: CompiledExpression | Expression, spec: FieldSpec, num_rounds: int,

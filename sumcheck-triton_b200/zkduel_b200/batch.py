@@ -97,9 +97,18 @@ class BatchProver:
     def launch(self) -> None:
         """Enqueues one run of every group (asynchronous). Every group is launched before any
         is joined to the caller's stream, so the groups run concurrently on their own streams."""
+        self._start()
+        self._join()
+
+    def _start(self) -> None:
+        """Every group, on its own streams, after the work already on the caller's stream."""
         lib = _lib.load()
         for g in self.groups:
             _lib.check(lib.sc_batch_launch(g.handle), "sc_batch_launch")
+
+    def _join(self) -> None:
+        """The caller's stream waits for every group."""
+        lib = _lib.load()
         for g in self.groups:
             _lib.check(lib.sc_batch_join(g.handle), "sc_batch_join")
 
@@ -296,7 +305,11 @@ class HostBatchProver:
                 K, _L, N = t.shape
                 _lib.check(lib.sc_tables_to_mont(self.ctx.handle, fld.handle, ctypes.c_void_p(t.data_ptr()),
                                                  ctypes.c_uint64(N), int(K)), "sc_tables_to_mont")
-            bp.launch()
+            bp._start()
+        # joined only now: a chunk's last rounds leave most of the GPU idle, and the next chunk's
+        # conversions and first rounds run beside them
+        for _a, _b, bp in self.chunks:
+            bp._join()
 
     def wait(self) -> None:
         for _a, _b, bp in self.chunks:

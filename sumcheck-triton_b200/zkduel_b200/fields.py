@@ -80,6 +80,12 @@ def from_limbs(words) -> int:
     return sum(int(w) << (32 * i) for i, w in enumerate(words))
 
 
+@lru_cache(maxsize=None)
+def _r_inverse(modulus: int, limbs: int) -> int:
+    """R^-1 mod p, R = 2^(32 limbs)."""
+    return pow(1 << (32 * limbs), -1, modulus)
+
+
 @dataclass(frozen=True)
 class FieldSpec:
     name: str
@@ -103,7 +109,7 @@ class FieldSpec:
 
     @property
     def r_inv(self) -> int:
-        return pow(self.r_mod, -1, self.modulus)
+        return _r_inverse(self.modulus, self.limbs)
 
     def to_limbs(self, value: int) -> list[int]:
         return to_limbs(int(value) % self.modulus, self.limbs)
@@ -116,6 +122,11 @@ class FieldSpec:
 
     def montgomery_limbs(self, value: int) -> list[int]:
         return to_limbs(self.montgomery_encode(value), self.limbs)
+
+    def decode_array(self, limbs) -> list[int]:
+        """Canonical values of an array of Montgomery-form uint32 limb vectors (last axis)."""
+        data, size, p, r_inv = limbs.tobytes(), 4 * self.limbs, self.modulus, self.r_inv
+        return [int.from_bytes(data[i:i + size], "little") * r_inv % p for i in range(0, len(data), size)]
 
     def decode_limbs(self, words) -> int:
         """Canonical value of a Montgomery-form limb vector."""
