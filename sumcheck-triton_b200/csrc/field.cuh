@@ -25,7 +25,7 @@
 #pragma once
 #include <cstdint>
 
-#include "field_gold.cuh"
+#include "field_gold_acc.cuh"
 #include "field_m127.cuh"
 #include "field_ptx.cuh"
 

@@ -9,7 +9,7 @@
 // The 256-bit product's words at even positions (i + j even) and at odd ones are two sets of
 // carry chains of multiply-adds, merged by one chain of additions: 16 multiply-add pairs, 3
 // carries, 7 additions; the reduction is 15 more instructions. Each statement is one asm block
-// (the carry flag does not survive between statements); tests/test_field_m127_emulated.py runs
+// (the carry flag does not survive between statements); tests/test_field_lazy_emulated.py runs
 // them on the CPU against big integers. Measured on B200 against the canonical product in C++
 // with 64-bit intermediates, called out of line: a 17-term gate over 2^127 - 1 at n = 16 843 ->
 // 684 us, a permutation check 315 -> 278 us, 40 served requests 7.12 -> 6.69 ms.

@@ -412,38 +412,51 @@ __device__ __forceinline__ void shape_ends(V v, D d, Fe<L>& x, Fe<L>& lead, cons
   fa_mul2(x, x, v(3), lead, lead, d(3), F);  // G (A B C + D E); A B C G
 }
 
-__device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[9], const GoldK k,
-                                                 std::integral_constant<int, kShapeZerocheck>) {
-  return gl_mul(gl_mul(d[2], d[1], k), gl_mul(d[4], d[5], k), k);
+// The same formulas in lazy Goldilocks arithmetic, added to a point's sum unreduced
+// (field_gold_acc.cuh): one reduction for the bracket, none for its product with the last factor.
+// The zerocheck's role 6 (S4) comes negated, so that its product is added.
+struct GoldSum {
+  uint32_t w[5];
+};
+__device__ __forceinline__ void shape_add(GoldSum& acc, const Fe<2> (&v)[9], const GoldK k,
+                                          std::integral_constant<int, kShapeZerocheck>) {
+  uint32_t t[5];
+  Fe<2> u, s;
+  gold_acc_first(t, v[5].w, v[4].w);  // M X2 + S1
+  gold_acc_add(t, t, v[0].w);
+  gold_acc_reduce(u.w, t, k);
+  gold_acc_first(t, v[1].w, u.w);     // X1 (S1 + M X2) + S2 X2 - S4 X3 + S5
+  gold_acc_mul(t, t, v[3].w, v[4].w);
+  gold_acc_mul(t, t, v[6].w, v[7].w);
+  gold_acc_add(t, t, v[8].w);
+  gold_acc_reduce(s.w, t, k);
+  gold_acc_mul(acc.w, acc.w, v[2].w, s.w);
 }
-
-__device__ __forceinline__ Fe<2> shape_lead_lazy(const Fe<2> (&d)[6], const GoldK k,
-                                                 std::integral_constant<int, kShapeAbcg>) {
-  return gl_mul(gl_mul(d[0], d[1], k), gl_mul(d[2], d[3], k), k);
+__device__ __forceinline__ void shape_add(GoldSum& acc, const Fe<2> (&v)[6], const GoldK k,
+                                          std::integral_constant<int, kShapeAbcg>) {
+  uint32_t t[5];
+  Fe<2> s;
+  gold_acc_first(t, gl_mul(v[0], v[1], k).w, v[2].w);
+  gold_acc_mul(t, t, v[4].w, v[5].w);
+  gold_acc_reduce(s.w, t, k);
+  gold_acc_mul(acc.w, acc.w, v[3].w, s.w);
 }
-
-// The same formulas in lazy Goldilocks arithmetic: operands and result in [0, 2^64).
-__device__ __forceinline__ Fe<2> shape_value_lazy(const Fe<2> (&v)[9], const GoldK k,
-                                                  std::integral_constant<int, kShapeZerocheck>) {
-  const Fe<2> u = gl_add(v[0], gl_mul(v[5], v[4], k), k);
-  Fe<2> s = gl_mul(v[1], u, k);
-  s = gl_add(s, gl_mul(v[3], v[4], k), k);
-  s = gl_sub(s, gl_mul(v[6], v[7], k), k);
-  s = gl_add(s, v[8], k);
-  return gl_mul(v[2], s, k);
+__device__ __forceinline__ void shape_add_lead(GoldSum& acc, const Fe<2> (&d)[9], const GoldK k,
+                                               std::integral_constant<int, kShapeZerocheck>) {
+  gold_acc_mul(acc.w, acc.w, gl_mul(d[2], d[1], k).w, gl_mul(d[4], d[5], k).w);
 }
-
-__device__ __forceinline__ Fe<2> shape_value_lazy(const Fe<2> (&v)[6], const GoldK k,
-                                                  std::integral_constant<int, kShapeAbcg>) {
-  const Fe<2> s = gl_add(gl_mul(gl_mul(v[0], v[1], k), v[2], k), gl_mul(v[4], v[5], k), k);
-  return gl_mul(v[3], s, k);
+__device__ __forceinline__ void shape_add_lead(GoldSum& acc, const Fe<2> (&d)[6], const GoldK k,
+                                               std::integral_constant<int, kShapeAbcg>) {
+  gold_acc_mul(acc.w, acc.w, gl_mul(d[0], d[1], k).w, gl_mul(d[2], d[3], k).w);
 }
 
 // 2-limb Goldilocks shape kernels evaluate their points in lazy arithmetic: the point steps
-// add a canonical difference (six ALU instructions, no compare or select), the formula's sums
-// take any representatives, and the point sums are made canonical once, after the thread's
-// last pair. Folds, stored tables and differences stay canonical. Measured on B200,
-// plain_goldilocks n = 24: 1.60 against 1.65 ms.
+// add a canonical difference (six ALU instructions, no compare or select), the formula's
+// products are summed unreduced, and the point sums are reduced once, after the thread's last
+// pair. Folds, stored tables and differences stay canonical. Measured on B200, zerocheck gate
+// n = 24: canonical sums 1.65 ms, lazy sums 1.60 ms (both a product reduced at a time, before
+// the leading coefficient took the last point); with reduced products 1.27 ms, with products
+// summed unreduced 1.18 ms.
 #ifndef SC_GOLD_LAZY
 #define SC_GOLD_LAZY 1
 #endif
@@ -524,6 +537,11 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
 #pragma unroll
     for (int t = 0; t <= DMAX; ++t) sm_put<L>(sv, t, tid, nthr, fe_zero<L>());
   }
+  GoldSum gsum[DMAX + 1];  // the lazy Goldilocks shapes' point sums
+#pragma unroll
+  for (int t = 0; t <= DMAX; ++t)
+#pragma unroll
+    for (int i = 0; i < 5; ++i) gsum[t].w[i] = 0;
   constexpr int NR = SHAPE == kShapeGeneric ? 1 : shape_tables(SHAPE);
   constexpr bool kGoldLazy = SHAPE != kShapeGeneric && L == 2 && K == kFieldGoldilocksFma && SC_GOLD_LAZY;
   constexpr bool kAsync = (kGoldLazy && SC_GOLD_ASYNC) || l8_async_stage(L, SHAPE);
@@ -696,7 +714,11 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       static_assert(DMAX == D, "shape kernels evaluate degree-4 shapes");
       const GoldK gk = gold_k(F);
       const std::integral_constant<int, SHAPE> shape{};
-      acc[0] = gl_add(acc[0], shape_value_lazy(sh_v, gk, shape), gk);
+      if constexpr (SHAPE == kShapeZerocheck) {
+        gold_neg(sh_v[6].w, sh_v[6].w, gk);
+        gold_neg(sh_d[6].w, sh_d[6].w, gk);
+      }
+      shape_add(gsum[0], sh_v, gk, shape);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const Fe<L> o = sh_d[r];
@@ -706,13 +728,13 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       if constexpr (kAsync) {
         if (!fold && q + stride < last) issue(q + stride);
       }
-      acc[D] = gl_add(acc[D], shape_lead_lazy(sh_d, gk, shape), gk);
-      if (!skip1) acc[1] = gl_add(acc[1], shape_value_lazy(sh_v, gk, shape), gk);
+      shape_add_lead(gsum[D], sh_d, gk, shape);
+      if (!skip1) shape_add(gsum[1], sh_v, gk, shape);
 #pragma unroll
       for (int t = 2; t < D; ++t) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) sh_v[r] = gl_add_c(sh_v[r], sh_d[r], gk);
-        acc[t] = gl_add(acc[t], shape_value_lazy(sh_v, gk, shape), gk);
+        shape_add(gsum[t], sh_v, gk, shape);
       }
     } else {
       // sh_v: the values at 0, sh_d: at 1; then the values at 1 and the differences
@@ -737,6 +759,10 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
       acc[2] = fa_add(acc[2], x, F);
       acc[3] = fa_add(acc[3], y, F);
     }
+  }
+  if constexpr (kGoldLazy) {
+#pragma unroll
+    for (int t = 0; t <= DMAX; ++t) gold_acc_reduce(acc[t].w, gsum[t].w, gold_k(F));
   }
   if constexpr (kStream) {
 #pragma unroll

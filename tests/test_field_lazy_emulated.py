@@ -1,6 +1,7 @@
 """The inline-PTX arithmetic of csrc/field_m127.cuh (any representatives of residues mod
-2^127 - 1 below 2^128), run on the CPU statement by statement against big integers: random
-operands and the edges of the representation (0, p, 2^127, 2^128 - 1, and their neighbours)."""
+2^127 - 1 below 2^128) and csrc/field_gold_acc.cuh (Goldilocks sums of products reduced once),
+run on the CPU statement by statement against big integers: random operands and the edges of
+the representations (0, p, 2^127, 2^128 - 1, full words, and their neighbours)."""
 
 from __future__ import annotations
 
@@ -10,7 +11,7 @@ from pathlib import Path
 
 import pytest
 
-HEADER = Path(__file__).resolve().parents[1] / "sumcheck-triton_b200" / "csrc" / "field_m127.cuh"
+CSRC = Path(__file__).resolve().parents[1] / "sumcheck-triton_b200" / "csrc"
 M32 = (1 << 32) - 1
 P = (1 << 127) - 1
 EDGES = [0, 1, 2, P - 1, P, P + 1, P + 2, (1 << 127) + 5, (1 << 128) - 3, (1 << 128) - 2, (1 << 128) - 1, 2 * P, 2 * P + 1]
@@ -18,21 +19,27 @@ EDGES = [0, 1, 2, P - 1, P, P + 1, P + 2, (1 << 127) + 5, (1 << 128) - 3, (1 << 
 
 def _programs():
     out = {}
-    for name, body in re.findall(r"void (m127_\w+)\((.*?)\n\}\n", HEADER.read_text(), re.S):
-        text = "".join(re.findall(r'"((?:[^"\\]|\\.)*)"', body.split("asm(")[1].split('\n      : "=&r"')[0]))
-        lines = [ln.strip().rstrip(";") for ln in text.replace("\\n", "\n").replace("\\t", "").split("\n")]
-        ins = re.findall(r'"r"\((\w)\[(\d)\]\)', body)
-        out[name] = ([ln for ln in lines if ln and ln not in "{}" and not ln.startswith(".reg")], ins)
+    for header in ("field_m127.cuh", "field_gold_acc.cuh"):
+        for name, body in re.findall(r"void ((?:m127|gold)_\w+)\((.*?)\n\}\n", (CSRC / header).read_text(), re.S):
+            asm = body.split("asm(")[1]
+            text = "".join(re.findall(r'"((?:[^"\\]|\\.)*)"', asm.split('\n      : "=&r"')[0]))
+            lines = [ln.strip().rstrip(";") for ln in text.replace("\\n", "\n").replace("\\t", "").split("\n")]
+            outs = len(re.findall(r'"=&r"', asm))
+            ins = re.findall(r'"r"\(([\w.]+)(?:\[(\d)\])?\)', asm)
+            out[name] = ([ln for ln in lines if ln and ln not in "{}" and not ln.startswith(".reg")], outs, ins)
     return out
 
 
 PROGRAMS = _programs()
+GOLD = (1 << 64) - (1 << 32) + 1
+GOLD_K = {"k.one": 1, "k.zero": 0, "k.eps": M32}
 
 
 def run(name, **operands):
-    """The value (four words) the statement leaves in %0..%3."""
-    lines, ins = PROGRAMS[name]
-    regs = {f"%{4 + i}": operands[v] >> (32 * int(k)) & M32 for i, (v, k) in enumerate(ins)}
+    """The value (its words low to high) the statement leaves in its outputs."""
+    lines, outs, ins = PROGRAMS[name]
+    operands.update(GOLD_K)
+    regs = {f"%{outs + i}": operands[v] >> (32 * int(k or 0)) & M32 for i, (v, k) in enumerate(ins)}
     flag = family = None
     val = lambda x: regs[x] if x in regs else int(x, 0) & M32  # noqa: E731
     for ln in lines:
@@ -42,7 +49,9 @@ def run(name, **operands):
         if kind in ("addc", "madc", "subc"):
             assert family == ("sub" if kind == "subc" else "add"), f"{name}: {ln} reads the other family's flag"
         cin = flag if kind in ("addc", "madc", "subc") else 0
-        if kind in ("mul", "mad", "madc"):
+        if kind == "mov":
+            s = a[0]
+        elif kind in ("mul", "mad", "madc"):
             prod = a[0] * a[1]
             s = (prod & M32 if ".lo" in op else prod >> 32) + (a[2] + cin if kind != "mul" else 0)
         elif kind in ("add", "addc"):
@@ -61,10 +70,8 @@ def run(name, **operands):
             raise ValueError(ln)
         if ".cc" in op:
             flag, family = int(s < 0 or s > M32), "sub" if kind.startswith("sub") else "add"
-        elif kind in ("mad", "madc", "add", "addc"):
-            assert s <= M32 or name == "m127_canon" or "s0, c" in ln, f"{name}: {ln} drops a carry"
         regs[d] = s & M32
-    return sum(regs[f"%{k}"] << (32 * k) for k in range(4))
+    return sum(regs[f"%{k}"] << (32 * k) for k in range(outs))
 
 
 def pairs(seed, count):
@@ -95,3 +102,30 @@ def test_canonical_form():
     for a, b in pairs(9, 1500):
         for x in (a, b):
             assert run("m127_canon", a=x) == x % P, hex(x)
+
+
+def test_goldilocks_sums_of_products():
+    rng = random.Random(3)
+    edges = [0, 1, M32, 1 << 32, GOLD - 1, GOLD, GOLD + 1, (1 << 64) - 1, (1 << 64) - (1 << 32), (1 << 63)]
+    word = lambda: rng.choice(edges) if rng.random() < 0.5 else rng.getrandbits(64)  # noqa: E731
+    r_inv = pow(1 << 64, -1, GOLD)
+    for _ in range(4000):
+        x, y = word(), word()
+        t = run("gold_acc_first", x=x, y=y)
+        assert t == x * y
+        want = x * y
+        for _ in range(rng.randrange(6)):
+            x, y = word(), word()
+            t = run("gold_acc_mul", t=t, x=x, y=y)
+            want += x * y
+        if rng.random() < 0.5:
+            x = word()
+            t = run("gold_acc_add", t=t, x=x)
+            want += x << 64
+        assert t == want
+        # the carries of up to 2^31 products above 128 bits
+        t += rng.choice([0, 0, rng.getrandbits(31), (1 << 31) - 1 - (t >> 128)]) << 128
+        t = min(t, ((1 << 31) << 128) - 1)
+        assert run("gold_acc_reduce", t=t) % GOLD == t * r_inv % GOLD, hex(t)
+    for a in edges[:6]:
+        assert run("gold_neg", a=a) == GOLD - a if a <= GOLD else True
