@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
   const int tid = threadIdx.x, nthr = blockDim.x;
   uint32_t dyn_bytes;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_bytes));
+  const uint32_t* table_of = nullptr;  // the challenge the fold table is of
   if (tid == 0) cur_expr = nullptr;
   pdl_begin();
   for (int pass = 0;; ++pass) {
@@ -131,8 +132,17 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
       Fe<L> r_prev = fe_zero<L>();
       if (R.args.fold) r_prev = k == 0 ? ld_fe_cg<L>(R.args.st.chals + (R.args.round - 1) * L) : ld_fe<L>(end.r);
       const uint64_t q0 = k == 0 ? I.start : 0, q1 = k == 0 ? I.start + I.count : R.args.pairs;
+      constexpr int kTable = fold_table_words<L, K>();
+      __shared__ __align__(16) uint32_t fold_table[kTable ? kTable : 4];
+      if constexpr (kTable != 0) {
+        const uint32_t* const r_at = R.args.st.chals + (R.args.round - 1) * L;  // one table for a round's items
+        if (R.args.fold && r_at != table_of) {
+          make_fold_table<L, K>(*R.args.fc, r_prev, F, fold_table);
+          table_of = r_at;
+        }
+      }
       process_pairs<L, K, DMAX>(R.args.src, R.args.dst, R.args.src_len, R.args.fold != 0, r_prev, E, sv, sd, q0 + tid,
-                                q1, nthr, R.args.skip1 != 0, acc, F);
+                                q1, nthr, R.args.skip1 != 0, acc, F, fold_table);
       __syncthreads();
       warp_sums<L, DMAX + 1>(acc, d, smem);
       const uint32_t part = k == 0 ? static_cast<uint32_t>(R.item_base + (it - R.first_item)) : 0;

@@ -19,9 +19,9 @@ constexpr uint64_t kSkip1MinPairs = uint64_t{1} << 12;
 
 inline bool round_skip1(int n, int j) { return j >= 1 && (uint64_t{1} << (n - j - 1)) >= kSkip1MinPairs; }
 
-// Rounds of at most tail_pairs() pairs run in one block (tail.cuh): for a generic expression
-// one launch proves the rest of the proof, for the compile-time shapes a launch proves one
-// round. One SM's arithmetic bounds such a round from above, so the line falls with the work of
+// Rounds of at most tail_pairs() pairs run in one block (tail.cuh), one launch for the rest of
+// the proof (with the context's timing on, the compile-time shapes keep a launch, and a time,
+// per round). One SM's arithmetic bounds such a round from above, so the line falls with the work of
 // a pair (`units`: products of its folds and of its d + 1 points); a launch and the grid's sums
 // bound the other side, and at 8 limbs several blocks are worth them earlier. Measured on B200, us a proof at n = 14 by the
 // largest round in one block (0: none):
@@ -33,13 +33,14 @@ inline bool round_skip1(int n, int j) { return j >= 1 && (uint64_t{1} << (n - j 
 //   a b, 8 limbs (7)                    0: 225   32: 203   64: 198   256: 197   1024: 239
 //   permutation check, 8 limbs (80)     0: 487   16: 428   32: 425   64: 430   128: 462
 //   12-term gate, 8 limbs (175)         0: 826   16: 661   32: 647   64: 658   256: 850
-//   zerocheck shape, 2 limbs            0: 188   16: 179   32: 179   64: 181   256: 193
-//   g(abc + de) shape, 8 limbs          0: 464   16: 394   32: 383   64: 374   128: 383
+//   zerocheck shape, 2 limbs            2: 172   16: 160   32: 158   128: 158  256: 167
+//   zerocheck shape, 4 limbs            2: 234   16: 222   32: 219   128: 210  256: 218
+//   g(abc + de) shape, 8 limbs          2: 279   16: 275   32: 273   64: 279   128: 290
 inline uint64_t tail_pairs(const sc_expr& ex, int L, bool shaped) {
   uint64_t units = 2 * static_cast<uint64_t>(ex.num_vars);
   for (int32_t len : ex.lens) units += static_cast<uint64_t>(ex.degree + 1) * (len - 1);
   const uint64_t budget = L >= 8 ? 2600 : 66000;
-  uint64_t p = shaped ? (L >= 8 ? 64 : 32) : 256;
+  uint64_t p = shaped ? (L >= 8 ? 32 : 128) : 256;
   const uint64_t least = L >= 8 ? 32 : 64;
   while (!shaped && p > least && p * units > budget) p >>= 1;
   while (p && tail_smem_words(p, ex.num_vars, L) * 4 > static_cast<size_t>(kMaxDynSmem)) p >>= 1;
@@ -182,7 +183,7 @@ struct ProveRun {
       if (j >= tail_j) {  // this round, or this and every later one, in one block
         TailArgs T;
         T.first = A;
-        T.rounds = shape == kShapeGeneric ? stop - j : 1;
+        T.rounds = shape == kShapeGeneric || !ctx->timing ? stop - j : 1;
         T.store = j + T.rounds < stop ? 1 : 0;
         const size_t tail_smem = tail_smem_words(A.pairs, K_, L) * 4;
         cudaEvent_t ev;
@@ -196,6 +197,7 @@ struct ProveRun {
         PartArgs T;
         T.round = A;
         T.lgP = 5;
+        while ((A.pairs >> T.lgP) == 0) --T.lgP;
         while ((A.pairs >> T.lgP) > static_cast<uint64_t>(ctx->sm_count) && T.lgP < 7 &&
                (size_t{4} << T.lgP) * K_ * L * 4 <= static_cast<size_t>(kMaxDynSmem))
           ++T.lgP;
@@ -445,6 +447,12 @@ int sc_field_init(int limbs, const uint32_t* modulus, uint32_t nprime, sc_field*
   for (int w = 0; w < 8; ++w) {
     std::memcpy(C.kdig[w], x, 4 * limbs);
     for (int i = 0; i < 32; ++i) hf.dbl(x, x);
+  }
+  uint32_t y[8] = {1};
+  for (int i = 0; i < 64; ++i) hf.dbl(y, y);
+  for (int w = 0; w < 8; ++w) {
+    std::memcpy(C.kfold[w], y, 4 * limbs);
+    for (int i = 0; i < 32; ++i) hf.dbl(y, y);
   }
   for (int t = 0; t < kMaxPoints; ++t) mont_small(hf, C.r2, static_cast<uint64_t>(t), C.pts[t]);
   // Lagrange weights 1 / prod_{s != t} (t - s) (Fermat inverse; verified, p must be prime)

@@ -25,6 +25,7 @@
 #pragma once
 #include <cstdint>
 
+#include "field_bls_fold.cuh"
 #include "field_gold_acc.cuh"
 #include "field_m127.cuh"
 #include "field_ptx.cuh"
@@ -383,10 +384,58 @@ __device__ __forceinline__ void fa_mul2(Fe<L>& r0, const Fe<L>& a0, const Fe<L>&
   }
 }
 
-// Two folds by one challenge, canonical: e = x0 + r (x1 - x0), o = x2 + r (x3 - x2).
+// x0 + r (x1 - x0) and x2 + r (x3 - x2), canonical, from the table of r (field_bls_fold.cuh).
+static __device__ __noinline__ Fe8x2 bls381_fold2_call(const Fe<8> x0, const Fe<8> x1, const Fe<8> x2, const Fe<8> x3,
+                                                       const uint32_t* table) {
+  const Words8 p = bls381_p();
+  Fe<8> d0, d1;
+  ptx_sub_mod<8>(d0.w, x1.w, x0.w, p.w);
+  ptx_sub_mod<8>(d1.w, x3.w, x2.w, p.w);
+  uint32_t e0[10], o0[9], e1[10], o1[9];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+    e0[i] = i < 2 ? 0u : x0.w[i < 2 ? 0 : i - 2];
+    e1[i] = i < 2 ? 0u : x2.w[i < 2 ? 0 : i - 2];
+    if (i < 9) o0[i] = o1[i] = 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint4 a = reinterpret_cast<const uint4*>(table)[2 * i], b = reinterpret_cast<const uint4*>(table)[2 * i + 1];
+    const uint32_t c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    bls_fold_row(e0, o0, d0.w[i], c);
+    bls_fold_row(e1, o1, d1.w[i], c);
+  }
+  Fe8x2 r;
+  bls_fold_end(r.x.w, e0, o0, p.w);
+  bls_fold_end(r.y.w, e1, o1, p.w);
+  const uint32_t zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  ptx_add_mod<8>(r.x.w, r.x.w, zero, p.w);  // less p where at or above it
+  ptx_add_mod<8>(r.y.w, r.y.w, zero, p.w);
+  if (r.x.w[7] >= p.w[7]) ptx_add_mod<8>(r.x.w, r.x.w, zero, p.w);
+  if (r.y.w[7] >= p.w[7]) ptx_add_mod<8>(r.y.w, r.y.w, zero, p.w);
+  return r;
+}
+
+// Whether a field's folds take a table of the challenge, and its words in shared memory.
+template <int L, int K>
+__host__ __device__ constexpr int fold_table_words() {
+  return L == 8 && K == kFieldBls381 ? 64 : 0;
+}
+
+// Two folds by one challenge, canonical: e = x0 + r (x1 - x0), o = x2 + r (x3 - x2). table: the
+// challenge's fold table where the field takes one and the caller has it.
 template <int L, int K>
 __device__ __forceinline__ void fe_fold2(Fe<L>& e, Fe<L>& o, const Fe<L>& x0, const Fe<L>& x1, const Fe<L>& x2,
-                                         const Fe<L>& x3, const Fe<L>& r, const FieldParams<L, K>& F) {
+                                         const Fe<L>& x3, const Fe<L>& r, const FieldParams<L, K>& F,
+                                         const uint32_t* table = nullptr) {
+  if constexpr (fold_table_words<L, K>() != 0) {
+    if (table) {
+      const Fe8x2 f = bls381_fold2_call(x0, x1, x2, x3, table);
+      e = f.x;
+      o = f.y;
+      return;
+    }
+  }
   if constexpr (any_rep<L, K>()) {
     e = fa_add(x0, fa_mul(r, fa_sub(x1, x0, F), F), F);
     o = fa_add(x2, fa_mul(r, fa_sub(x3, x2, F), F), F);

@@ -63,6 +63,7 @@ struct FieldConsts {
   uint32_t one[kMaxLimbs];                   // R mod p
   uint32_t r2[kMaxLimbs];                    // R^2 mod p
   uint32_t r3[kMaxLimbs];                    // R^3 mod p
+  uint32_t kfold[8][kMaxLimbs];              // 2^(64 + 32 i) mod p (fold tables, field.cuh)
   uint32_t pts[kMaxPoints][kMaxLimbs];       // Montgomery image of t = 0..7
   uint32_t kdig[8][kMaxLimbs];               // R^2 2^(32 i) mod p: digest word i
   uint32_t lag[kMaxPoints][kMaxPoints][kMaxLimbs];  // lag[d][t] = 1 / prod_{s<=d, s!=t} (t - s)
@@ -520,7 +521,8 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
                                               uint64_t src_len, bool fold,
                                               const Fe<L>& r_prev, const ExprDev& E, uint32_t* sv, uint32_t* sd,
                                               uint64_t first, uint64_t last, uint64_t stride, bool skip1,
-                                              Fe<L> (&acc)[DMAX + 1], const FieldParams<L, K>& F) {
+                                              Fe<L> (&acc)[DMAX + 1], const FieldParams<L, K>& F,
+                                              const uint32_t* fold_table = nullptr) {
   if constexpr (SHAPE != kShapeGeneric && L == 2 && K == kFieldGoldilocks && SC_GOLD_SHAPE_FMA) {
     // the shape kernels' folds and points with every Goldilocks carry on the FMA pipe
     FieldParams<2, kFieldGoldilocksFma> G;
@@ -657,7 +659,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
           const uint4 v = __ldcs(reinterpret_cast<const uint4*>(src + (static_cast<uint64_t>(k) * L + l) * src_len) + q);
           x0.w[l] = v.x; x1.w[l] = v.y; x2.w[l] = v.z; x3.w[l] = v.w;
         }
-        fe_fold2(e, o, x0, x1, x2, x3, r_prev, F);
+        fe_fold2(e, o, x0, x1, x2, x3, r_prev, F, fold_table);
         const uint64_t dst_len = src_len >> 1;
 #pragma unroll
         for (int l = 0; l < L; ++l)
@@ -776,6 +778,19 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
   }
 }
 
+template <int L>
+__device__ __forceinline__ Fe<L> fc_get(const uint32_t* row) {
+  return ld_fe<L>(row);
+}
+
+// The fold table of r into shared memory (field_bls_fold.cuh); every thread of the block calls.
+template <int L, int K>
+__device__ __forceinline__ void make_fold_table(const FieldConsts& fc, const Fe<L>& r, const FieldParams<L, K>& F,
+                                                uint32_t* table) {
+  if (threadIdx.x < 8) st_fe<L>(table + threadIdx.x * L, fe_mul(r, fc_get<L>(fc.kfold[threadIdx.x]), F));
+  __syncthreads();
+}
+
 // ---- reduction
 //
 // Point sums are added word by word as integers: a 32-bit word splits into 16-bit halves whose
@@ -883,10 +898,6 @@ __device__ __forceinline__ bool grid_sums(const uint32_t* scratch, int d, uint32
   return grid_end<L>(d, parts, sums, counter, end);
 }
 
-template <int L>
-__device__ __forceinline__ Fe<L> fc_get(const uint32_t* row) {
-  return ld_fe<L>(row);
-}
 
 // a b R^-1 mod p, fully reduced, for a < p and any b < 2^(32 L).
 template <int L, int K>
@@ -1245,8 +1256,14 @@ __global__ void __launch_bounds__(kernel_threads(L), SHAPE ? round_min_blocks(L,
   Fe<L> r_prev = fe_zero<L>();
   if (A.fold) r_prev = ld_fe_cg<L>(A.st.chals + (A.round - 1) * L);
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * nthr;
+  constexpr int kTable = fold_table_words<L, K>();
+  __shared__ __align__(16) uint32_t fold_table[kTable ? kTable : 4];
+  if constexpr (kTable != 0) {
+    if (A.fold) make_fold_table<L, K>(*A.fc, r_prev, F, fold_table);
+  }
   process_pairs<L, K, DMAX, SHAPE>(A.src, A.dst, A.src_len, A.fold != 0, r_prev, E, sv, sd,
-                                   static_cast<uint64_t>(blockIdx.x) * nthr + tid, A.pairs, stride, A.skip1 != 0, acc, F);
+                                   static_cast<uint64_t>(blockIdx.x) * nthr + tid, A.pairs, stride, A.skip1 != 0, acc, F,
+                                   fold_table);
 
   // the block's integer sums to the grid's; the last block finalises the round
   __syncthreads();

@@ -1,6 +1,6 @@
 """The inline-PTX arithmetic of csrc/field_m127.cuh (any representatives of residues mod
-2^127 - 1 below 2^128) and csrc/field_gold_acc.cuh (Goldilocks sums of products reduced once),
-run on the CPU statement by statement against big integers: random operands and the edges of
+2^127 - 1 below 2^128), csrc/field_gold_acc.cuh (Goldilocks sums of products reduced once) and
+csrc/field_bls_fold.cuh (folds over the BLS12-381 scalar field from a table of the challenge), run on the CPU statement by statement against big integers: random operands and the edges of
 the representations (0, p, 2^127, 2^128 - 1, full words, and their neighbours)."""
 
 from __future__ import annotations
@@ -19,14 +19,15 @@ EDGES = [0, 1, 2, P - 1, P, P + 1, P + 2, (1 << 127) + 5, (1 << 128) - 3, (1 << 
 
 def _programs():
     out = {}
-    for header in ("field_m127.cuh", "field_gold_acc.cuh"):
-        for name, body in re.findall(r"void ((?:m127|gold)_\w+)\((.*?)\n\}\n", (CSRC / header).read_text(), re.S):
+    for header in ("field_m127.cuh", "field_gold_acc.cuh", "field_bls_fold.cuh"):
+        for name, body in re.findall(r"void ((?:m127|gold|bls)_\w+)\((.*?)\n\}\n", (CSRC / header).read_text(), re.S):
             asm = body.split("asm(")[1]
-            text = "".join(re.findall(r'"((?:[^"\\]|\\.)*)"', asm.split('\n      : "=&r"')[0]))
+            text = "".join(re.findall(r'"((?:[^"\\]|\\.)*)"', re.split(r'\n      : "[=+]', asm)[0]))
             lines = [ln.strip().rstrip(";") for ln in text.replace("\\n", "\n").replace("\\t", "").split("\n")]
-            outs = len(re.findall(r'"=&r"', asm))
-            ins = re.findall(r'"r"\(([\w.]+)(?:\[(\d)\])?\)', asm)
-            out[name] = ([ln for ln in lines if ln and ln not in "{}" and not ln.startswith(".reg")], outs, ins)
+            outs = len(re.findall(r'"(?:=&|\+)r"', asm))
+            tied = re.findall(r'"\+r"\((\w+)\[(\d)\]\)', asm)
+            ins = tied + re.findall(r'"r"\(([\w.]+)(?:\[(\d)\])?\)', asm)
+            out[name] = (bool(tied), [ln for ln in lines if ln and ln not in "{}" and not ln.startswith(".reg")], outs, ins)
     return out
 
 
@@ -37,9 +38,10 @@ GOLD_K = {"k.one": 1, "k.zero": 0, "k.eps": M32}
 
 def run(name, **operands):
     """The value (its words low to high) the statement leaves in its outputs."""
-    lines, outs, ins = PROGRAMS[name]
+    tied, lines, outs, ins = PROGRAMS[name]
     operands.update(GOLD_K)
-    regs = {f"%{outs + i}": operands[v] >> (32 * int(k or 0)) & M32 for i, (v, k) in enumerate(ins)}
+    first = 0 if tied else outs  # read-write operands come first and are inputs too
+    regs = {f"%{first + i}": operands[v] >> (32 * int(k or 0)) & M32 for i, (v, k) in enumerate(ins)}
     flag = family = None
     val = lambda x: regs[x] if x in regs else int(x, 0) & M32  # noqa: E731
     for ln in lines:
@@ -102,6 +104,22 @@ def test_canonical_form():
     for a, b in pairs(9, 1500):
         for x in (a, b):
             assert run("m127_canon", a=x) == x % P, hex(x)
+
+
+def test_bls_folds_from_a_table():
+    p = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
+    rng = random.Random(4)
+    edge = lambda: rng.choice([0, 1, p - 1, p - 2, (1 << 254) - 1, rng.randrange(p), rng.randrange(p)])  # noqa: E731
+    for _ in range(400):
+        r, x0, x = edge(), edge(), edge()
+        table = [r * (1 << (32 * i + 64)) % p for i in range(8)]
+        e, o = x0 << 64, 0
+        for i in range(8):
+            eo = run("bls_fold_row", e=e, o=o, x=x >> (32 * i) & M32, c=table[i])
+            e, o = eo & ((1 << 320) - 1), eo >> 320
+        assert e + (o << 32) == (x0 << 64) + sum((x >> (32 * i) & M32) * table[i] for i in range(8))
+        got = run("bls_fold_end", e=e, o=o, p=p)
+        assert got % p == (x0 + r * x) % p and got < x0 + p + (p >> 28)
 
 
 def test_goldilocks_sums_of_products():
