@@ -20,33 +20,10 @@ using namespace sc_host;
 namespace {
 // Rounds with at least this many pairs derive g(1) from the claim (see capi.cu).
 constexpr uint64_t kBatchSkip1MinPairs = uint64_t{1} << 12;
-// Tail rounds (batch_round_kernel: from a proof's first one-tile round on, that item's block
-// proves the rest of the proof) are off in batches. Measured on B200 with the 512-proof mixed
-// stream: 9.0k proofs/s with tails, 9.9k without. A 256-bit tail of ~10 rounds takes a block
-// ~200 us, longer than the late ticks it replaces (~30-45 us each), and every late tick then
-// holds some proof's tail; without tails the proofs' small rounds overlap within each tick.
-#ifndef SC_BATCH_TAILS
-#define SC_BATCH_TAILS 0
-#endif
-constexpr bool kBatchTails = SC_BATCH_TAILS != 0;
 #ifndef SC_BATCH_DMAX6
 #define SC_BATCH_DMAX6 1
 #endif
 constexpr bool kBatchDmax6 = SC_BATCH_DMAX6 != 0;  // see dispatch_dmax
-
-// Tails for fields of at most this many limbs only (0: none).
-#ifndef SC_BATCH_TAIL_MAX_L
-#define SC_BATCH_TAIL_MAX_L 0
-#endif
-
-// Ticks proof p takes: one per round, or up to its first one-tile round with tails.
-inline int proof_ticks(int n, uint64_t tile, int L) {
-  if (kBatchTails || L <= SC_BATCH_TAIL_MAX_L) {
-    for (int t = 0; t < n; ++t)
-      if ((uint64_t{1} << n) >> (t + 1) <= tile) return t + 1;
-  }
-  return n;
-}
 
 // A tick whose rounds, cut into parts of kSmallPartPairs pairs, fill the class's grid at most
 // once is cut that way, and a part is spread over its block's threads (tail.cuh): a thread a
@@ -219,9 +196,6 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
     if ((rc = batch_kernel_setup(L, B->kind, C.dmax, kmax, B->class_threads[ci], ctx->sm_count, &C.threads, &C.grid,
                                  &C.smem)))
       return rc;
-    C.max_rounds = 0;  // ticks of the class
-    for (int p : C.proofs)
-      C.max_rounds = std::max(C.max_rounds, proof_ticks(B->n[p], static_cast<uint64_t>(C.threads) * B->ppt[p], B->L));
     B->classes.push_back(std::move(C));
   }
   // per-proof state and fold buffers (16-byte aligned carve-outs of two pools)
@@ -260,16 +234,15 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
       uint64_t parts = 0;
       bool fits = true;
       for (int p : C.proofs)
-        if (t < proof_ticks(B->n[p], static_cast<uint64_t>(C.threads) * B->ppt[p], L)) {
+        if (t < B->n[p]) {
           parts += small_parts(B->n[p], t);
           fits = fits && small_part_smem(B->n[p], t, B->K[p], L) <= C.smem;
         }
       const bool small = fits && parts <= static_cast<uint64_t>(C.grid);
       for (int p : C.proofs) {
         const uint64_t tile = static_cast<uint64_t>(C.threads) * B->ppt[p];
-        const int ticks = proof_ticks(B->n[p], tile, B->L);
-        if (t >= ticks) continue;
         const int n = B->n[p];
+        if (t >= n) continue;
         const uint64_t N = uint64_t{1} << n;
         BatchRound R;
         std::memset(&R, 0, sizeof(R));
@@ -303,12 +276,6 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
         A.st.claim = s + o.claim;
         A.sums = reinterpret_cast<uint64_t*>(st + B->state_words) + static_cast<size_t>(p) * kSumCopies * kMaxPoints * L;
         R.expr = exprs_dev + p;
-        if (t == ticks - 1 && ticks < n) {
-          R.tail_rounds = n - ticks;
-          R.skip1_min_pairs = static_cast<uint32_t>(kBatchSkip1MinPairs);
-          R.fold_a = pool + fold_a[p];
-          R.fold_b = pool + fold_b[p];
-        }
         const uint64_t nitems = small ? small_parts(n, t) : (A.pairs + tile - 1) / tile;
         const uint64_t step = small ? A.pairs / nitems : tile;
         R.first_item = static_cast<int>(items.size()) - C.tick_item0[t];  // tick-relative
