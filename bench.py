@@ -106,7 +106,7 @@ def parse():
                     help="profile mode: a burst of 120 requests of the served stream (num_vars 12..18) through "
                          "the continuous server, then exit")
     ap.add_argument("--profile-aux", action="store_true",
-                    help="profile mode: the plain path's generic kernels (point-parallel 8-limb, 2-limb generic, "
+                    help="profile mode: the plain path's generic kernels (8-limb and 2-limb generic, "
                          "tail launch), a resume refold and a host-table conversion, each twice, then exit")
     return ap.parse_args()
 
@@ -757,7 +757,7 @@ def profile_served(args) -> int:
 
 def profile_aux(args) -> int:
     """Kernels outside the plain configs and the batch, on inputs larger than L2, twice each
-    (the first warms up): a generic 256-bit proof at n = 21 (point-parallel kernel, tail
+    (the first warms up): a generic 256-bit proof at n = 21 (generic round kernel, parts, tail
     launch), a generic 64-bit proof at n = 22 (generic round kernel), the refold of a 64-bit
     n = 22 transcript resumed at round 10 (fold_kernel), the Montgomery conversion of
     host tables (convert_tables_kernel), and the IMAD-rate probe (imad_probe_kernel)."""

@@ -67,7 +67,7 @@ int sc_version(void);
 const char* sc_last_error(void);
 
 /* A prover context on `device`, issuing all work on `stream` (a cudaStream_t; NULL for
- * the legacy default stream). Owns the scratch buffers (fold ping-pong, block partials,
+ * the legacy default stream). Owns the scratch buffers (fold ping-pong, round sums,
  * proof state), grown on demand. One context per host thread.
  * Replaces: the CUDA executable's per-run setup (field_sumcheck.cu:1178-1225). */
 int sc_ctx_create(int device, void* stream, sc_ctx** out);
@@ -321,7 +321,7 @@ int sc_prove_resume(sc_ctx* ctx, const sc_field* field, const sc_expr* expr,
  * call (expression, num_rounds, table kinds, seed, challenge mode): its tables are
  * generated on the device from the seed when it is admitted and stay resident, with its
  * fold buffers and transcript state, until it completes. Requests are admitted in arrival
- * order while the sum of admitted footprints (tables + fold buffers + partials + state)
+ * order while the sum of admitted footprints (tables + fold buffers + state and sums)
  * stays within hbm_budget_bytes and fewer than max_inflight are in flight.
  *
  * SC_SERVE_CONTINUOUS: continuous batching. A request whose round 0 is larger than one wave

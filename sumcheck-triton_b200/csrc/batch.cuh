@@ -8,8 +8,8 @@ namespace sc {
 //
 // Many independent proofs advance together, one launch per "tick" and degree class: a
 // persistent kernel whose blocks pull (proof round, tile of pairs) items from a device work
-// queue (an atomic counter over the tick's item list). Every item leaves one partial in its
-// round's partial slots; the block that finishes the last item of a proof's round (per-proof
+// queue (an atomic counter over the tick's item list). Every item adds its point sums to
+// its round's integer sums; the block that finishes the last item of a proof's round (per-proof
 // atomic ticket) reads that round's sums and finalises it -- SHA3 challenge included --
 // while the other blocks go on with other proofs' items. A round's items may be spread over
 // several ticks (the served prover slices large rounds): the ticket counts to the round's

@@ -11,8 +11,11 @@
 //   L = 1  inline-PTX mad.lo.cc / madc.hi.cc chain (field_ptx.cuh)     2.30  (C++ form 1.68)
 //   L = 2  Goldilocks modulus: the special reduction below              0.81
 //          any other modulus: CIOS with 64-bit intermediates (C++)     0.56  (PTX chains 0.51)
-//   L = 4  CIOS with 64-bit intermediates                               0.167 (PTX chains 0.157)
-//   L = 8  p < 2^255: even/odd-chain PTX product (ptx_mont_mul_eo)      0.065 (128 threads x 8 blocks/SM)
+//   L = 4  2^127 - 1: multiply-add chains on any representative (field_m127.cuh)
+//          other moduli: p < 2^127 the even/odd chains below, else CIOS 0.167 (PTX chains 0.157)
+//   L = 8  BLS12-381 r: even/odd chains, constant modulus, one or two products a call
+//          (bls381_mul_call, bls381_mul2_call)                         0.066-0.069
+//          p < 2^255: even/odd-chain PTX product (ptx_mont_mul_eo)     0.055-0.058
 //          other moduli: CIOS with 64-bit intermediates                0.0456 (two-chain PTX 0.034)
 //
 // The even/odd form keeps the products of even and odd limbs in two accumulators, so each is

@@ -18,7 +18,7 @@
 //      server stream). Every request whose current round has at most one wave of tiles
 //      left runs all of them; the larger rounds share the tick's budget (two waves by
 //      default) oldest request first. A round larger than its share advances over several
-//      ticks; its partial slots and ticket live in the request's block, so the launch
+//      ticks; its sums and ticket live in the request's block, so the launch
 //      holding its last tile finalises it (SHA3 challenge included) wherever that falls. A
 //      request whose last round was issued gets its state copied to pinned memory and its
 //      block freed (both stream-ordered) in the same tick;
@@ -933,7 +933,7 @@ int sc_server_create(int device, const sc_field* field, int policy, uint64_t hbm
   int no = 0;
   if (e == cudaSuccess) e = cudaMemPoolSetAttribute(S->pool, cudaMemPoolReuseAllowInternalDependencies, &no);
   if (e != cudaSuccess) return bail(fail(SC_ERR_CUDA, "memory pool attribute: %s", cudaGetErrorString(e)));
-  // one tile size for every class (a request's partial slots are sized by it)
+  // one tile size for every class (a request's rounds are cut by it)
   int cls_threads = kernel_threads(S->L);
   if (threads) cls_threads = std::min(threads, cls_threads);
   const int per_thread = round_smem_words_per_thread(max_tables, S->L, 7) * 4;

@@ -80,7 +80,7 @@ def from_limbs(words) -> int:
     return sum(int(w) << (32 * i) for i, w in enumerate(words))
 
 
-@lru_cache(maxsize=None)
+@lru_cache(maxsize=64)
 def _r_inverse(modulus: int, limbs: int) -> int:
     """R^-1 mod p, R = 2^(32 limbs)."""
     return pow(1 << (32 * limbs), -1, modulus)
