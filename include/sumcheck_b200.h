@@ -229,8 +229,8 @@ int sc_batch_results(sc_batch* batch, uint32_t* out_round_polys, uint32_t* out_c
 int sc_batch_classes(sc_batch* batch, int32_t* out_degree_class, int32_t* out_ticks, int capacity,
                      int* count);
 int sc_batch_class_proofs(sc_batch* batch, int cls, int32_t* out_indices, int capacity, int* count);
-/* Start and end of every tick of the last run, in ms from the run's start (CUDA events
- * recorded inside the graph around each launch), class after class in sc_batch_classes
+/* Start and end of every tick of the last run, in ms from the start of its first tick (the
+ * device's global timer, by the first block to start and the last to end), class after class in sc_batch_classes
  * order, available after sc_batch_wait. Classes overlap in time; a kernel's duration is
  * end - start. Only the first `capacity` are copied; *count is the number of ticks. */
 int sc_batch_tick_times(sc_batch* batch, float* out_start_ms, float* out_end_ms, int capacity,

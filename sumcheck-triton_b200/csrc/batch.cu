@@ -48,11 +48,6 @@ struct BatchClass {
   int head0 = 0;                                         // this class's first queue counter
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
-  // timing events before the first tick and after every tick, recorded inside the graph on a
-  // branch of their own (marks)
-  std::vector<cudaEvent_t> tick_events;
-  cudaStream_t marks = nullptr;
-  cudaEvent_t step = nullptr, marked = nullptr;
 };
 }  // namespace
 
@@ -74,7 +69,6 @@ struct sc_batch {
   uint32_t* host_state = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ready = nullptr, done = nullptr, fork = nullptr;
-  cudaEvent_t origin = nullptr;  // timing origin of a run (recorded inside the graph)
   cudaGraphExec_t exec = nullptr;
 };
 
@@ -161,23 +155,20 @@ int batch_kernel_launch(int L, int K, int dmax, const sc_field* field, unsigned 
 
 namespace {
 
-// The time the class's last queued kernel ends into tick event i. Event nodes between the ticks
-// would be links of the chain of kernels; on a branch of their own they leave one kernel directly
-// behind the other. Measured on B200: 64 mixed proofs 4.44 -> 4.39 ms, 24 proofs from host memory
-// 2.65 -> 2.13 ms. Setting a tick up while the one before it ends (launch_after) did not pay: its waiting
-// blocks hold room the other classes' ticks use (4.53 / 2.5 ms; for small ticks alone 4.38 / 2.15).
-int batch_mark(const BatchClass& C, int i) {
-  SC_CUDA(cudaEventRecord(C.step, C.stream));
-  SC_CUDA(cudaStreamWaitEvent(C.marks, C.step, 0));
-  SC_CUDA(cudaEventRecordWithFlags(C.tick_events[i], C.marks, cudaEventRecordExternal));
-  return SC_OK;
+// A tick. Its blocks record its start and end (BatchTickArgs::span): event nodes would be links of
+// the chain of kernels and are made, and made part of the graph, for every batch. Measured on B200 with
+// two event nodes a tick, one on a branch beside the kernels, and none: 64 mixed proofs 4.45, 4.39 and
+// 4.31 ms; 24 proofs from host memory, batches made on the way, 2.66, 2.13 and 1.49 ms.
+// Setting a tick up while the one before it ends (launch_after) did not pay: its waiting blocks hold
+// room the other classes' ticks use (64 mixed proofs 4.53 ms; for small ticks alone no change).
+int batch_tick(sc_batch* B, const BatchClass& C, const BatchTickArgs& T) {
+  const unsigned grid = static_cast<unsigned>(std::min(C.grid, std::max(1, T.num_items)));
+  return batch_kernel_launch(B->L, B->kind, C.dmax, B->field, grid, C.threads, C.smem, C.stream, T);
 }
 
-int batch_tick(sc_batch* B, const BatchClass& C, int t, const BatchTickArgs& T) {
-  const unsigned grid = static_cast<unsigned>(std::min(C.grid, std::max(1, T.num_items)));
-  const int rc = batch_kernel_launch(B->L, B->kind, C.dmax, B->field, grid, C.threads, C.smem, C.stream, T);
-  return rc ? rc : batch_mark(C, t + 1);
-}
+// The ticks' queue counters, then their spans (16-byte aligned), zeroed before each run.
+inline size_t span_offset(const sc_batch* B) { return (static_cast<size_t>(std::max(1, B->total_heads)) * 4 + 15) & ~size_t{15}; }
+inline size_t heads_bytes(const sc_batch* B) { return span_offset(B) + static_cast<size_t>(std::max(1, B->total_heads)) * 16; }
 
 template <int L>
 int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const* tables) {
@@ -312,7 +303,7 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
   }
   if ((rc = ensure(ctx, B->rounds, rounds.size() * sizeof(BatchRound)))) return rc;
   if ((rc = ensure(ctx, B->items, items.size() * sizeof(BatchItem)))) return rc;
-  if ((rc = ensure(ctx, B->heads, static_cast<size_t>(std::max(1, B->total_heads)) * 4))) return rc;
+  if ((rc = ensure(ctx, B->heads, heads_bytes(B)))) return rc;
   SC_CUDA(cudaMemcpy(B->rounds.p, rounds.data(), rounds.size() * sizeof(BatchRound), cudaMemcpyHostToDevice));
   SC_CUDA(cudaMemcpy(B->items.p, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice));
   SC_CUDA(cudaMemcpy(B->exprs.p, ed.data(), ed.size() * sizeof(ExprDev), cudaMemcpyHostToDevice));
@@ -322,12 +313,10 @@ int batch_setup(sc_batch* B, const sc_expr* const* exprs, const uint32_t* const*
 // The launch sequence of one run (captured once into the graph).
 int batch_issue(sc_batch* B) {
   SC_CUDA(cudaMemsetAsync(B->state.p, 0, B->state_words * 4 + B->count * sums_bytes(B->L), B->stream));
-  SC_CUDA(cudaMemsetAsync(B->heads.p, 0, static_cast<size_t>(std::max(1, B->total_heads)) * 4, B->stream));
-  SC_CUDA(cudaEventRecordWithFlags(B->origin, B->stream, cudaEventRecordExternal));
+  SC_CUDA(cudaMemsetAsync(B->heads.p, 0, heads_bytes(B), B->stream));
   SC_CUDA(cudaEventRecord(B->fork, B->stream));
   for (BatchClass& C : B->classes) {
     SC_CUDA(cudaStreamWaitEvent(C.stream, B->fork, 0));
-    if (const int rc = batch_mark(C, 0)) return rc;
     for (int t = 0; t < C.max_rounds; ++t) {
       BatchTickArgs T;
       T.rounds = static_cast<const BatchRound*>(B->rounds.p) + C.tick_round0[t];
@@ -336,13 +325,12 @@ int batch_issue(sc_batch* B) {
       T.lgP = -1;
       T.head = static_cast<uint32_t*>(B->heads.p) + C.head0 + t;
       T.tile = 0;
-      const int rc = batch_tick(B, C, t, T);
+      T.span = reinterpret_cast<unsigned long long*>(static_cast<char*>(B->heads.p) + span_offset(B)) + 2 * (C.head0 + t);
+      const int rc = batch_tick(B, C, T);
       if (rc) return rc;
     }
     SC_CUDA(cudaEventRecord(C.done, C.stream));
     SC_CUDA(cudaStreamWaitEvent(B->stream, C.done, 0));
-    SC_CUDA(cudaEventRecord(C.marked, C.marks));
-    SC_CUDA(cudaStreamWaitEvent(B->stream, C.marked, 0));
   }
   SC_CUDA(cudaMemcpyAsync(B->host_state, B->state.p, B->state_words * 4, cudaMemcpyDeviceToHost, B->stream));
   return SC_OK;
@@ -398,19 +386,10 @@ int sc_batch_create_tiled(sc_ctx* ctx, const sc_field* field, int count, const s
   if (!rc && e == cudaSuccess) e = cudaEventCreateWithFlags(&B->ready, cudaEventDisableTiming);
   if (!rc && e == cudaSuccess) e = cudaEventCreateWithFlags(&B->done, cudaEventDisableTiming);
   if (!rc && e == cudaSuccess) e = cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming);
-  if (!rc && e == cudaSuccess) e = cudaEventCreate(&B->origin);
   for (size_t c = 0; !rc && e == cudaSuccess && c < B->classes.size(); ++c) {
     BatchClass& C = B->classes[c];
     e = cudaStreamCreateWithFlags(&C.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&C.marks, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&C.step, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&C.marked, cudaEventDisableTiming);
-    for (int i = 0; e == cudaSuccess && i <= C.max_rounds; ++i) {
-      cudaEvent_t ev;
-      e = cudaEventCreate(&ev);
-      if (e == cudaSuccess) C.tick_events.push_back(ev);
-    }
   }
   if (!rc && e != cudaSuccess) rc = fail(SC_ERR_CUDA, "batch streams/events: %s", cudaGetErrorString(e));
   if (rc) {
@@ -484,16 +463,20 @@ int sc_batch_tick_times(sc_batch* B, float* out_start_ms, float* out_end_ms, int
   int k = 0;
   for (const BatchClass& C : B->classes) k += C.max_rounds;
   *count = k;
-  int i = 0;
-  for (const BatchClass& C : B->classes)
-    for (int t = 0; t < C.max_rounds; ++t, ++i) {
-      if (i >= capacity) continue;
-      float a = 0.f, b = 0.f;
-      SC_CUDA(cudaEventElapsedTime(&a, B->origin, C.tick_events[t]));
-      SC_CUDA(cudaEventElapsedTime(&b, B->origin, C.tick_events[t + 1]));
-      if (out_start_ms) out_start_ms[i] = a;
-      if (out_end_ms) out_end_ms[i] = b;
-    }
+  if (capacity < 1 || k < 1) return SC_OK;
+  if (!B->exec) return fail(SC_ERR_CUDA, "tick times: the batch has not run");
+  SC_CUDA(cudaSetDevice(B->ctx->device));
+  SC_CUDA(cudaEventQuery(B->done));  // the last run has ended
+  std::vector<unsigned long long> span(static_cast<size_t>(2) * k);
+  SC_CUDA(cudaMemcpyAsync(span.data(), static_cast<const char*>(B->heads.p) + span_offset(B), span.size() * 8,
+                          cudaMemcpyDeviceToHost, B->stream));
+  SC_CUDA(cudaStreamSynchronize(B->stream));
+  unsigned long long origin = ~0ull;
+  for (int i = 0; i < k; ++i) origin = std::min(origin, ~span[2 * i]);
+  for (int i = 0; i < k && i < capacity; ++i) {  // in the order of the classes' ticks, as head0 counts them
+    if (out_start_ms) out_start_ms[i] = static_cast<float>(~span[2 * i] - origin) * 1e-6f;
+    if (out_end_ms) out_end_ms[i] = static_cast<float>(span[2 * i + 1] - origin) * 1e-6f;
+  }
   return SC_OK;
 }
 
@@ -562,17 +545,12 @@ int sc_batch_destroy(sc_batch* B) {
     if (b->p) cudaFree(b->p);
   if (B->host_state) cudaFreeHost(B->host_state);
   for (BatchClass& C : B->classes) {
-    for (cudaEvent_t e : C.tick_events) cudaEventDestroy(e);
     if (C.done) cudaEventDestroy(C.done);
-    if (C.step) cudaEventDestroy(C.step);
-    if (C.marked) cudaEventDestroy(C.marked);
-    if (C.marks) cudaStreamDestroy(C.marks);
     if (C.stream) cudaStreamDestroy(C.stream);
   }
   if (B->ready) cudaEventDestroy(B->ready);
   if (B->done) cudaEventDestroy(B->done);
   if (B->fork) cudaEventDestroy(B->fork);
-  if (B->origin) cudaEventDestroy(B->origin);
   if (B->stream) cudaStreamDestroy(B->stream);
   delete B;
   return SC_OK;

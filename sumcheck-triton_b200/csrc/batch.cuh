@@ -49,7 +49,15 @@ struct BatchTickArgs {
   uint32_t* head;          // queue counter of this tick (zero before the launch); nullptr:
                            // block b does item b alone (grid = num_items)
   uint64_t tile;           // pairs per item when items is nullptr
+  unsigned long long* span;  // non-null (zero before the launch): [0] the complement of the first
+                             // block's start, [1] the last one's end (nanoseconds)
 };
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 
 // prove_tail out of line: the tick's own register budget does not see it.
 template <int L, int K>
@@ -86,6 +94,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
   const uint32_t* table_of = nullptr;  // the challenge the fold table is of
   if (tid == 0) cur_expr = nullptr;
   pdl_begin();
+  if (T.span && tid == 0) atomicMax(T.span, ~global_ns());
   for (int pass = 0;; ++pass) {
     __syncthreads();
     if (tid == 0)
@@ -167,6 +176,7 @@ __global__ void __launch_bounds__(kernel_threads(L), batch_min_blocks(L, DMAX))
       __syncthreads();
     }
   }
+  if (T.span && tid == 0) atomicMax(T.span + 1, global_ns());
 }
 
 }  // namespace sc

@@ -431,6 +431,7 @@ int issue_large(sc_server* S, ServeRequest* R) {
     A.lgP = part[t];
     A.head = nullptr;
     A.tile = tiles[t];
+    A.span = nullptr;
     rc = batch_kernel_launch(S->L, S->kind, C.dclass, S->field, static_cast<unsigned>(A.num_items), C.threads, C.smem,
                              lane, A, t > R->first);
     if (rc) return rc;
@@ -658,6 +659,7 @@ int issue_tick(sc_server* S, bool* issued) {
     A.lgP = -1;
     A.head = reinterpret_cast<uint32_t*>(T.dev) + c;
     A.tile = 0;
+    A.span = nullptr;
     SC_CUDA(cudaStreamWaitEvent(C.stream, S->fork, 0));
     const unsigned grid = static_cast<unsigned>(std::min(C.grid, std::max(1, A.num_items)));
     int rc = batch_kernel_launch(S->L, S->kind, C.dclass, S->field, grid, C.threads, C.smem, C.stream, A);
