@@ -348,7 +348,7 @@ def busy_ms(intervals) -> float:
 def group_alone_rooflines(work, batch_items, work_per_round, tuning, device, hbm_peak: float,
                           imad_rate: float) -> dict:
     """Each field group of the stream proved alone (its own BatchProver, the same tiles),
-    outside the timed region: its ticks' busy time (CUDA events inside the graph, last of 3
+    outside the timed region: its ticks' busy time (the device's timer, last of 3
     timed runs), and its algorithmic bytes and IMAD over that time against the group's own
     bound -- HBM for the 2-limb group, the IMAD rate for the 8-limb group. In the timed step
     the two groups share the SMs, so their by-class rates there are not rooflines."""
@@ -594,8 +594,8 @@ def main() -> int:
         ms_plain, plain_launch_ms = ms_step, launch_ms
 
     # roofline of the dominant kernel class: algorithmic work per launch over CUDA-event
-    # durations. Batched: the tick times of the last run of the timed region (events inside
-    # the graph); plain: every launch of its timed region.
+    # durations. Batched: the tick times of the last run of the timed region (the device's
+    # timer, read by the ticks' blocks); plain: every launch of its timed region.
     per_class = {}
 
     def add(L, ms, b, im, launches=1):
@@ -615,8 +615,7 @@ def main() -> int:
     if path == "batched":
         # Degree classes of one field run concurrently on their own streams: a field's
         # kernel time is the union of its ticks' [start, end] intervals (busy time).
-        # a class's work is every round of its proofs (the last tick of a proof also proves its
-        # tail rounds, so ticks and rounds do not map one to one)
+        # a class's work is every round of its proofs
         classes = batcher.tick_times()
         spans = {}
         for c in classes:

@@ -64,3 +64,20 @@ def test_every_degree_matches_c_oracle(modulus, bits, degree):
 @pytest.mark.parametrize("n", [15, 17])
 def test_many_blocks_match_c_oracle(bits, n):
     check(expression(3, n), get_field(bits), n, seed=n)
+
+
+def test_tick_times_follow_each_other():
+    from zkduel_b200.batch import BatchProver
+
+    for bits, n in ((32, 1), (64, 5), (256, 9)):
+        spec = get_field(bits)
+        expr = ((1, ("a", "b")), (3, ("c",)))
+        bp = BatchProver([(expr, bits, n, api.generate_tables(spec, 3, n, [0] * 3, 7))])
+        with pytest.raises(Exception):
+            bp.tick_times()  # not run yet
+        for _ in range(2):
+            bp.run()
+            (c,) = bp.tick_times()
+            assert len(c["ms"]) == n and c["start"][0] == 0.0
+            assert all(0 < b - a < 1e3 for a, b in zip(c["start"], c["end"]))
+            assert all(nxt >= end for end, nxt in zip(c["end"], c["start"][1:]))
