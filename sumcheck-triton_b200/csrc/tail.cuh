@@ -162,7 +162,8 @@ __device__ __forceinline__ void tail_eval(const ExprDev& E, const FieldParams<L,
 // barrier. A (shared memory) describes the first of them, with A.pairs a power of two, and is
 // advanced from round to round; r_ready: end.r holds the challenge its fold needs. smem:
 // tail_smem_words(A.pairs, tables, L) words. store: T_j of the last of the rounds also goes to
-// A.dst. The rounds after the first never take g(1) from the claim.
+// A.dst. The first round may take g(1) from the claim or check it (A's flags); the rounds after it
+// do neither, whatever their size: point 1 is one more task beside the others here.
 template <int L, int K>
 __device__ __forceinline__ void prove_tail(RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F, int rounds,
                                            bool r_ready, bool store, uint32_t* smem, RoundEnd<L>& end) {
@@ -177,7 +178,7 @@ __device__ __forceinline__ void prove_tail(RoundArgs& A, const ExprDev& E, const
     tail_fold<L, K>(A, nv, F, r, 0, lgP, k == 0 ? nullptr : nxt, store && k == rounds - 1, cur);
     for (int i = tid; i < kMaxPoints * L * 2; i += nthr) end.half[i] = 0;
     __syncthreads();
-    tail_eval<L, K>(E, F, cur, lgP, k == 0 && A.skip1, end.half);
+    tail_eval<L, K>(E, F, cur, lgP, A.skip1 != 0, end.half);
     if (tid == 0) A.last = cur;
     __syncthreads();
     finish_round<L, K>(A, E, F, consts, [&](int i) { return end.half_sum(i); }, end);
@@ -187,6 +188,7 @@ __device__ __forceinline__ void prove_tail(RoundArgs& A, const ExprDev& E, const
       ++A.round;
       A.pairs >>= 1;
       A.fold = 1;
+      A.skip1 = A.want_claim = A.check_claim = 0;  // the claim belonged to the first round
     }
     // T_j becomes the source; T_{j+1} goes where T_{j-1} was (the first time: behind T_j)
     uint32_t* const t = cur;

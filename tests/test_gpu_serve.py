@@ -171,6 +171,21 @@ def test_other_fields_and_errors():
             srv.result(rid)
 
 
+@pytest.mark.parametrize("pairs_per_thread,max_tables", [(32, 24), (64, 32)])
+@pytest.mark.parametrize("bits", [32, 64, 128])
+@pytest.mark.parametrize("expr", [((1, ("a", "a")),), ((3, ("a", "a", "a")), (1, ("a",)))], ids=["d2", "d3"])
+def test_tails_that_start_with_a_round_from_the_claim(bits, expr, pairs_per_thread, max_tables):
+    """Tiles of 8192 pairs or more and one table: a block's tail starts at a round of 4096 pairs,
+    which takes g(1) from the claim; the rounds after it must not."""
+    spec = get_field(bits)
+    with ProofServer(spec, max_tables=max_tables, pairs_per_thread=pairs_per_thread) as srv:
+        jobs = [(n, srv.submit(expr, n, 60 + n)) for n in (13, 14, 15)]
+        srv.drain(timeout_ms=60_000)
+        for n, rid in jobs:
+            t = api.generate_tables(spec, 1, n, [0], 60 + n)
+            _same(srv.result(rid), api.prove_device(t, expr, spec, n))
+
+
 def test_replay_reports_latencies():
     reqs = served_stream(40, rate_per_s=2000.0, seed=3, min_vars=6, max_vars=12)
     with ProofServer(SPEC) as srv:
