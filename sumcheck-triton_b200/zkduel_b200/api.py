@@ -206,8 +206,8 @@ class Proof:
 
     @property
     def round_polys(self) -> list[list[int]]:
-        values, d1 = self.field.decode_array(self.round_polys_mont), self.degree + 1
-        return [values[i:i + d1] for i in range(0, len(values), d1)]
+        values, n = self.field.decode_array(self.round_polys_mont), len(self.round_polys_mont)
+        return [values[i * len(values) // n:(i + 1) * len(values) // n] for i in range(n)]
 
     @property
     def challenges(self) -> list[int]:

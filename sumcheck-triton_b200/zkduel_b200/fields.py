@@ -24,8 +24,11 @@ import random
 from dataclasses import dataclass
 from functools import lru_cache
 
+import numpy as np
+
 MASK32 = 0xFFFFFFFF
 SUPPORTED_LIMBS = (1, 2, 4, 8)
+_WORD = np.dtype("<u4")
 MAX_POINTS = 8  # interpolation points t = 0..7, so degree <= 7 (field_sumcheck.cu:29)
 
 
@@ -124,8 +127,12 @@ class FieldSpec:
         return to_limbs(self.montgomery_encode(value), self.limbs)
 
     def decode_array(self, limbs) -> list[int]:
-        """Canonical values of an array of Montgomery-form uint32 limb vectors (last axis)."""
-        data, size, p, r_inv = limbs.tobytes(), 4 * self.limbs, self.modulus, self.r_inv
+        """Canonical values of an array of Montgomery-form limb vectors (last axis): native uint32
+        arrays, as the library writes them, from their bytes; other types and lists word by word."""
+        if getattr(limbs, "dtype", None) != _WORD:
+            a = np.asarray(limbs, dtype=object)
+            return [self.decode_limbs(v) for v in a.reshape(-1, a.shape[-1])] if a.size else []
+        data, size, p, r_inv = limbs.tobytes(), 4 * limbs.shape[-1], self.modulus, self.r_inv
         return [int.from_bytes(data[i:i + size], "little") * r_inv % p for i in range(0, len(data), size)]
 
     def decode_limbs(self, words) -> int:

@@ -10,7 +10,7 @@ import pytest
 from conftest import load_jsonl
 from zkduel_b200 import expression as X
 from zkduel_b200 import fields as F
-from zkduel_b200.api import host_tables_to_limbs
+from zkduel_b200.api import Proof, host_tables_to_limbs
 from zkduel_b200.workloads import KERNEL_WORKLOADS, WORKLOADS, get_kernel_workload, get_workload
 
 GUARD = load_jsonl("guard_cases.jsonl")
@@ -105,3 +105,27 @@ def test_host_tables_to_limbs():
     big = [[f256.modulus + 3, -1]]
     out = host_tables_to_limbs(big, f256)
     assert F.from_limbs(out[0, :, 0].tolist()) == 3 and F.from_limbs(out[0, :, 1].tolist()) == f256.modulus - 1
+
+
+@pytest.mark.parametrize("bits", [32, 64, 128, 256])
+@pytest.mark.parametrize("kind", ["uint32", "uint64", "int64", ">u4", "object", "list", "strided"])
+def test_proof_decodes_limbs_of_any_integer_type(kind, bits):
+    """A proof read back from a file or built by a caller may hold its limbs in wider types or lists."""
+    f = F.FIELD_SPECS[bits]
+    rng = random.Random(bits)
+    values = lambda *shape: np.array([rng.randrange(f.modulus) for _ in range(int(np.prod(shape)))], dtype=object).reshape(shape)  # noqa: E731
+    polys, chals, finals, claim = values(3, 4), values(3), values(5), values(1)
+
+    def limbs(v):
+        a = np.array([f.montgomery_limbs(x) for x in v.ravel()], dtype=np.uint32).reshape(*v.shape, f.limbs)
+        if kind == "list":
+            return a.tolist()
+        if kind == "strided":
+            return np.repeat(a, 2, axis=-1)[..., ::2]
+        return a.astype(kind)
+
+    p = Proof(f, 3, 3, ("a",), limbs(polys), limbs(chals), limbs(finals), limbs(claim)[0], 0)
+    assert p.round_polys == polys.tolist() and p.challenges == chals.tolist()
+    assert p.claim0 == claim[0] and p.final_claim == finals[0] and p.final_values == finals[1:].tolist()
+    empty = Proof(f, 0, 3, (), limbs(polys)[:0], limbs(chals)[:0], limbs(finals)[:1], limbs(claim)[0], 0)
+    assert empty.round_polys == [] and empty.challenges == [] and empty.final_values == []
