@@ -263,7 +263,7 @@ def host_tables_to_limbs(values: Sequence[Sequence[int]] | np.ndarray, spec: Fie
                 arr = arr % np.uint64(q)
         K, N = arr.shape
         words = np.ascontiguousarray(arr).view(np.dtype("<u4")).reshape(K, N, 2)
-        return np.ascontiguousarray(words[:, :, :L].transpose(0, 2, 1))
+        return words[:, :, :L].transpose(0, 2, 1).copy()  # a copy also where the order is already right
     rows = [np.array([int(x) % q for x in row], dtype=object) for row in values]
     K, N = len(rows), len(rows[0]) if rows else 0
     out = np.empty((K, L, N), dtype=np.uint32)

@@ -129,3 +129,18 @@ def test_proof_decodes_limbs_of_any_integer_type(kind, bits):
     assert p.claim0 == claim[0] and p.final_claim == finals[0] and p.final_values == finals[1:].tolist()
     empty = Proof(f, 0, 3, (), limbs(polys)[:0], limbs(chals)[:0], limbs(finals)[:1], limbs(claim)[0], 0)
     assert empty.round_polys == [] and empty.challenges == [] and empty.final_values == []
+
+
+@pytest.mark.parametrize("bits", [32, 64])
+@pytest.mark.parametrize("entries", [0, 1, 2, 8])
+def test_host_limbs_are_the_callers_to_change(bits, entries):
+    """The limbs never share memory with the caller's table, at any length."""
+    f = F.FIELD_SPECS[bits]
+    vals = np.arange(3 * entries, dtype=np.uint64).reshape(3, entries)
+    out = host_tables_to_limbs(vals, f)
+    assert out.shape == (3, f.limbs, entries) and out.dtype == np.uint32 and out.flags.c_contiguous
+    assert not np.shares_memory(out, vals) and out.flags.writeable
+    vals.flags.writeable = False
+    out = host_tables_to_limbs(vals, f)
+    out[...] = 7
+    assert vals.tolist() == np.arange(3 * entries).reshape(3, entries).tolist()
