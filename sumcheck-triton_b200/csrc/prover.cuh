@@ -1053,9 +1053,10 @@ __device__ __forceinline__ void begin_message(RoundEnd<L>& end, int d, int j, in
 }
 
 // The end of round j, with g_j complete in end.g() and begin_message done; every thread of the
-// block calls, after a barrier. Warp 0 derives r_j (into end.r too, for a caller that goes on
-// with the next round in this block, after a barrier of its own); the next warp, if there is
-// one, stores the round polynomial, the checksum and the claim of round 0 meanwhile.
+// block calls, after a barrier. Warp 0 checks the claim, derives r_j (into end.r too, for a caller
+// that goes on with the next round in this block, after a barrier of its own) and writes the next
+// claim; the next warp, if there is one, stores the round polynomial, the checksum and the claim
+// of round 0 meanwhile.
 template <int L, int K>
 __device__ __forceinline__ void finalize_round(const RoundArgs& A, const ExprDev& E, const FieldParams<L, K>& F,
                                                const EndConsts<L>& consts, RoundEnd<L>& end) {
@@ -1065,7 +1066,7 @@ __device__ __forceinline__ void finalize_round(const RoundArgs& A, const ExprDev
   const int j = A.round;
   const FieldConsts& fc = *A.fc;
   if (warp == (blockDim.x > 32 ? 1 : 0)) {
-    // round polynomial, checksum, claim checks
+    // round polynomial, checksum, the first round's claim
     uint64_t cs = 0;
     for (int i = lane; i < (d + 1) * L; i += 32) {
       const uint32_t w = g_sm[i];
@@ -1076,20 +1077,20 @@ __device__ __forceinline__ void finalize_round(const RoundArgs& A, const ExprDev
     for (int off = 16; off > 0; off >>= 1) cs += __shfl_down_sync(0xffffffffu, cs, off);
     if (lane == 0) {
       *A.st.checksum += cs;
-      if (j == 0 || (A.check_claim && !A.skip1)) {
-        const Fe<L> s = fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F);
-        if (j == 0) st_fe<L>(A.st.claim0, s);
-        if (A.check_claim && !A.skip1) {
-          const Fe<L> c = ld_fe_cg<L>(A.st.claim);
-          bool eq = true;
-#pragma unroll
-          for (int l = 0; l < L; ++l) eq = eq && s.w[l] == c.w[l];
-          if (!eq) atomicOr(A.st.status, kStatusClaim);
-        }
-      }
+      if (j == 0) st_fe<L>(A.st.claim0, fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F));
     }
   }
   if (warp != 0) return;
+  if (A.check_claim && !A.skip1) {  // by the warp that writes the next claim below, and before it does
+    if (lane == 0) {
+      const Fe<L> s = fe_add(ld_fe<L>(g_sm), ld_fe<L>(g_sm + L), F), c = ld_fe_cg<L>(A.st.claim);
+      bool eq = true;
+#pragma unroll
+      for (int l = 0; l < L; ++l) eq = eq && s.w[l] == c.w[l];
+      if (!eq) atomicOr(A.st.status, kStatusClaim);
+    }
+    __syncwarp();
+  }
   const bool last_round = j == A.num_rounds - 1;
   const bool claim = A.want_claim || last_round;
   // What the end of the round reads from global memory, before the hash: the digest's weights

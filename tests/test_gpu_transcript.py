@@ -236,3 +236,28 @@ def test_resume_checks_the_recorded_claim_against_the_tables(bw, expr, n, j):
         tr.prove_rounds(other, expr, spec, n, a)
     # the context proves normally afterwards
     _same(api.prove_device(t, expr, spec, n, "sha3"), whole)
+
+
+@pytest.mark.parametrize("mode", ["sha3", "fixed", "explicit"])
+@pytest.mark.parametrize("bw,expr,n,j", [
+    (32, ((1, ("a", "b")),), 16, 1),   # a first round of 16384 pairs and more: it checks the recorded
+    (64, ((1, ("x", "y")),), 16, 2),   # claim and writes the one of the round after it
+    (64, ZEROCHECK, 15, 1),
+    (128, ((1, ("a", "b", "c")), (3, ("d",))), 16, 2),
+    (256, ((1, ("a", "b")), (3, ("c",))), 17, 1),
+    (256, ((1, ("a", "b", "c", "g")), (1, ("d", "e", "g"))), 15, 1),
+])
+def test_resume_checks_the_claim_before_the_next_one_is_written(bw, expr, n, j, mode):
+    spec = get_field(bw)
+    t, _ = _tables(spec, expr, n, 700 + n)
+    rng = random.Random(n)
+    ch = [rng.randrange(spec.modulus) for _ in range(n)] if mode == "explicit" else None
+    args = (ch,) if ch else ()
+    whole = api.prove_device(t, expr, spec, n, mode, *args)
+    a = tr.prove_rounds(t, expr, spec, j, tr.start(expr, spec, n, mode), *args)
+    for _ in range(5):
+        _same(tr.result(tr.prove_rounds(t, expr, spec, n, a, *args), expr, spec), whole)
+    bad = a.words.copy()
+    bad[-spec.limbs] ^= 1
+    with pytest.raises(_lib.SumcheckError, match="device status 1"):
+        tr.prove_rounds(t, expr, spec, n, tr.Transcript(bad), *args)
