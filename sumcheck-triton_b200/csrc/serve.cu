@@ -441,8 +441,6 @@ int issue_large(sc_server* S, ServeRequest* R) {
   SC_CUDA(cudaFreeAsync(R->block, lane));
   R->block = nullptr;
   SC_CUDA(cudaEventRecord(S->stage_events[R->slot], lane));
-  ++S->lane_load[R->lane];
-  S->lane_inflight.push_back(R);
   return SC_OK;
 }
 
@@ -513,10 +511,14 @@ int admit(sc_server* S) {
     R->t_admit = S->now();
     S->admitted_bytes += R->footprint;
     mark_busy(S);
+    // listed before anything is issued: if that fails, fail_all finds the request
     if (R->large) {
+      ++S->lane_load[R->lane];
+      S->lane_inflight.push_back(R);
       int rc = issue_large(S, R);
       if (rc) return rc;
     } else {
+      S->active.push_back(R);
       SC_CUDA(cudaMemsetAsync(R->state, 0, state_and_sums_bytes(R->so, S->L), S->stream));
       if (R->first)
         SC_CUDA(cudaMemcpyAsync(R->state, R->resume_state.data(), R->so.total_words * 4, cudaMemcpyHostToDevice,
@@ -529,7 +531,6 @@ int admit(sc_server* S) {
         rc = resume_folds(S->field, R->n, R->K, R->tables, R->fold_a, R->fold_b, R->state + R->so.chals, R->first,
                           S->ctx->sm_count, S->stream);
       if (rc) return rc;
-      S->active.push_back(R);
     }
     std::lock_guard<std::mutex> lk(S->mu);
     S->stats.peak_inflight = std::max<uint64_t>(S->stats.peak_inflight, S->active.size() + S->lane_inflight.size());
@@ -556,6 +557,7 @@ int issue_tick(sc_server* S, bool* issued) {
   for (ServeRequest* R : suspend_now) {
     R->suspending = true;
     S->active.erase(std::find(S->active.begin(), S->active.end(), R));
+    T.completing.push_back(R);
   }
   const int nc = static_cast<int>(S->classes.size());
   std::vector<std::vector<BatchRound>> rounds(nc);
@@ -674,7 +676,6 @@ int issue_tick(sc_server* S, bool* issued) {
     SC_CUDA(cudaFreeAsync(R->block, S->stream));
     R->block = nullptr;
     S->admitted_bytes -= R->footprint;
-    T.completing.push_back(R);
   }
   for (ServeRequest* R : done_now) {
     SC_CUDA(cudaMemcpyAsync(S->stage_host + static_cast<size_t>(R->slot) * S->stage_words, R->state,
@@ -699,19 +700,36 @@ int issue_tick(sc_server* S, bool* issued) {
   return SC_OK;
 }
 
-// Fails every request the worker holds (after a CUDA error the stream is unusable).
+// Fails every request the worker holds, after a failed call, and takes back what they held: their
+// blocks (once the work issued for them has ended), staging slots and budget.
 void fail_all(sc_server* S, int rc) {
-  const double t = S->now();
+  for (ServeClass& C : S->classes) cudaStreamSynchronize(C.stream);
+  cudaStreamSynchronize(S->stream);
+  for (cudaStream_t st : S->lane) cudaStreamSynchronize(st);
   std::vector<ServeRequest*> all(S->waiting.begin(), S->waiting.end());
   all.insert(all.end(), S->active.begin(), S->active.end());
   all.insert(all.end(), S->lane_inflight.begin(), S->lane_inflight.end());
-  for (int s = 0; s < kSlots; ++s)
-    for (ServeRequest* R : S->slots[s].completing) all.push_back(R);
   S->waiting.clear();
   S->active.clear();
   S->lane_inflight.clear();
-  for (int s = 0; s < kSlots; ++s) S->slots[s].completing.clear();
+  for (TickSlot& T : S->slots) {
+    all.insert(all.end(), T.completing.begin(), T.completing.end());
+    T.completing.clear();
+    T.busy = false;
+  }
   S->slots_in_flight.clear();
+  for (ServeRequest* R : all) {
+    if (R->block) cudaFreeAsync(R->block, S->stream);
+    R->block = nullptr;
+    R->slot = -1;
+  }
+  S->admitted_bytes = 0;
+  std::fill(S->lane_load, S->lane_load + kLanes, 0);
+  S->free_stage.clear();
+  for (int i = S->max_inflight - 1; i >= 0; --i) S->free_stage.push_back(i);
+  cudaGetLastError();
+  mark_idle_if_done(S);
+  const double t = S->now();
   for (ServeRequest* R : all) publish(S, R, rc, t);
 }
 
@@ -751,13 +769,7 @@ void loop_continuous(sc_server* S) {
       else
         lane_only = !S->lane_inflight.empty();
     }
-    if (rc) {
-      fail_all(S, rc);
-      cudaStreamSynchronize(S->stream);
-      for (cudaStream_t st : S->lane) cudaStreamSynchronize(st);
-      std::fill(S->lane_load, S->lane_load + kLanes, 0);
-      cudaGetLastError();
-    }
+    if (rc) fail_all(S, rc);
   }
 }
 
