@@ -97,8 +97,10 @@ class BatchProver:
     def launch(self) -> None:
         """Enqueues one run of every group (asynchronous). Every group is launched before any
         is joined to the caller's stream, so the groups run concurrently on their own streams."""
-        self._start()
-        self._join()
+        try:
+            self._start()
+        finally:  # also the groups launched before one that failed
+            self._join()
 
     def _start(self) -> None:
         """Every group, on its own streams, after the work already on the caller's stream."""
@@ -289,27 +291,30 @@ class HostBatchProver:
         main = self.stream
         for st in self.copy_streams:
             st.wait_stream(main)  # the device tables are free again
-        k = 0
-        for a, b, bp in self.chunks:
-            for i in range(a, b):
-                with torch.cuda.stream(self.copy_streams[k % len(self.copy_streams)]):
-                    self.dev_tables[i].copy_(self.host[i], non_blocking=True)
-                k += 1
-            for st in self.copy_streams:  # this chunk's copies, not the later ones
-                ev = torch.cuda.Event()
-                ev.record(st)
-                main.wait_event(ev)
-            for i in range(a, b):
-                t = self.dev_tables[i]
-                fld = get_device_field(self.specs[i], self.ctx.device)
-                K, _L, N = t.shape
-                _lib.check(lib.sc_tables_to_mont(self.ctx.handle, fld.handle, ctypes.c_void_p(t.data_ptr()),
-                                                 ctypes.c_uint64(N), int(K)), "sc_tables_to_mont")
-            bp._start()
-        # joined only now: a chunk's last rounds leave most of the GPU idle, and the next chunk's
-        # conversions and first rounds run beside them
-        for _a, _b, bp in self.chunks:
-            bp._join()
+        try:
+            k = 0
+            for a, b, bp in self.chunks:
+                for i in range(a, b):
+                    with torch.cuda.stream(self.copy_streams[k % len(self.copy_streams)]):
+                        self.dev_tables[i].copy_(self.host[i], non_blocking=True)
+                    k += 1
+                for st in self.copy_streams:  # this chunk's copies, not the later ones
+                    ev = torch.cuda.Event()
+                    ev.record(st)
+                    main.wait_event(ev)
+                for i in range(a, b):
+                    t = self.dev_tables[i]
+                    fld = get_device_field(self.specs[i], self.ctx.device)
+                    K, _L, N = t.shape
+                    _lib.check(lib.sc_tables_to_mont(self.ctx.handle, fld.handle, ctypes.c_void_p(t.data_ptr()),
+                                                     ctypes.c_uint64(N), int(K)), "sc_tables_to_mont")
+                bp._start()
+        finally:
+            # joined only now: a chunk's last rounds leave most of the GPU idle, and the next chunk's
+            # conversions and first rounds run beside them. Also when a later chunk could not be
+            # started: the tables are free for others once the caller's stream says so.
+            for _a, _b, bp in self.chunks:
+                bp._join()
 
     def wait(self) -> None:
         for _a, _b, bp in self.chunks:
