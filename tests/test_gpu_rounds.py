@@ -66,6 +66,45 @@ def test_many_blocks_match_c_oracle(bits, n):
     check(expression(3, n), get_field(bits), n, seed=n)
 
 
+@pytest.mark.parametrize("entry", ["noalloc", "split"])
+@pytest.mark.parametrize("degree", range(1, 8))
+@pytest.mark.parametrize("modulus,bits", MODULI, ids=[f"{m:#x}"[:12] + f"-{b}" for m, b in MODULI])
+def test_a_launch_per_round_matches_c_oracle(modulus, bits, degree, entry):
+    """The round kernel alone (sc_prove runs it for the largest rounds only): every register class,
+    with and without a fold, and rounds of 4096 pairs that take g(1) from the claim -- on one rank,
+    and from the shares of two."""
+    from test_gpu_split import _emulate
+    from test_zz_no_alloc import _noalloc
+
+    spec = field_for_modulus(modulus, bits)
+    expr = expression(degree, 300 + degree)
+    terms, k = O.indexed_terms(expr)
+    n = 14 if entry == "noalloc" else 15  # two ranks: 2^14 entries each
+    tables = api.generate_tables(spec, k, n, [0] * k, degree)
+    want = C.prove_seeded(terms, k, spec.modulus, spec.limbs, n, [0] * k, degree)
+    if entry == "noalloc":
+        ctx = api.get_context(tables.device)
+        ce = api.CompiledExpression(api.encode_expression(expr), spec.modulus)
+        rc, *got = _noalloc(ctx, api.get_device_field(spec, ctx.device), ce, n, tables, "sha3", spec.limbs, degree, k)
+        assert rc == api._lib.SC_OK, api._lib.last_error()
+        results = [got]
+    else:
+        results = [(p.round_polys_mont, p.challenges_mont, p.finals_mont, p.claim0_mont, p.checksum)
+                   for p in _emulate(tables, expr, spec, n, 2)]
+    for polys, chals, finals, claim0, checksum in results:
+        assert np.array_equal(polys, want["round_polys"])
+        assert np.array_equal(chals, want["challenges"])
+        assert np.array_equal(finals, want["finals"])
+        assert np.array_equal(claim0, want["claim0"])
+        assert checksum == want["checksum"]
+
+
+@pytest.mark.parametrize("degree", [2, 4, 7])
+@pytest.mark.parametrize("modulus,bits,n", [(m, b, 18 if b == 256 else 16) for m, b in MODULI[:4] + MODULI[-2:]])
+def test_large_rounds_then_parts_and_a_tail_match_c_oracle(modulus, bits, n, degree):
+    check(expression(degree, 500 + degree), field_for_modulus(modulus, bits), n, seed=n + degree)
+
+
 def test_tick_times_follow_each_other():
     from zkduel_b200.batch import BatchProver
 
