@@ -130,7 +130,7 @@ class FieldSpec:
         """Canonical values of an array of Montgomery-form limb vectors (last axis): native uint32
         arrays, as the library writes them, from their bytes; other types and lists word by word."""
         if getattr(limbs, "dtype", None) != _WORD:
-            a = np.asarray(limbs, dtype=object)
+            a = np.asarray(limbs.tolist() if hasattr(limbs, "tolist") else limbs, dtype=object)
             return [self.decode_limbs(v) for v in a.reshape(-1, a.shape[-1])] if a.size else []
         data, size, p, r_inv = limbs.tobytes(), 4 * limbs.shape[-1], self.modulus, self.r_inv
         return [int.from_bytes(data[i:i + size], "little") * r_inv % p for i in range(0, len(data), size)]

@@ -144,3 +144,21 @@ def test_host_limbs_are_the_callers_to_change(bits, entries):
     out = host_tables_to_limbs(vals, f)
     out[...] = 7
     assert vals.tolist() == np.arange(3 * entries).reshape(3, entries).tolist()
+
+
+@pytest.mark.parametrize("bits", [32, 256])
+def test_proof_decodes_limbs_held_on_a_device(bits):
+    """Tensors that do not convert to numpy (as a GPU's do not) are read word by word too."""
+    torch = pytest.importorskip("torch")
+
+    class OnDevice(torch.Tensor):
+        def __array__(self, *_args, **_kwargs):
+            raise TypeError("can't convert cuda:0 device type tensor to numpy")
+
+    f = F.FIELD_SPECS[bits]
+    rng = random.Random(bits)
+    values = [rng.randrange(f.modulus) for _ in range(6)]
+    limbs = torch.tensor([f.montgomery_limbs(x) for x in values], dtype=torch.int64).as_subclass(OnDevice)
+    p = Proof(f, 3, 1, ("a",), limbs.reshape(3, 2, f.limbs), limbs[:3], limbs[:2], limbs[5], 0)
+    assert p.round_polys == [values[:2], values[2:4], values[4:]] and p.challenges == values[:3]
+    assert p.claim0 == values[5] and p.final_claim == values[0] and p.final_values == values[1:2]
