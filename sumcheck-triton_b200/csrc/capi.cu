@@ -435,7 +435,6 @@ int sc_field_init(int limbs, const uint32_t* modulus, uint32_t nprime, sc_field*
   std::memcpy(C.p, hf.p, 4 * limbs);
   C.np = nprime;
   C.limbs = limbs;
-  C.p_small = big ? 0u : hf.p[0];
   // R mod p, R^2 mod p, R^2 2^(32 i) mod p by doubling from 1
   uint32_t x[8] = {0};
   x[0] = 1;

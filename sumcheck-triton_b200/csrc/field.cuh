@@ -461,14 +461,6 @@ __device__ __forceinline__ Fe<L> fe_fold(const Fe<L>& x0, const Fe<L>& x1, const
   }
 }
 
-template <int L>
-__device__ __forceinline__ bool fe_is_zero(const Fe<L>& a) {
-  uint32_t o = 0;
-#pragma unroll
-  for (int i = 0; i < L; ++i) o |= a.w[i];
-  return o == 0;
-}
-
 // Multiply by a small non-negative integer c by double-and-add. The result equals the
 // Montgomery product with c's Montgomery image; an addition chain is cheaper than a product
 // for the small coefficients constraint expressions carry.

@@ -32,7 +32,6 @@ using namespace sc_host;
 
 namespace {
 constexpr size_t kNoAllocScratchBytes = size_t{32} << 20;
-constexpr int kNoAllocMaxBlocks = 1184;  // 148 SMs x 8
 constexpr int kMaxDevices = 64;
 }  // namespace
 
@@ -82,7 +81,7 @@ static int run(sc_ctx* ctx, const sc_field* f, const sc_expr* ex, int n, const u
   int bps = 0;
   SC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, round_kernel<L, K, DMAX>, threads, smem));
   if (bps < 1) return fail(SC_ERR_UNSUPPORTED, "round kernel does not fit on an SM (K=%d, L=%d)", K_, L);
-  const uint64_t grid_max = std::min<uint64_t>(static_cast<uint64_t>(bps) * ctx->sm_count, kNoAllocMaxBlocks);
+  const uint64_t grid_max = static_cast<uint64_t>(bps) * ctx->sm_count;
 
   // carve the scratch array: field constants, proof state and sums, fold A, fold B
   const StateOffsets so = state_offsets(n, K_, L);

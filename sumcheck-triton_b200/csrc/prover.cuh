@@ -59,7 +59,6 @@ struct FieldConsts {
   uint32_t p[kMaxLimbs];
   uint32_t np;
   uint32_t limbs;
-  uint32_t p_small;                          // p if p < 2^32, else 0
   uint32_t one[kMaxLimbs];                   // R mod p
   uint32_t r2[kMaxLimbs];                    // R^2 mod p
   uint32_t r3[kMaxLimbs];                    // R^3 mod p
@@ -483,19 +482,12 @@ __device__ __forceinline__ void shape_add_lead(GoldSum& acc, const Fe<2> (&d)[6]
 #ifndef SC_GOLD_ASYNC
 #define SC_GOLD_ASYNC 1
 #endif
-// The same stage for the 8-limb g(abc + de) shape kernel (SC_L8_ASYNC; 96 KB a block of 128
-// threads, 2 blocks an SM) measured slower on B200: plain BLS n = 22 3.37 against 3.25 ms
-// (255 registers with 120 bytes of spills, against none). Off.
-#ifndef SC_L8_ASYNC
-#define SC_L8_ASYNC 0
-#endif
-__host__ __device__ constexpr bool gold_async_stage(int L, int K, int shape) {
+// The same stage for the 8-limb g(abc + de) shape kernel (96 KB a block of 128 threads, 2 blocks
+// an SM) measured slower on B200: plain BLS n = 22 3.37 against 3.25 ms (255 registers with 120
+// bytes of spills, against none).
+__host__ __device__ constexpr bool shape_async_stage(int L, int K, int shape) {
   return SC_GOLD_ASYNC && L == 2 && K == kFieldGoldilocks && shape != kShapeGeneric && SC_GOLD_SHAPE_FMA &&
          SC_GOLD_LAZY;
-}
-__host__ __device__ constexpr bool l8_async_stage(int L, int shape) { return SC_L8_ASYNC && L >= 8 && shape == kShapeAbcg; }
-__host__ __device__ constexpr bool shape_async_stage(int L, int K, int shape) {
-  return gold_async_stage(L, K, shape) || l8_async_stage(L, shape);
 }
 // Dynamic shared memory (bytes) of a compile-time shape round kernel of `threads` threads.
 __host__ __device__ constexpr size_t shape_round_smem_bytes(int L, int K, int shape, int threads) {
@@ -546,7 +538,7 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
     for (int i = 0; i < 5; ++i) gsum[t].w[i] = 0;
   constexpr int NR = SHAPE == kShapeGeneric ? 1 : shape_tables(SHAPE);
   constexpr bool kGoldLazy = SHAPE != kShapeGeneric && L == 2 && K == kFieldGoldilocksFma && SC_GOLD_LAZY;
-  constexpr bool kAsync = (kGoldLazy && SC_GOLD_ASYNC) || l8_async_stage(L, SHAPE);
+  constexpr bool kAsync = kGoldLazy && SC_GOLD_ASYNC;
   const int nv = SHAPE == kShapeGeneric ? E.num_vars : NR;
   // kAsync: this thread's stage, after the block reduction's scratch (16-byte aligned)
   uint32_t* const stage = sv + reduce_scratch_words(nthr, L);
