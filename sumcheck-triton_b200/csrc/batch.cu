@@ -29,7 +29,7 @@ constexpr bool kBatchDmax6 = SC_BATCH_DMAX6 != 0;  // see dispatch_dmax
 // once is cut that way, and a part is spread over its block's threads (tail.cuh): a thread a
 // pair leaves most of the GPU idle while it walks through the pair. Measured on B200: 64 mixed
 // proofs 4.72 -> 4.44 ms, 24 proofs from host memory 4.19 -> 3.09 ms; with parts of 64 pairs
-// 4.49 / 3.25 ms, with ticks of up to two grids 4.44 / 3.10 ms.
+// 4.49 / 3.25 ms, with ticks of up to two grids 4.44 / 3.10 ms. Parts below 32 pairs were not timed.
 constexpr uint64_t kSmallPartPairs = 32;
 inline uint64_t small_parts(int n, int t) { return std::max<uint64_t>(1, ((uint64_t{1} << n) >> (t + 1)) / kSmallPartPairs); }
 inline size_t small_part_smem(int n, int t, int K, int L) {
@@ -158,7 +158,8 @@ namespace {
 // A tick. Its blocks record its start and end (BatchTickArgs::span): event nodes would be links of
 // the chain of kernels and are made, and made part of the graph, for every batch. Measured on B200 with
 // two event nodes a tick, one on a branch beside the kernels, and none: 64 mixed proofs 4.45, 4.39 and
-// 4.31 ms; 24 proofs from host memory, batches made on the way, 2.66, 2.13 and 1.49 ms.
+// 4.31 ms; a later run of 24 proofs from host memory in 4 chunks 2.66, 2.13 and 1.49 ms (a prover's
+// first run also captures and instantiates the graphs).
 // Setting a tick up while the one before it ends (launch_after) did not pay: its waiting blocks hold
 // room the other classes' ticks use (64 mixed proofs 4.53 ms; for small ticks alone no change).
 int batch_tick(sc_batch* B, const BatchClass& C, const BatchTickArgs& T) {

@@ -3,8 +3,9 @@
 // Host side of the prover: field and expression set-up, the scratch-owning context,
 // table generation and the per-proof launch sequence. The reference drives its CUDA
 // kernels from a CLI loop with a blocking device-to-host copy per interpolation point
-// (cuda/src/field_sumcheck.cu:1012-1088); here a proof is num_rounds launches of one
-// fused round kernel on the caller's stream and a single copy of the results at the end.
+// (cuda/src/field_sumcheck.cu:1012-1088); here a proof is one fused launch per large round,
+// queued ahead of the round before it, one launch for all small last rounds, and a single copy
+// of the results at the end, all on the caller's stream.
 #include "host_common.h"
 
 using namespace sc;

@@ -86,7 +86,7 @@ __device__ __forceinline__ void gold_mul_fma(uint32_t (&r)[2], const uint32_t (&
 }
 
 // Lazy forms: operands anywhere in [0, 2^64) (any representative of their residue), results
-// in [0, 2^64), nothing canonical until gold_canon. 2^64 = 2^32 - 1 = eps (mod p), so a carry
+// in [0, 2^64), nothing made canonical (gold_canon would). 2^64 = 2^32 - 1 = eps (mod p), so a carry
 // out of bit 63 is worth eps and a borrow -eps.
 
 // r = a + b for a in [0, 2^64) and b < p: s = a + b, then s + eps on a carry, which cannot

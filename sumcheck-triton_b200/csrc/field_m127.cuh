@@ -2,7 +2,8 @@
 //
 // With p = 2^127 - 1, 2^128 = 2 (mod p): a carry out of 128 bits is worth 2 and a borrow -2, so
 // sums, differences and products stay in four words with no compare and no select, and a value
-// is made canonical (m127_canon) only where it leaves a thread. R = 2^128 = 2 (mod p), so the
+// is made canonical (m127_canon) only by a fold, whose result is stored, and by fe_mul; point sums
+// leave a thread as any representative and are reduced once a round. R = 2^128 = 2 (mod p), so the
 // Montgomery product x y / R = x y / 2: with x y = hi 2^128 + lo it is hi + lo / 2, and
 // lo / 2 = (lo >> 1) + (lo & 1) 2^126.
 //

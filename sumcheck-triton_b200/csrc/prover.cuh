@@ -192,8 +192,9 @@ __device__ __forceinline__ Fe<L> add_or_sub(const Fe<L>& acc, const Fe<L>& x, bo
 
 // The generic evaluator over Goldilocks in lazy arithmetic (field.cuh gl_*): stepped values,
 // products and point sums are any representatives in [0, 2^64); the values and differences it
-// reads are canonical, and process_pairs makes the point sums canonical after the thread's
-// last pair. Measured on B200, the mixed stream's 64-bit group alone: 5.93 against 6.07 ms.
+// reads are canonical. A thread's point sums leave it as they are: the round's integer sums are
+// reduced mod p once (sums_to_points). Measured on B200, the mixed stream's 64-bit group alone,
+// when the sums were still made canonical per thread: 5.93 against 6.07 ms.
 #ifndef SC_GOLD_LAZY_GENERIC
 #define SC_GOLD_LAZY_GENERIC 1
 #endif
@@ -462,9 +463,11 @@ __device__ __forceinline__ void shape_add_lead(GoldSum& acc, const Fe<2> (&d)[6]
 #endif
 
 // Folds (if fold) and evaluates pairs q = first, first + stride, ... < last, adding the
-// point sums into acc. Generic: every table's value and difference go to this block's
-// [K][L][nthr] shared arrays sv / sd for eval_pair. Shape kernels keep them in registers
-// (tables read in role order) and evaluate the shape's compile-time formula at each point.
+// point sums into acc. Generic, up to 4 limbs: every table's values at 0 and 1 go to this
+// block's [K][L][nthr] shared arrays sv / sd for eval_pair; at 8 limbs the tables are read from
+// memory at every use and sv holds the point sums and products (streamed_tables). Shape kernels
+// keep values and differences in registers (tables read in role order) and evaluate the shape's
+// compile-time formula at each point.
 // 2-limb shape kernels issue every load of a pair before its folds and run 2 blocks/SM
 // (<= 128 registers for the loaded words): measured on B200, Goldilocks n = 24 went from
 // 2.18 ms (loads interleaved with folds, 3 blocks/SM) to 2.01 ms.
@@ -743,9 +746,6 @@ __device__ __forceinline__ void process_pairs(const uint32_t* __restrict__ src, 
         const Fe<L> o = sh_d[r];
         sh_d[r] = fe_sub(o, sh_v[r], F);
         sh_v[r] = o;
-      }
-      if constexpr (kAsync) {
-        if (!fold && q + stride < last) issue(q + stride);
       }
       if (!skip1) acc[1] = fa_add(acc[1], shape_value<L, K>([&](int i) { return sh_v[i]; }, F, shape), F);
       shape_value2<L, K>([&](int i) { return fa_add(sh_v[i], sh_d[i], F); },
@@ -1183,11 +1183,9 @@ __host__ __device__ constexpr int round_smem_words_per_thread(int K, int L, int 
   return streamed_tables(L) ? 2 * dmax * L : 2 * K * L;
 }
 
-// Launch shape per limb count: 8-limb kernels hold (DMAX + 1) x 8-word point arrays per
-// thread, so they run 128-thread blocks and ask the compiler for at least 3 blocks per SM
-// (<= 168 registers; on B200 the mixed 512-proof stream ran 10% slower with 2 or 4 blocks
-// with the C++ product, 5% and 4% slower with the even/odd product); smaller fields run
-// 256-thread blocks.
+// Launch shape per limb count: 8-limb kernels run 128-thread blocks, smaller fields 256-thread
+// blocks. Blocks an SM asked of the compiler at 8 limbs: batch_min_blocks below for the generic
+// kernels (SC_L8_MIN_BLOCKS, <= 168 registers, above degree 4), round_min_blocks for the shapes.
 __host__ __device__ constexpr int kernel_threads(int L) { return L >= 8 ? 128 : 256; }
 #ifndef SC_L8_MIN_BLOCKS
 #define SC_L8_MIN_BLOCKS 3
@@ -1212,14 +1210,15 @@ __host__ __device__ constexpr int kernel_min_blocks(int L) {
 #ifndef SC_SHAPE_MIN_BLOCKS
 #define SC_SHAPE_MIN_BLOCKS 2
 #endif
-// Shape kernels of the 1- and 2-limb fields are memory-bound: ask for more resident blocks.
-// The 8-limb shape kernels hold every table's value and difference in registers: at 3 blocks
+// The 1- and 2-limb shape kernels run 2 blocks of 256 threads: at 3 the 2-limb ones spilled
+// (zerocheck gate n = 24 1.66 against 1.55 ms with the pair staged in shared memory). The 8-limb
+// shape kernels hold every table's value and difference in registers: at 3 blocks
 // of 128 threads they spilled; at 2 (no spills) plain BLS n = 22 took 3.28 against 3.37 ms
-// with the even/odd product (the batched 8-limb kernels stay at 3, where 2 was 5% slower).
+// with the even/odd product.
 #ifndef SC_SHAPE_L8_MIN_BLOCKS
 #define SC_SHAPE_L8_MIN_BLOCKS 2
 #endif
-// The batched kernel per limb count and degree class: at 8 limbs 4 blocks/SM up to degree 4
+// The generic kernels, plain and batched, per limb count and degree class: at 8 limbs 4 blocks/SM up to degree 4
 // (128 registers), 3 above (shared memory for 7-8 points' products and sums). 5 and 4 blocks
 // spilled more than they hid (64 mixed proofs 5.09 ms against 4.84; 3 and 3 blocks 4.99).
 __host__ __device__ constexpr int batch_min_blocks(int L, int dmax) {
