@@ -36,6 +36,11 @@ inline size_t small_part_smem(int n, int t, int K, int L) {
   return static_cast<size_t>(std::min<uint64_t>((uint64_t{1} << n) >> (t + 1), kSmallPartPairs)) * 2 * K * L * 4;
 }
 
+// Every thread of a round's tiles adds words below 2^32 to its 64-bit sums (prover.cuh, block_sums):
+// up to 2^32 threads fit, with the carries of sums_to_points. A proof of 2^33 pairs or more takes as
+// many pairs a thread as keep to that (the other paths' grids are bounded by the GPU).
+inline int min_pairs_per_thread(int n) { return n <= 33 ? 1 : 1 << (n - 33); }
+
 struct BatchClass {
   int dclass = 2;
   int dmax = 2;  // the kernel instance: dclass, or 6 for a degree <= 7 class without degree 7
@@ -372,7 +377,7 @@ int sc_batch_create_tiled(sc_ctx* ctx, const sc_field* field, int count, const s
   for (int c = 0; c < 3; ++c) B->class_threads[c] = class_threads ? class_threads[c] : 0;
   for (int p = 0; p < count; ++p) {
     const int v = proof_pairs_per_thread ? proof_pairs_per_thread[p] : 0;
-    B->ppt.push_back(v ? v : 2);
+    B->ppt.push_back(std::max(v ? v : 2, min_pairs_per_thread(num_rounds[p])));
   }
   for (int p = 0; p < count; ++p) B->n.push_back(num_rounds[p]);
   int rc;

@@ -152,3 +152,24 @@ def test_host_batch_prover_equals_single_proofs(chunks):
         for s, t, p in zip(specs, dev, res):
             _same(p, api.prove_device(t, s.expression, get_field(s.bit_width), s.num_vars, "sha3"))
     hb.close()
+
+
+def test_sums_of_the_largest_rounds_fit_their_words():
+    """One pair a thread over 2^34 entries: 2^33 threads add a word each to a round's 64-bit sums.
+    A constant table of p - 1 makes every word as large as it can be, and has a known proof."""
+    spec, n = get_field(32), 34
+    free, _total = torch.cuda.mem_get_info()
+    need = (1 << n) * 4 * 7 // 4 + (10 << 30)  # table, fold buffers, work items
+    if free < need:
+        pytest.skip(f"needs {need / 2**30:.0f} GiB of device memory")
+    top = spec.modulus - 1  # as a Montgomery word; sums of such words are sums mod p
+    table = torch.full((1, 1, 1 << n), top - (1 << 32), dtype=torch.int32, device="cuda")
+    bp = BatchProver([(((1, ("a",)),), 32, n, table)], tile={1: (0, 1)})
+    bp.run()
+    (proof,) = bp.results()
+    bp.close()
+    del table
+    torch.cuda.empty_cache()
+    want = [[top * (1 << (n - 1 - j)) % spec.modulus] * 2 for j in range(n)]
+    assert proof.round_polys_mont[:, :, 0].tolist() == want
+    assert proof.finals_mont[:, 0].tolist() == [top, top]
